@@ -43,8 +43,11 @@ extern "C" {
 #define PAWAN_PREC_F64 1        /* FP64, same algebra as the FP32 kernel */
 #define PAWAN_PREC_F64_PLAIN 2  /* FP64, the reference's formula term by term */
 
-/* Tiling of the pair kernel (the compiled variants are listed by
- * pawan_system_autotune's candidates; set_tiling rejects others). */
+/* Tiling of the pair kernel (the tilings of each kind are listed by
+ * pawan_tile_candidates; set_tiling rejects others).  FP32 with packed > 0 runs
+ * on the symmetric pair engine, which computes each unordered pair once for
+ * both particles; there only items_per_slot matters.  packed = 0 is the
+ * one-sided kernel the other fields describe. */
 typedef struct {
   int threads;            /* threads per block = sources per shared-memory tile: 128 or 256 */
   int threads_per_target; /* threads sharing one target's sources: 1, 2 or 4 */
@@ -52,14 +55,9 @@ typedef struct {
   int unroll;             /* unroll depth of the source loop */
   int blocks_per_sm;      /* blocks per SM the registers are bounded for, 0 = default */
   int items_per_slot;     /* work items per resident block (source chunking) */
-  int packed;             /* far tiles two sources per FP32x2 instruction: 1 with
-                             1/rho^2 from the MUFU reciprocal, 2 from rsqrt
-                             squared; 0: one source per instruction */
-  int split_near;         /* FP32: 1 computes the near tile pairs in a pass of
-                             their own before the far pass (each kernel with its
-                             own registers; faster where near pairs are many),
-                             2 the same with the near pass two sources per
-                             FP32x2 instruction; 0: one pass */
+  int packed;             /* FP32: 1 or 2 (alike): the symmetric engine, the
+                             default; 0: one-sided, one source per instruction */
+  int split_near;         /* FP32 with packed > 0: 0, 1 or 2, accepted alike */
 } pawan_tiling;
 
 typedef struct pawan_ctx pawan_ctx;
@@ -325,10 +323,9 @@ int pawan_server_fetch(pawan_server *srv, long long id, double *state, size_t si
                        double *t_submit, double *t_admit, double *t_done);
 int pawan_server_cancel(pawan_server *srv, long long id);
 int pawan_server_stats(pawan_server *srv, pawan_serve_stats *out);
-/* The tiling the engine's pair launches use (FP32: 128 threads, packed far
- * path mode 1, the packed near pass; sources in fixed 8,192-source chunks, so
- * items_per_slot is not used), for running a request alone with the same
- * arithmetic. */
+/* The tiling the engine's pair launches use (FP32: the symmetric engine, in
+ * slots of at most 400 MB per request), for running a request alone with the
+ * same FP32 arithmetic. */
 int pawan_server_get_tiling(pawan_server *srv, pawan_tiling *out);
 /* Host-side fault injection, for testing how callers and the engine recover
  * (no GPU fault is made).  PAWAN_FAULT_ALLOC: the next `count` admissions

@@ -64,9 +64,8 @@ class Tiling(ctypes.Structure):
 
 def _tiling(threads, threads_per_target=1, unroll=4, items_per_slot=16, targets_per_thread=1,
             blocks_per_sm=0, packed=0, split_near=0) -> Tiling:
-    """packed: 0 one source per instruction on far tiles; 1 two sources per FP32x2
-    instruction with 1/rho^2 from the MUFU reciprocal; 2 the same with 1/rho^2
-    from rsqrt squared (True means 1)."""
+    """packed: 1 or 2 the symmetric pair engine (FP32; True means 1), 0 the
+    one-sided kernel of the other fields."""
     return Tiling(threads, threads_per_target, targets_per_thread, unroll, blocks_per_sm, items_per_slot,
                   int(packed), int(split_near))
 

@@ -17,7 +17,7 @@ size_t pawan_system::device_bytes() const {
          vol.bytes() + wake_id.bytes() + pos32.bytes() + vor32.bytes() + poslo.bytes() +
          vorlo.bytes() + pos64.bytes() +
          vor64.bytes() + diag_scratch.bytes() + diag_out.bytes() + Xc.bytes() + field.bytes() +
-         (plan ? plan->partial.bytes() + plan->rates.bytes() + plan->tile_count.bytes() : 0);
+         (plan ? plan->partial.bytes() + plan->rates.bytes() + plan->tile_count.bytes() + plan->slots.bytes() : 0);
 }
 
 // =================================================================== C ABI
@@ -147,7 +147,7 @@ int pawan_ctx_create(int device, pawan_ctx **out) {
   if (prop.major != 10) return PAWAN_ERR_CUDA;  // built for sm_100a only
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess)
     return PAWAN_ERR_CUDA;
-  if (cudaMalloc(&ctx->d_counter, 2 * sizeof(int)) != cudaSuccess) {
+  if (cudaMalloc(&ctx->d_counter, sizeof(int)) != cudaSuccess) {
     cudaStreamDestroy(ctx->stream);
     return PAWAN_ERR_NOMEM;
   }

@@ -40,10 +40,6 @@ struct SegDesc {
   double *partial;      // [ceil(n / tpb)][nchunks][6][tpb] (unused when nchunks == 1)
   double *rates;        // [6][n]
   int *tile_count;      // [ceil(n / tpb)] items of the tile done in this launch (0 between launches)
-  // with a separate near pass (split tilings): each item's sums over its near
-  // tile pairs, [ceil(n / tpb)][nchunks][6][tpb], and whether it had any
-  double *near_partial;
-  unsigned char *near_flag;  // [ceil(n / tpb)][nchunks]
   int n;
   int nchunks;
   double nu;
@@ -109,6 +105,38 @@ enum StageMode : int {
   STAGE_EULER = 5,   // x = x + r*dt; pack x   (integration.cpp:37-45)
   STAGE_PACK = 6,    // pack x only
   STAGE_SHARD = 7,   // this process's block of rates -> xchg_out (no state change)
+};
+
+// ---- symmetric pair engine (pair_sym.cu) ----
+// Tiles of 128 particles; groups of 1 tile (small systems) or 4 (large ones).
+constexpr int kSymTile = 128;
+constexpr int kSymGroup = 4;
+
+// One solve as the symmetric kernels see it.
+struct SymSeg {
+  const float4 *pos32, *vor32, *poslo, *vorlo;
+  const double4 *pos64, *vor64;
+  const float4 *boxes;  // (lo, hi) per tile
+  double *rates;        // [6][n]
+  int n;
+  double nu;
+  float near2;          // squared box distance below which a tile pair is near
+};
+
+// Group a against the groups [b0, b1), a <= b0.  Slots hold the six sums of a
+// group's particles ([tile][6][128] doubles): the item's sums of group a go to
+// slot `islot`, those of group b to slot jbase[jb + b] + a - row0 (none where
+// islot or jbase is negative: another process's targets).
+struct SymItem {
+  int seg, a, b0, b1, islot, row0, jb;
+};
+
+// One tile of the slot sums: `count` slots `stride` doubles apart from
+// slots[first], in that order, into rates[.][128 t ..] (added to what is there
+// when `add`).
+struct SymSum {
+  long long first;
+  int stride, count, seg, t, add;
 };
 
 // Smoothing kernel of a system: the reference's high-order algebraic kernel

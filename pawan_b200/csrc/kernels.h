@@ -11,14 +11,8 @@ namespace pawan {
 // shared-memory tile), `p` threads per target, `r` targets per thread
 // (targets per block = tb / p * r), `unroll` = unroll depth of the source loop,
 // `minb` = blocks per SM the registers are bounded for (0: the default),
-// `packed` = far tiles computed two sources per FP32x2 instruction (1: 1/rho^2
-// from the MUFU reciprocal on uniform-radius tiles, 2: from rsqrt squared;
-// 0: one source per instruction).
-// `split` = 1: near tile pairs are computed by a pass of their own before the
-// far pass (which then skips them), each kernel with its own register
-// allocation, the near pass forming alpha_i x alpha_j by the projection form
-// (19 operations instead of the one pass's 27); `split` = 2: the same with the
-// near pass two sources per FP32x2 instruction.
+// `packed` > 0: the symmetric engine (pair_sym.cu), which the other fields and
+// `split` do not change; 0: the one-sided scalar kernel.
 struct PairConfig {
   int tb;
   int p;
@@ -36,10 +30,21 @@ inline int targets_per_block(const PairConfig &c) { return c.tb / c.p * c.r; }
 // FP32 pair math, FP64 accumulation of per-tile partial sums.
 bool pairs_f32_supported(const PairConfig &c, int kernel);
 cudaError_t pairs_f32_occupancy(const PairConfig &c, bool diffusion, int kernel, int *blocks_per_sm);
-// next_item: two counters (the far pass's and the near pass's), zero at launch.
+// next_item: the work-item counter, zero at launch.  The packed tilings are the
+// symmetric engine's (below): supported here, launched there.
 cudaError_t launch_pairs_f32(const PairConfig &c, bool diffusion, int kernel, int grid,
                              const WorkItem *items, int n_items, const SegDesc *segs,
                              int *next_item, cudaStream_t s);
+
+// The symmetric pair engine (FP32): each unordered pair once, sums into the
+// items' slots; one block per item.  group: items over groups of kSymGroup
+// tiles, else over single tile pairs.
+cudaError_t sym_f32_occupancy(bool group, bool diffusion, int kernel, int *blocks_per_sm);
+cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
+                           const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s);
+// Sums the slots of each listed tile into its rates.
+cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const SymSeg *segs, const double *slots,
+                            cudaStream_t s);
 
 // FP64 with the same algebra as the FP32 kernel ("tuned FP64").
 bool pairs_f64_supported(const PairConfig &c, int kernel);

@@ -1,0 +1,725 @@
+// All-pairs interaction, FP32 pair math with FP64 accumulation, every unordered
+// particle pair once: the symmetric pair engine (the FP32 hot path).
+//
+// Reference: the pair physics of INTERACT (src/interaction/interaction_utils.h:363-407)
+// with KERNEL (src/interaction/highorder.h:48-60), summed over all unordered
+// pairs of a system by __interaction::interact (src/interaction/interaction.cpp:95-108).
+// The pair algebra and the tile-pair classes are pair_f32.cu's (its file
+// comment derives them); what differs is that a pair's distance, kernel
+// factors, alpha_i x alpha_j and triple product are formed once and added to
+// both particles.
+//
+// Symmetric forms.  Far (x' = x - c, beta = alpha x x', d = x'_i - x'_j):
+//   u_i   += m (alpha_j x d),       u_j   -= m (alpha_i x d)
+//   W_i    = sum m beta_j, Q_i = sum m alpha_j, G_i = sum g d
+//   W_j    = sum m beta_i, Q_j = sum m alpha_i, N_j = sum g d = -G_j
+//   with t~ = alpha_j.beta_i + alpha_i.beta_j (= -alpha_i.(alpha_j x d)) and
+//   g = -fh t, so u = A (Q x x' - W), dalpha = alpha x (A Q) + 3 A G on either side.
+// Near (hi/lo differences): u_i += q (alpha_j x d), u_j -= q (alpha_i x d), and
+// one vector s = q (alpha_i x alpha_j) + 3 F t d + 15 nu Dp (v_i alpha_j -
+// v_j alpha_i), antisymmetric in (i, j): dalpha_i += s, dalpha_j -= s.  The
+// diffusion vector is formed as v_i delta + (v_i - v_j) alpha_i from delta =
+// alpha_j - alpha_i, accurate for nearly equal strengths.
+//
+// Layout.  A warp computes a 128 x 128 tile pair (I, J): each lane holds R
+// targets of I (4 on far tiles, 2 on near ones) and their sums in registers,
+// and 32 sources of J at a time sit in shared memory, one per lane.  At step k
+// lane l takes source l ^ k (bank-conflict-free), and the sums of that source
+// travel with it by shuffle (9 floats far, 6 near), so after 32 steps every
+// source has met all the warp's targets and its sums are back at its own lane.
+// Sums are FP32 over 32 sources (near, small systems) or 128 (far, large
+// ones) on the target's side and over 128 (64 near) targets on the source's,
+// then folded into FP64.
+//
+// What bounds it: register-file reads of the FMA pipe.  A far step of one
+// target is 37 FMA-pipe operations and one MUFU for two interactions (the
+// one-sided packed loop: 28 for one); 23 of them read three different
+// registers, at about two reads per cycle and lane.  The step's 3 loads, 9
+// shuffles and address are shared by four targets; with two the shared-memory
+// pipe (21 of its cycles per step) would be the limit.  One right-hand side of
+// the ring pair at N = 131,072: 14.2 ms (1,210 G interactions/s) against 18.4 ms
+// one-sided; 20,011 unordered particles (near tile pairs only, mixed radii)
+// 0.87 ms against 1.48.
+//
+// Work items.  Large systems: a block of four warps takes a group of 4 tiles
+// (512 particles) against a run of groups; in round r warp w computes tile w
+// against tile (w + r) % 4 of the group, so no two warps add to one source's
+// FP64 sums at a time and their order is fixed.  Small systems: one tile pair
+// per block, each warp 32 of its sources.  An item writes its target-side sums
+// once and its source-side sums per group, each to a slot of its own; a
+// separate kernel sums a particle's slots in a fixed order, so results do not
+// depend on scheduling.
+#include <mutex>
+#include <set>
+#include <utility>
+
+#include "device.cuh"
+#include "kernels.h"
+#include "pair_scalars.cuh"
+
+namespace pawan {
+namespace {
+
+constexpr int kWarps = 4;
+constexpr int kThreads = 32 * kWarps;
+constexpr int kBlocks = 3;          // per SM: 168 registers, no spills (four blocks of 128 ran 4 % slower)
+constexpr int kT = kSymTile;        // particles per tile
+constexpr int kStageBytes = 1792;   // per warp: 3 x float4[32], float2[32]
+constexpr unsigned kFull = 0xffffffffu;
+
+struct Stage {
+  float4 *s0, *s1, *s2;
+  float2 *s3;
+};
+
+__device__ __forceinline__ Stage stage_of(char *base) {
+  Stage s;
+  s.s0 = reinterpret_cast<float4 *>(base);
+  s.s1 = reinterpret_cast<float4 *>(base + 512);
+  s.s2 = reinterpret_cast<float4 *>(base + 1024);
+  s.s3 = reinterpret_cast<float2 *>(base + 1536);
+  return s;
+}
+
+// Particles past the end: far from everything (as a source and as a target on
+// opposite sides, so that they never coincide), zero strength and volume; every
+// product they enter is exactly zero.
+constexpr float kPadSource = 1e18f, kPadTarget = -1e18f;
+
+enum FarClass { FAR_Z = 0, FAR_NZ = 1, FAR_SER = 2 };
+
+struct FarTarget {
+  float x, y, z;     // x' = x - c
+  float ax, ay, az;  // strength (hi)
+  float bx, by, bz;  // beta = alpha x x'
+  float h, v;
+};
+
+struct Sums9 {
+  float wx, wy, wz, qx, qy, qz, gx, gy, gz;
+};
+
+__device__ __forceinline__ void rotate(Sums9 &a, int m) {
+  a.wx = __shfl_xor_sync(kFull, a.wx, m);
+  a.wy = __shfl_xor_sync(kFull, a.wy, m);
+  a.wz = __shfl_xor_sync(kFull, a.wz, m);
+  a.qx = __shfl_xor_sync(kFull, a.qx, m);
+  a.qy = __shfl_xor_sync(kFull, a.qy, m);
+  a.qz = __shfl_xor_sync(kFull, a.qz, m);
+  a.gx = __shfl_xor_sync(kFull, a.gx, m);
+  a.gy = __shfl_xor_sync(kFull, a.gy, m);
+  a.gz = __shfl_xor_sync(kFull, a.gz, m);
+}
+
+// Adds a pair's weight m to both particles' W and Q sums.
+__device__ __forceinline__ void add_wq(const FarTarget &T, const float4 &s, const float4 &e, float m, Sums9 &a,
+                                       Sums9 &b) {
+  a.wx = fmaf(m, e.x, a.wx);
+  a.wy = fmaf(m, e.y, a.wy);
+  a.wz = fmaf(m, e.z, a.wz);
+  a.qx = fmaf(m, s.x, a.qx);
+  a.qy = fmaf(m, s.y, a.qy);
+  a.qz = fmaf(m, s.z, a.qz);
+  b.wx = fmaf(m, T.bx, b.wx);
+  b.wy = fmaf(m, T.by, b.wy);
+  b.wz = fmaf(m, T.bz, b.wz);
+  b.qx = fmaf(m, T.ax, b.qx);
+  b.qy = fmaf(m, T.ay, b.qy);
+  b.qz = fmaf(m, T.az, b.qz);
+}
+
+// t~ = alpha_j.beta_i + alpha_i.beta_j
+__device__ __forceinline__ float far_t(const FarTarget &T, const float4 &s, const float4 &e) {
+  return fmaf(T.az, e.z, fmaf(T.ay, e.y, fmaf(T.ax, e.x,
+         fmaf(s.z, T.bz, fmaf(s.y, T.by, s.x * T.bx)))));
+}
+
+// 32 sources of a far tile with the Z terms against R targets per lane.  kap:
+// the diffusion factor in the units of the G sums (5 nu, or 80 nu / h with one
+// radius).
+template <bool UNI, bool DIFF, int KERN, int R>
+__device__ __forceinline__ void far_block_z(const Stage &st, int lane, const FarTarget (&T)[R], float hu,
+                                            float kap, Sums9 (&a)[R], Sums9 &b) {
+  const float s2u = 2.f * hu, c240 = -480.f * hu;
+#pragma unroll 1
+  for (int kk = 0; kk < 32; kk += 2) {
+    const int base = lane ^ kk;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const float4 p = st.s0[base ^ u], s = st.s1[base ^ u], e = st.s2[base ^ u];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float dx = T[r].x - p.x, dy = T[r].y - p.y, dz = T[r].z - p.z;
+        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        const float ri = rsqrtf(r2);
+        float m, fh, dp;
+        if (KERN == KERNEL_GAUSSIAN)
+          gauss_scalars(T[r].h + p.w, r2, ri, m, fh, dp);
+        else if (UNI)
+          kernel_scalars_uniform(hu, c240, rsqrtf(r2 + s2u), ri, m, fh, dp);
+        else
+          kernel_scalars(T[r].h + p.w, rsqrtf(r2 + (T[r].h + p.w)), ri, m, fh, dp);
+        const float g = -fh * far_t(T[r], s, e);
+        float gx = g * dx, gy = g * dy, gz = g * dz;
+        if (DIFF) {
+          const float kd = kap * dp;
+          gx = fmaf(kd, fmaf(T[r].v, s.x, -s.w * T[r].ax), gx);
+          gy = fmaf(kd, fmaf(T[r].v, s.y, -s.w * T[r].ay), gy);
+          gz = fmaf(kd, fmaf(T[r].v, s.z, -s.w * T[r].az), gz);
+        }
+        add_wq(T[r], s, e, m, a[r], b);
+        a[r].gx += gx;
+        a[r].gy += gy;
+        a[r].gz += gz;
+        b.gx += gx;
+        b.gy += gy;
+        b.gz += gz;
+      }
+      // lane l holds the sums of source l ^ k and next takes l ^ (k + 1)
+      const int k = kk + u;
+      rotate(b, (k ^ (k + 1)) & 31);
+    }
+  }
+}
+
+// The same without the Z terms (FAR_NZ, FAR_SER), R even: two targets per
+// FP32x2 instruction where no source operand enters (distance, kernel factors),
+// scalar FMAs for the rest.  The loop is held by register-file reads -- an FMA
+// of three different registers takes 1.5 issue slots, one of an FP32x2 pair
+// half -- which is what the packing saves: 1,435 G interactions/s against 1,340
+// of the scalar loop in a loop of its own on one B200, 1,210 against 1,150 in
+// this kernel on the ring pair at N = 131,072.
+template <int CLS, bool UNI, int KERN, int R>
+__device__ __forceinline__ void far_block(const Stage &st, int lane, const FarTarget (&T)[R], float hu,
+                                          Sums9 (&a)[R], Sums9 &b) {
+  const float2 one2 = make_float2(1.f, 1.f), half2 = make_float2(0.5f, 0.5f), nhalf2 = make_float2(-0.5f, -0.5f);
+  const float2 h2 = make_float2(hu, hu), nh2 = make_float2(-hu, -hu), s2u2 = make_float2(2.f * hu, 2.f * hu);
+#pragma unroll 1
+  for (int kk = 0; kk < 32; kk += 2) {
+    const int base = lane ^ kk;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const float4 p = st.s0[base ^ u], s = st.s1[base ^ u], e = st.s2[base ^ u];
+#pragma unroll
+      for (int r = 0; r < R; r += 2) {
+        const FarTarget &X = T[r], &Y = T[r + 1];
+        const float2 dx = make_float2(X.x - p.x, Y.x - p.x), dy = make_float2(X.y - p.y, Y.y - p.y),
+                     dz = make_float2(X.z - p.z, Y.z - p.z);
+        const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+        const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+        const float2 ri2 = __fmul2_rn(ri, ri);
+        float2 m;
+        if (CLS == FAR_SER && KERN == KERNEL_GAUSSIAN) {
+          m = __fmul2_rn(ri, ri2);
+        } else if (CLS == FAR_SER && UNI) {
+          m = __fmul2_rn(__fmul2_rn(__fmul2_rn(ri, ri2), __ffma2_rn(nh2, ri2, one2)), ri2);
+        } else if (CLS == FAR_SER) {
+          const float2 eps = __fmul2_rn(make_float2(X.h + p.w, Y.h + p.w), ri2);
+          m = __fmul2_rn(__fmul2_rn(__fmul2_rn(eps, ri), ri2), __ffma2_rn(nhalf2, eps, one2));
+        } else if (UNI) {
+          const float2 sr = __fadd2_rn(r2, s2u2);
+          const float2 y = make_float2(rcp_approx(sr.x), rcp_approx(sr.y));
+          m = __fmul2_rn(__fmul2_rn(__ffma2_rn(__fmul2_rn(h2, y), y, y), ri), ri2);
+        } else {
+          const float2 sig2 = make_float2(X.h + p.w, Y.h + p.w);
+          const float2 sr = __fadd2_rn(r2, sig2);
+          const float2 y = make_float2(rcp_approx(sr.x), rcp_approx(sr.y));
+          const float2 ph = __ffma2_rn(__fmul2_rn(__fmul2_rn(half2, sig2), y), y, y);
+          m = __fmul2_rn(__fmul2_rn(__fmul2_rn(ph, sig2), ri), ri2);
+        }
+        const float2 g = __fmul2_rn(__fmul2_rn(m, ri2), make_float2(far_t(X, s, e), far_t(Y, s, e)));
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float gq = q ? g.y : g.x, ex = q ? dx.y : dx.x, ey = q ? dy.y : dy.x, ez = q ? dz.y : dz.x;
+          Sums9 &c = a[r + q];
+          add_wq(T[r + q], s, e, q ? m.y : m.x, c, b);
+          c.gx = fmaf(gq, ex, c.gx);
+          c.gy = fmaf(gq, ey, c.gy);
+          c.gz = fmaf(gq, ez, c.gz);
+          b.gx = fmaf(gq, ex, b.gx);
+          b.gy = fmaf(gq, ey, b.gy);
+          b.gz = fmaf(gq, ez, b.gz);
+        }
+      }
+      const int k = kk + u;
+      rotate(b, (k ^ (k + 1)) & 31);
+    }
+  }
+}
+
+// FP32 far sums of one particle into its six FP64 sums acc[k * stride]:
+// u += As2 (Q x x' - W), dalpha += alpha x (As2 Q) + g3 G, with alpha = hi + lo.
+__device__ __forceinline__ void fold_far(const Sums9 &s, float x, float y, float z, float ax, float ay,
+                                         float az, float lx, float ly, float lz, double As2, double g3,
+                                         double *acc, int stride) {
+  const double Qx = As2 * s.qx, Qy = As2 * s.qy, Qz = As2 * s.qz;
+  const double xp = x, yp = y, zp = z;
+  const double px = (double)ax + (double)lx, py = (double)ay + (double)ly, pz = (double)az + (double)lz;
+  acc[0] += (Qy * zp - Qz * yp) - As2 * s.wx;
+  acc[stride] += (Qz * xp - Qx * zp) - As2 * s.wy;
+  acc[2 * stride] += (Qx * yp - Qy * xp) - As2 * s.wz;
+  acc[3 * stride] += (py * Qz - pz * Qy) + g3 * s.gx;
+  acc[4 * stride] += (pz * Qx - px * Qz) + g3 * s.gy;
+  acc[5 * stride] += (px * Qy - py * Qx) + g3 * s.gz;
+}
+
+// A far tile pair: sub-blocks [k0, k1) of 32 sources of tile J against all
+// targets of tile I, R per lane and pass.  accI: the warp's [6][128] target
+// sums; accJ: [6][128] source sums of tile J.
+template <int CLS, bool UNI, bool DIFF, int KERN, int R>
+__device__ __forceinline__ void far_pair(const SymSeg &sg, int I, int J, int k0, int k1, float cx,
+                                         float cy, float cz, float hu, const Stage &st, int lane,
+                                         double *accI, double *accJ) {
+  const double As2 = UNI ? kInv4Pi * 2.0 * (double)hu : kInv4Pi;
+  const float kap = (CLS == FAR_Z && DIFF) ? (float)(UNI ? 80.0 * sg.nu / (double)hu : 5.0 * sg.nu) : 0.f;
+  const float4 *__restrict__ pos = sg.pos32;
+  const float4 *__restrict__ vor = sg.vor32;
+  const float4 *__restrict__ vlo = sg.vorlo;
+  const int n = sg.n;
+#pragma unroll 1
+  for (int t0 = 0; t0 < kT; t0 += 32 * R) {
+    FarTarget T[R];
+    Sums9 a[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int i = I * kT + t0 + 32 * r + lane;
+      T[r] = FarTarget{kPadTarget, kPadTarget, kPadTarget, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 1.f, 0.f};
+      if (i < n) {
+        const float4 p = __ldg(pos + i), q = __ldg(vor + i);
+        const float x = p.x - cx, y = p.y - cy, z = p.z - cz;
+        T[r] = FarTarget{x, y, z, q.x, q.y, q.z, fmaf(q.y, z, -q.z * y), fmaf(q.z, x, -q.x * z),
+                         fmaf(q.x, y, -q.y * x), p.w, q.w};
+      }
+      a[r] = Sums9{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    }
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k) {
+      const int j = J * kT + 32 * k + lane;
+      float4 p = make_float4(kPadSource, kPadSource, kPadSource, 1.f), q = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 l = q, e = q;
+      if (j < n) {
+        p = __ldg(pos + j);
+        q = __ldg(vor + j);
+        l = __ldg(vlo + j);
+        p.x -= cx;
+        p.y -= cy;
+        p.z -= cz;
+        e = make_float4(fmaf(q.y, p.z, -q.z * p.y), fmaf(q.z, p.x, -q.x * p.z), fmaf(q.x, p.y, -q.y * p.x), 0.f);
+      }
+      e.w = l.x;
+      st.s0[lane] = p;
+      st.s1[lane] = q;
+      st.s2[lane] = e;
+      st.s3[lane] = make_float2(l.y, l.z);
+      __syncwarp();
+      Sums9 b{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if constexpr (CLS == FAR_Z)
+        far_block_z<UNI, DIFF, KERN, R>(st, lane, T, hu, kap, a, b);
+      else
+        far_block<CLS, UNI, KERN, R>(st, lane, T, hu, a, b);
+      const float4 pj = st.s0[lane], qj = st.s1[lane], ej = st.s2[lane];
+      const float2 lj = st.s3[lane];
+      fold_far(b, pj.x, pj.y, pj.z, qj.x, qj.y, qj.z, ej.w, lj.x, lj.y, As2, -3.0 * As2,
+               accJ + 32 * k + lane, kT);
+      __syncwarp();
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int i = I * kT + t0 + 32 * r + lane;
+      const float4 l = i < n ? __ldg(vlo + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      fold_far(a[r], T[r].x, T[r].y, T[r].z, T[r].ax, T[r].ay, T[r].az, l.x, l.y, l.z, As2, 3.0 * As2,
+               accI + t0 + 32 * r + lane, kT);
+    }
+  }
+}
+
+struct NearTarget {
+  float xh, yh, zh, xl, yl, zl;  // position hi, lo
+  float ax, ay, az, lx, ly, lz;  // strength hi, lo
+  float iaa;                     // 1 / |alpha_hi|^2 (0 for alpha = 0)
+  float cx, cy, cz;              // alpha_lo x alpha_hi
+  float h, v;
+};
+
+struct Sums6 {
+  float ux, uy, uz, sx, sy, sz;
+};
+
+__device__ __forceinline__ void rotate(Sums6 &a, int m) {
+  a.ux = __shfl_xor_sync(kFull, a.ux, m);
+  a.uy = __shfl_xor_sync(kFull, a.uy, m);
+  a.uz = __shfl_xor_sync(kFull, a.uz, m);
+  a.sx = __shfl_xor_sync(kFull, a.sx, m);
+  a.sy = __shfl_xor_sync(kFull, a.sy, m);
+  a.sz = __shfl_xor_sync(kFull, a.sz, m);
+}
+
+// 32 sources of a near tile against R targets per lane.  DIAG: both tiles are
+// the same one, every ordered pair is visited and only the targets' sums are
+// kept; the pair of a particle with itself falls on step 0 of target `self`
+// (no target when it is outside 0..R-1).  kap: the diffusion factor in the
+// units of the s sums (15 nu, or 240 nu / h with one radius).
+template <bool UNI, bool DIAG, bool DIFF, int KERN, int R>
+__device__ __forceinline__ void near_block(const Stage &st, int lane, const NearTarget (&T)[R], int self,
+                                           float hu, float kap, Sums6 (&a)[R], Sums6 &b) {
+  const float s2u = 2.f * hu, c240 = -480.f * hu;
+#pragma unroll 1
+  for (int kk = 0; kk < 32; kk += 2) {
+    const int base = lane ^ kk;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      // (hi position, h), (lo position, volume), (strength, lo.x), (lo.y, lo.z)
+      const float4 p = st.s0[base ^ u], pl = st.s1[base ^ u], s = st.s2[base ^ u];
+      const float2 l = st.s3[base ^ u];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float dx = (T[r].xh - p.x) + (T[r].xl - pl.x);
+        const float dy = (T[r].yh - p.y) + (T[r].yl - pl.y);
+        const float dz = (T[r].zh - p.z) + (T[r].zl - pl.z);
+        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        const float ri = rsqrtf(r2);
+        float q, fh, dp;
+        if (KERN == KERNEL_GAUSSIAN)
+          gauss_scalars(T[r].h + p.w, r2, ri, q, fh, dp);
+        else if (UNI)
+          kernel_scalars_uniform(hu, c240, rsqrtf(r2 + s2u), ri, q, fh, dp);
+        else
+          kernel_scalars(T[r].h + p.w, rsqrtf(r2 + (T[r].h + p.w)), ri, q, fh, dp);
+        // alpha_j x d, and alpha_i x alpha_j from the hi/lo strengths
+        const float cx = fmaf(s.y, dz, -s.z * dy);
+        const float cy = fmaf(s.z, dx, -s.x * dz);
+        const float cz = fmaf(s.x, dy, -s.y * dx);
+        float wx, wy, wz;
+        projection_cross(T[r].ax, T[r].ay, T[r].az, T[r].iaa, T[r].cx, T[r].cy, T[r].cz, s.x, s.y, s.z,
+                         s.w, l.x, l.y, wx, wy, wz);
+        const float t = fmaf(dz, wz, fmaf(dy, wy, dx * wx));
+        const float ft = 3.0f * fh * t;
+        float sx = fmaf(ft, dx, q * wx);
+        float sy = fmaf(ft, dy, q * wy);
+        float sz = fmaf(ft, dz, q * wz);
+        if (DIFF) {
+          const float kd = kap * dp, dv = T[r].v - pl.w;
+          const float ex = (s.x - T[r].ax) + (s.w - T[r].lx);
+          const float ey = (s.y - T[r].ay) + (l.x - T[r].ly);
+          const float ez = (s.z - T[r].az) + (l.y - T[r].lz);
+          sx = fmaf(kd, fmaf(T[r].v, ex, dv * T[r].ax), sx);
+          sy = fmaf(kd, fmaf(T[r].v, ey, dv * T[r].ay), sy);
+          sz = fmaf(kd, fmaf(T[r].v, ez, dv * T[r].az), sz);
+        }
+        if (DIAG && u == 0) {
+          const bool own = kk == 0 && r == self;
+          q = own ? 0.f : q;
+          sx = own ? 0.f : sx;
+          sy = own ? 0.f : sy;
+          sz = own ? 0.f : sz;
+        }
+        a[r].ux = fmaf(q, cx, a[r].ux);
+        a[r].uy = fmaf(q, cy, a[r].uy);
+        a[r].uz = fmaf(q, cz, a[r].uz);
+        a[r].sx += sx;
+        a[r].sy += sy;
+        a[r].sz += sz;
+        if (!DIAG) {
+          // alpha_i x d; subtracted at the fold
+          b.ux = fmaf(q, fmaf(T[r].ay, dz, -T[r].az * dy), b.ux);
+          b.uy = fmaf(q, fmaf(T[r].az, dx, -T[r].ax * dz), b.uy);
+          b.uz = fmaf(q, fmaf(T[r].ax, dy, -T[r].ay * dx), b.uz);
+          b.sx += sx;
+          b.sy += sy;
+          b.sz += sz;
+        }
+      }
+      const int k = kk + u;
+      if (!DIAG) rotate(b, (k ^ (k + 1)) & 31);
+    }
+  }
+}
+
+__device__ __forceinline__ void fold_near(const Sums6 &s, double As2, double *acc, int stride) {
+  acc[0] += As2 * s.ux;
+  acc[stride] += As2 * s.uy;
+  acc[2 * stride] += As2 * s.uz;
+  acc[3 * stride] += As2 * s.sx;
+  acc[4 * stride] += As2 * s.sy;
+  acc[5 * stride] += As2 * s.sz;
+}
+
+template <bool UNI, bool DIAG, bool DIFF, int KERN>
+__device__ __forceinline__ void near_pair(const SymSeg &sg, int I, int J, int k0, int k1, float hu,
+                                          const Stage &st, int lane, double *accI, double *accJ) {
+  constexpr int R = 2;
+  const double As2 = UNI ? kInv4Pi * 2.0 * (double)hu : kInv4Pi;
+  const float kap = DIFF ? (float)(UNI ? 240.0 * sg.nu / (double)hu : 15.0 * sg.nu) : 0.f;
+  const int n = sg.n;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+  for (int t0 = 0; t0 < kT; t0 += 32 * R) {
+    NearTarget T[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int i = I * kT + t0 + 32 * r + lane;
+      float4 p = make_float4(kPadTarget, kPadTarget, kPadTarget, 1.f), pl = zero, q = zero, l = zero;
+      if (i < n) {
+        p = __ldg(sg.pos32 + i);
+        pl = __ldg(sg.poslo + i);
+        q = __ldg(sg.vor32 + i);
+        l = __ldg(sg.vorlo + i);
+      }
+      const float aa = fmaf(q.z, q.z, fmaf(q.y, q.y, q.x * q.x));
+      T[r] = NearTarget{p.x, p.y, p.z, pl.x, pl.y, pl.z, q.x, q.y, q.z, l.x, l.y, l.z,
+                        aa > 0.f ? 1.0f / aa : 0.f, fmaf(l.y, q.z, -l.z * q.y),
+                        fmaf(l.z, q.x, -l.x * q.z), fmaf(l.x, q.y, -l.y * q.x), p.w, q.w};
+    }
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k) {
+      const int j = J * kT + 32 * k + lane;
+      float4 p = make_float4(kPadSource, kPadSource, kPadSource, 1.f), pl = zero, q = zero, l = zero;
+      if (j < n) {
+        p = __ldg(sg.pos32 + j);
+        pl = __ldg(sg.poslo + j);
+        q = __ldg(sg.vor32 + j);
+        l = __ldg(sg.vorlo + j);
+      }
+      st.s0[lane] = p;
+      st.s1[lane] = make_float4(pl.x, pl.y, pl.z, q.w);
+      st.s2[lane] = make_float4(q.x, q.y, q.z, l.x);
+      st.s3[lane] = make_float2(l.y, l.z);
+      __syncwarp();
+      Sums6 a[R], b{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int r = 0; r < R; ++r) a[r] = b;
+      near_block<UNI, DIAG, DIFF, KERN, R>(st, lane, T, k - t0 / 32, hu, kap, a, b);
+#pragma unroll
+      for (int r = 0; r < R; ++r) fold_near(a[r], As2, accI + t0 + 32 * r + lane, kT);
+      if (!DIAG) fold_near(b, -As2, accJ + 32 * k + lane, kT);
+      __syncwarp();
+    }
+  }
+}
+
+// One tile pair (I <= J), sub-blocks [k0, k1) of J's sources, in the class that
+// the two tiles' boxes allow.  The classes and their bounds are pair_f32.cu's;
+// the far formulation is centred on the smaller of the two boxes, whose
+// half-diagonal bounds |x'_i| + |x'_j| by 3 |d| for every pair.
+template <bool DIFF, int KERN>
+__device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, const Stage &st,
+                                          int lane, double *accI, double *accJ) {
+  const float4 alo = __ldg(sg.boxes + 2 * I), ahi = __ldg(sg.boxes + 2 * I + 1);
+  const float4 blo = __ldg(sg.boxes + 2 * J), bhi = __ldg(sg.boxes + 2 * J + 1);
+  const bool uni = KERN == KERNEL_HIGHORDER && alo.w == ahi.w && blo.w == bhi.w && alo.w == blo.w;
+  const float hu = alo.w;
+  if (I == J) {
+    if (uni)
+      near_pair<true, true, DIFF, KERN>(sg, I, J, k0, k1, hu, st, lane, accI, accJ);
+    else
+      near_pair<false, true, DIFF, KERN>(sg, I, J, k0, k1, hu, st, lane, accI, accJ);
+    return;
+  }
+  const float gap2 = box_gap2(alo, ahi, blo, bhi);
+  const float da = box_half_diag2(alo, ahi), db = box_half_diag2(blo, bhi);
+  const bool first = da < db;
+  const bool far = gap2 > 0.f && gap2 >= sg.near2 && gap2 >= (first ? da : db);
+  if (!far) {
+    if (uni)
+      near_pair<true, false, DIFF, KERN>(sg, I, J, k0, k1, hu, st, lane, accI, accJ);
+    else
+      near_pair<false, false, DIFF, KERN>(sg, I, J, k0, k1, hu, st, lane, accI, accJ);
+    return;
+  }
+  const float4 lo = first ? alo : blo, hi = first ? ahi : bhi;
+  const float cx = 0.5f * (lo.x + hi.x), cy = 0.5f * (lo.y + hi.y), cz = 0.5f * (lo.z + hi.z);
+  const float sig2max = ahi.w + bhi.w;
+  if (KERN == KERNEL_GAUSSIAN) {
+    if (gap2 >= 49.f * sig2max)
+      far_pair<FAR_SER, false, DIFF, KERN, 4>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+    else
+      far_pair<FAR_Z, false, DIFF, KERN, 2>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+    return;
+  }
+  if (gap2 >= 256.f * sig2max) {
+    if (uni)
+      far_pair<FAR_SER, true, DIFF, KERN, 4>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+    else
+      far_pair<FAR_SER, false, DIFF, KERN, 4>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+  } else if (gap2 >= 36.f * sig2max) {
+    if (uni)
+      far_pair<FAR_NZ, true, DIFF, KERN, 4>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+    else
+      far_pair<FAR_NZ, false, DIFF, KERN, 4>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+  } else {
+    if (uni)
+      far_pair<FAR_Z, true, DIFF, KERN, 2>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+    else
+      far_pair<FAR_Z, false, DIFF, KERN, 2>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+  }
+}
+
+// Large systems: item = group a of four tiles against the groups [b0, b1).
+template <bool DIFF, int KERN>
+__global__ void __launch_bounds__(kThreads, kBlocks)
+    sym_f32_group_kernel(const SymItem *__restrict__ items, const SymSeg *__restrict__ segs,
+                         const int *__restrict__ jbase, double *__restrict__ slots) {
+  extern __shared__ float4 smem_sym[];
+  double *const accI = reinterpret_cast<double *>(smem_sym);  // [4 warps][6][128]
+  double *const accJ = accI + kWarps * 6 * kT;                // [4 tiles][6][128]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const Stage st = stage_of(reinterpret_cast<char *>(accJ + kWarps * 6 * kT) + warp * kStageBytes);
+  const SymItem it = items[blockIdx.x];
+  const SymSeg &sg = segs[it.seg];
+  const int nt = (sg.n + kT - 1) / kT;
+  for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accI[q] = 0.0;
+  for (int b = it.b0; b < it.b1; ++b) {
+    for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accJ[q] = 0.0;
+    __syncthreads();
+    for (int r = 0; r < kWarps; ++r) {
+      const int c = (warp + r) & 3;
+      const int I = it.a * kWarps + warp, J = b * kWarps + c;
+      // inside one group: each unordered tile pair once (rounds 0, 1 and half of 2)
+      const bool mine = b > it.a || r < 2 || (r == 2 && warp < 2);
+      if (mine && I < nt && J < nt)
+        tile_pair<DIFF, KERN>(sg, min(I, J), max(I, J), 0, 4, st, lane,
+                              (I <= J ? accI + warp * 6 * kT : accJ + c * 6 * kT),
+                              (I <= J ? accJ + c * 6 * kT : accI + warp * 6 * kT));
+      __syncthreads();
+    }
+    if (b == it.a) {
+      for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accI[q] += accJ[q];
+    } else {
+      const int jb = jbase[it.jb + b];
+      if (jb >= 0) {
+        double *out = slots + ((size_t)jb + it.a - it.row0) * kWarps * 6 * kT;
+        for (int q = tid; q < kWarps * 6 * kT; q += kThreads) out[q] = accJ[q];
+      }
+    }
+    __syncthreads();
+  }
+  if (it.islot >= 0) {
+    double *out = slots + (size_t)it.islot * kWarps * 6 * kT;
+    for (int q = tid; q < kWarps * 6 * kT; q += kThreads) out[q] = accI[q];
+  }
+}
+
+// Small systems: item = one tile pair (a, b0); each warp 32 sources of tile b0.
+template <bool DIFF, int KERN>
+__global__ void __launch_bounds__(kThreads, kBlocks)
+    sym_f32_tile_kernel(const SymItem *__restrict__ items, const SymSeg *__restrict__ segs,
+                        const int *__restrict__ jbase, double *__restrict__ slots) {
+  extern __shared__ float4 smem_sym[];
+  double *const accI = reinterpret_cast<double *>(smem_sym);  // [4 warps][6][128]
+  double *const accJ = accI + kWarps * 6 * kT;                // [6][128]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const Stage st = stage_of(reinterpret_cast<char *>(accJ + 6 * kT) + warp * kStageBytes);
+  const SymItem it = items[blockIdx.x];
+  const SymSeg &sg = segs[it.seg];
+  double *const mine = accI + warp * 6 * kT;
+#pragma unroll
+  for (int q = 0; q < 24; ++q) mine[32 * q + lane] = 0.0;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) accJ[k * kT + tid] = 0.0;
+  tile_pair<DIFF, KERN>(sg, it.a, it.b0, warp, warp + 1, st, lane, mine, accJ);
+  if (it.b0 > it.a) {
+    const int jb = jbase[it.jb + it.b0];
+    if (jb >= 0) {
+      double *out = slots + ((size_t)jb + it.a) * 6 * kT;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) out[k * kT + tid] = accJ[k * kT + tid];
+    }
+  }
+  __syncthreads();
+  if (it.islot >= 0) {
+    double *out = slots + (size_t)it.islot * 6 * kT;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int q = k * kT + tid;
+      out[q] = ((accI[q] + accI[6 * kT + q]) + accI[12 * kT + q]) + accI[18 * kT + q];
+    }
+  }
+}
+
+// One block per tile: thread (k, q) sums component k of particle q over the
+// tile's slots in slot order.  HBM- or L2-bound reads of 6 KB rows, eight in
+// flight per thread.
+__global__ void __launch_bounds__(6 * kT)
+    sym_sums_kernel(const SymSum *__restrict__ sums, const SymSeg *__restrict__ segs,
+                    const double *__restrict__ slots) {
+  const SymSum s = sums[blockIdx.x];
+  const SymSeg &sg = segs[s.seg];
+  const int k = threadIdx.x / kT, i = s.t * kT + threadIdx.x % kT;
+  if (i >= sg.n) return;
+  const double *p = slots + s.first + threadIdx.x;
+  double *out = sg.rates + (size_t)k * sg.n + i;
+  double r = s.add ? *out : 0.0;
+  int c = 0;
+  for (; c + 8 <= s.count; c += 8) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = __ldcs(p + (size_t)(c + u) * s.stride);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) r += v[u];
+  }
+  for (; c < s.count; ++c) r += __ldcs(p + (size_t)c * s.stride);
+  *out = r;
+}
+
+using KernelFn = void (*)(const SymItem *, const SymSeg *, const int *, double *);
+
+KernelFn select(bool group, bool diffusion, int kernel) {
+  if (kernel == KERNEL_GAUSSIAN) {
+    if (group)
+      return diffusion ? &sym_f32_group_kernel<true, KERNEL_GAUSSIAN> : &sym_f32_group_kernel<false, KERNEL_GAUSSIAN>;
+    return diffusion ? &sym_f32_tile_kernel<true, KERNEL_GAUSSIAN> : &sym_f32_tile_kernel<false, KERNEL_GAUSSIAN>;
+  }
+  if (group)
+    return diffusion ? &sym_f32_group_kernel<true, KERNEL_HIGHORDER> : &sym_f32_group_kernel<false, KERNEL_HIGHORDER>;
+  return diffusion ? &sym_f32_tile_kernel<true, KERNEL_HIGHORDER> : &sym_f32_tile_kernel<false, KERNEL_HIGHORDER>;
+}
+
+size_t smem_bytes(bool group) {
+  const size_t acc = (size_t)kWarps * 6 * kT * sizeof(double);
+  return acc + (group ? acc : acc / kWarps) + (size_t)kWarps * kStageBytes;
+}
+
+// Opts a kernel in to its dynamic shared memory beyond the default 48 KB (once
+// per kernel and device).
+cudaError_t prepare(KernelFn f, size_t bytes) {
+  static std::mutex mu;
+  static std::set<std::pair<int, KernelFn>> done;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(mu);
+  if (done.count({dev, f})) return cudaSuccess;
+  e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) done.insert({dev, f});
+  return e;
+}
+
+}  // namespace
+
+cudaError_t sym_f32_occupancy(bool group, bool diffusion, int kernel, int *blocks_per_sm) {
+  KernelFn f = select(group, diffusion, kernel);
+  const size_t bytes = smem_bytes(group);
+  cudaError_t e = prepare(f, bytes);
+  if (e != cudaSuccess) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, kThreads, bytes);
+}
+
+cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
+                           const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
+  if (n_items <= 0) return cudaSuccess;
+  KernelFn f = select(group, diffusion, kernel);
+  const size_t bytes = smem_bytes(group);
+  cudaError_t e = prepare(f, bytes);
+  if (e != cudaSuccess) return e;
+  f<<<n_items, kThreads, bytes, s>>>(items, segs, jbase, slots);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const SymSeg *segs, const double *slots,
+                            cudaStream_t s) {
+  if (n_sums <= 0) return cudaSuccess;
+  sym_sums_kernel<<<n_sums, 6 * kT, 0, s>>>(sums, segs, slots);
+  return cudaGetLastError();
+}
+
+}  // namespace pawan

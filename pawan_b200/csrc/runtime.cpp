@@ -30,12 +30,10 @@ int cuda_fail(pawan_ctx *ctx, cudaError_t e, const char *where) {
   return fail(ctx, PAWAN_ERR_CUDA, m);
 }
 
-// Defaults measured on the ring pair and the helical wake (N = 131,072 and
-// 262,144): two targets per thread, 256 threads, shallow unroll, fine chunks.
 TileChoice default_tile(int precision) {
   TileChoice t;
   if (precision == PAWAN_PREC_F32) {
-    t.pc = PairConfig{128, 1, 4, 1, 0, 2};  // packed far path, unroll 4
+    t.pc = PairConfig{128, 1, 4, 1, 0, 2};  // the symmetric engine
   } else {
     t.pc = PairConfig{128, 1, 1};
   }
@@ -46,11 +44,9 @@ TileChoice default_tile(int precision) {
 std::vector<TileChoice> tile_candidates(int precision, int kernel) {
   std::vector<TileChoice> v;
   if (precision == PAWAN_PREC_F32) {
-    // (threads per target, targets per thread, unroll, blocks per SM) as
-    // compiled in pair_f32.cu (0 = the default register bound)
-    // (.., packed) among those compiled in pair_f32.cu: the ones that led on
-    // some workload (threads per target > 1 for small systems, two targets
-    // per thread or packed pairs for large ones)
+    // (threads per target, targets per thread, unroll, blocks per SM, packed):
+    // the scalar tilings as compiled in pair_f32.cu (0 = the default register
+    // bound), the packed ones all the symmetric engine's
     const int shapes[][5] = {{1, 1, 4, 0, 0}, {2, 1, 4, 0, 0}, {4, 1, 4, 0, 0}, {1, 2, 1, 0, 0},
                              {1, 2, 2, 0, 0}, {1, 1, 4, 5, 0}, {1, 1, 1, 0, 1}, {1, 1, 2, 0, 1},
                              {1, 1, 4, 0, 1}, {1, 1, 2, 5, 1}, {1, 1, 2, 0, 2}, {1, 1, 4, 0, 2}};
@@ -60,9 +56,6 @@ std::vector<TileChoice> tile_candidates(int precision, int kernel) {
         t.pc = PairConfig{tb, sh[0], sh[2], sh[1], sh[3], sh[4]};
         if (pairs_f32_supported(t.pc, kernel)) v.push_back(t);
       }
-    // the packed unroll-4 shapes again with a separate near pass, scalar (1) or
-    // packed (2) (ahead where near tile pairs are many: ragged batches of small
-    // rings, scrambled states)
     for (int split : {1, 2})
       for (int tb : {128, 256})
         for (int pk : {1, 2}) {
@@ -90,6 +83,10 @@ bool Plan::stale() const {
     if (systems[s]->nu != nus[s] || systems[s]->geometry_version != geometry_versions[s])
       return true;
   return false;
+}
+
+bool tile_symmetric(int precision, const PairConfig &pc) {
+  return precision == PAWAN_PREC_F32 && pc.packed > 0;
 }
 
 static int occupancy(pawan_ctx *ctx, int precision, const PairConfig &pc, bool diffusion,
@@ -120,6 +117,205 @@ static size_t shard_first(const pawan_system *y) { return (size_t)y->shard.rank 
 static size_t shard_count(const pawan_system *y) {
   const size_t f = shard_first(y);
   return f >= y->n ? 0 : std::min(y->shard.size, y->n - f);
+}
+
+// ---- symmetric pair engine: work decomposition ----
+// A system of up to kSymTilesMax tiles is covered by single tile pairs (enough
+// blocks to fill the device from a few thousand particles on), a larger one by
+// groups of kSymGroup tiles, whose sums are written once per four tile pairs.
+constexpr int kSymTilesMax = 256;
+// Bound on one system's slots: the rows of groups are processed in phases, the
+// slots of a phase summed into the rates before the next reuses them.  The
+// serving engine holds many systems at a time, so its bound is smaller.
+constexpr double kSymSlotBytes = 2.0e9, kSymSlotBytesServing = 4.0e8;
+
+namespace {
+
+// The decomposition of one system: groups of g tiles, the runs of column groups
+// per row, and the phases' row ranges [rows[p], rows[p + 1]).
+struct SymLayout {
+  int g = 1, ng = 0, run = 1;
+  std::vector<int> rows;
+  int runs(int a) const { return (ng - a + run - 1) / run; }
+  // slots of group t in the phase of rows [r0, r1)
+  int slots(int t, int r0, int r1) const {
+    return std::max(0, std::min(t, r1) - r0) + (t >= r0 && t < r1 ? runs(t) : 0);
+  }
+};
+
+SymLayout sym_layout(size_t n, int items_per_slot, double bytes) {
+  SymLayout l;
+  const int nt = (int)((n + kSymTile - 1) / kSymTile);
+  l.g = nt <= kSymTilesMax ? 1 : kSymGroup;
+  l.ng = (nt + l.g - 1) / l.g;
+  if (l.g > 1) {
+    // longer runs write fewer target-side sums; at least some dozens of items
+    // per resident block (444 of them) keep the last ones from trailing
+    const double pairs = 0.5 * (double)l.ng * (double)(l.ng + 1);
+    l.run = std::max(1, std::min(4, (int)(pairs / (444.0 * std::max(1, items_per_slot)))));
+  }
+  const double slot = 48.0 * kSymTile * l.g;
+  l.rows.push_back(0);
+  if (l.g == 1) {
+    l.rows.push_back(l.ng);
+    return l;
+  }
+  int r0 = 0;
+  while (r0 < l.ng) {
+    int r1 = r0;
+    double used = 0.0;  // row a adds its runs and one slot per later group
+    while (r1 < l.ng) {
+      const double more = slot * (double)(l.runs(r1) + l.ng - 1 - r1);
+      if (r1 > r0 && used + more > bytes) break;
+      used += more;
+      ++r1;
+    }
+    l.rows.push_back(r1);
+    r0 = r1;
+  }
+  return l;
+}
+
+}  // namespace
+
+double sym_slot_bytes(size_t n, bool serving) {
+  const SymLayout l = sym_layout(n, 32, serving ? kSymSlotBytesServing : kSymSlotBytes);
+  double most = 0.0;
+  for (size_t p = 0; p + 1 < l.rows.size(); ++p) {
+    double c = 0.0;
+    for (int t = 0; t < l.ng; ++t) c += l.slots(t, l.rows[p], l.rows[p + 1]);
+    most = std::max(most, c);
+  }
+  return most * 48.0 * kSymTile * l.g;
+}
+
+// Items, slots and sums of a plan on the symmetric engine.  A system's
+// decomposition depends on its own size and the tiling only, so its arithmetic
+// does not depend on the other systems of the plan.
+static int build_sym_work(pawan_ctx *ctx, Plan &p, bool serving) {
+  struct Costed {
+    SymItem w;
+    double cost;
+    int late;  // 0: holds tile pairs next to the diagonal (near ones, which take longest)
+  };
+  std::vector<SymLayout> lay;
+  size_t n_phases = 0;
+  for (auto *y : p.systems) {
+    lay.push_back(sym_layout(y->n, p.tile.items_per_slot, serving ? kSymSlotBytesServing : kSymSlotBytes));
+    n_phases = std::max(n_phases, lay.back().rows.size() - 1);
+  }
+  // systems with the most tiles first
+  std::vector<size_t> order(p.systems.size());
+  std::iota(order.begin(), order.end(), (size_t)0);
+  std::stable_sort(order.begin(), order.end(),
+                   [&](size_t a, size_t b) { return p.systems[a]->n > p.systems[b]->n; });
+  std::vector<SymItem> items;
+  std::vector<SymSum> sums;
+  std::vector<int> jbase;
+  size_t group_slots = 0, tile_slots = 0;  // most doubles of any phase
+  std::vector<std::vector<SymSum>> tile_sums(n_phases);
+  p.phases.assign(n_phases, Plan::Phase{});
+  for (size_t ph = 0; ph < n_phases; ++ph) {
+    Plan::Phase &P = p.phases[ph];
+    P.sum0 = (int)sums.size();
+    size_t used[2] = {0, 0};  // slots so far: single-tile systems, grouped ones
+    std::vector<Costed> mine[2];
+    std::vector<SymSum> of_tiles;
+    for (size_t s : order) {
+      const SymLayout &l = lay[s];
+      if (ph + 1 >= l.rows.size()) continue;
+      const pawan_system *y = p.systems[s];
+      const int grouped = l.g > 1 ? 1 : 0, per = kSymTile * l.g;
+      const int n = (int)y->n, nt = (n + kSymTile - 1) / kSymTile;
+      const int r0 = l.rows[ph], r1 = l.rows[ph + 1];
+      // groups whose particles this process computes (all of them when the
+      // system is not sharded; block starts are multiples of a group)
+      const int f = y->shard.active ? (int)shard_first(y) : 0;
+      const int e = y->shard.active ? f + (int)shard_count(y) : n;
+      auto owned = [&](int t) { return t * per < e && (t + 1) * per > f; };
+      auto particles = [&](int t) { return (double)(std::min(n, (t + 1) * per) - t * per); };
+      const int jb = (int)jbase.size();
+      std::vector<int> i0(l.ng, -1);
+      for (int t = 0; t < l.ng; ++t) {
+        const int c = l.slots(t, r0, r1);
+        if (!owned(t) || c == 0) {
+          jbase.push_back(-1);
+          continue;
+        }
+        const size_t first = used[grouped];
+        used[grouped] += (size_t)c;
+        if (used[grouped] > (size_t)INT32_MAX / 2) return fail(ctx, PAWAN_ERR_INVALID, "too many work items");
+        jbase.push_back(t > r0 ? (int)first : -1);
+        if (t >= r0 && t < r1) i0[t] = (int)first + (t - r0);
+        for (int q = 0; q < l.g && t * l.g + q < nt; ++q) {
+          const long long at = (long long)first * 6 * per + (long long)q * 6 * kSymTile;
+          (grouped ? sums : of_tiles).push_back(SymSum{at, 6 * per, c, (int)s, t * l.g + q, ph > 0 ? 1 : 0});
+        }
+      }
+      std::vector<Costed> late;
+      for (int a = r0; a < r1; ++a) {
+        int k = 0;
+        for (int b0 = a; b0 < l.ng; b0 += l.run, ++k) {
+          const int b1 = std::min(l.ng, b0 + l.run);
+          double cost = 0.0;  // interactions credited: ordered pairs of owned targets
+          bool any = owned(a);
+          for (int b = b0; b < b1; ++b) {
+            any = any || owned(b);
+            const double both = particles(a) * particles(b);
+            cost += (owned(a) ? both : 0.0) + (b != a && owned(b) ? both : 0.0);
+          }
+          if (!any) continue;
+          const Costed c{SymItem{(int)s, a, b0, b1, i0[a] < 0 ? -1 : i0[a] + k, r0, jb}, cost, 0};
+          if (b0 <= a + (l.g > 1 ? 1 : 2))
+            mine[grouped].push_back(c);
+          else
+            late.push_back(c);
+        }
+      }
+      mine[grouped].insert(mine[grouped].end(), late.begin(), late.end());
+    }
+    P.groups = (int)mine[1].size();
+    P.tiles = (int)mine[0].size();
+    for (int k : {1, 0})
+      for (const Costed &c : mine[k]) {
+        items.push_back(c.w);
+        p.item_costs.push_back(c.cost);
+      }
+    group_slots = std::max(group_slots, used[1] * 6 * kSymTile * kSymGroup);
+    tile_slots = std::max(tile_slots, used[0] * 6 * kSymTile);
+    tile_sums[ph] = of_tiles;
+    sums.insert(sums.end(), of_tiles.begin(), of_tiles.end());
+    P.sums = (int)sums.size() - P.sum0;
+  }
+  // the single-tile items' slots lie behind the groups'
+  for (size_t ph = 0; ph < n_phases; ++ph) {
+    const size_t k = tile_sums[ph].size(), at = (size_t)(p.phases[ph].sum0 + p.phases[ph].sums) - k;
+    for (size_t q = 0; q < k; ++q) sums[at + q].first += (long long)group_slots;
+  }
+  p.tile_slots = group_slots;
+  if (items.size() > (size_t)INT32_MAX) return fail(ctx, PAWAN_ERR_INVALID, "too many work items");
+  p.n_items = (int)items.size();
+  std::vector<SymSeg> segs;
+  for (size_t s = 0; s < p.systems.size(); ++s) {
+    const pawan_system *y = p.systems[s];
+    const StageDesc &g = p.stage_host[s];
+    segs.push_back(SymSeg{g.pos32, g.vor32, g.poslo, g.vorlo, g.pos64, g.vor64, g.boxes,
+                          const_cast<double *>(g.rates), (int)y->n, y->nu, (float)(y->r_near * y->r_near)});
+  }
+  PAWAN_CUDA(ctx, p.slots.alloc(group_slots + tile_slots));
+  PAWAN_CUDA(ctx, p.sym_items.alloc(items.size()));
+  PAWAN_CUDA(ctx, p.sym_segs.alloc(segs.size()));
+  PAWAN_CUDA(ctx, p.sym_jbase.alloc(jbase.size()));
+  PAWAN_CUDA(ctx, p.sym_sums.alloc(sums.size()));
+  PAWAN_CUDA(ctx, cudaMemcpyAsync(p.sym_items.p, items.data(), items.size() * sizeof(SymItem),
+                                  cudaMemcpyHostToDevice, ctx->stream));
+  PAWAN_CUDA(ctx, cudaMemcpyAsync(p.sym_segs.p, segs.data(), segs.size() * sizeof(SymSeg),
+                                  cudaMemcpyHostToDevice, ctx->stream));
+  PAWAN_CUDA(ctx, cudaMemcpyAsync(p.sym_jbase.p, jbase.data(), jbase.size() * sizeof(int),
+                                  cudaMemcpyHostToDevice, ctx->stream));
+  PAWAN_CUDA(ctx, cudaMemcpyAsync(p.sym_sums.p, sums.data(), sums.size() * sizeof(SymSum),
+                                  cudaMemcpyHostToDevice, ctx->stream));
+  return PAWAN_OK;
 }
 
 // Work decomposition.  Target tiles of tb/p particles; sources in chunks of
@@ -153,10 +349,16 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
     p->interactions += targets * (double)s->n;
   }
   int bps = 0;
-  PAWAN_TRY(occupancy(ctx, precision, tile.pc, p->diffusion, kernel, &bps));
+  p->sym = tile_symmetric(precision, tile.pc);
+  if (p->sym) {
+    cudaError_t e = sym_f32_occupancy(true, p->diffusion, kernel, &bps);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy query");
+  } else {
+    PAWAN_TRY(occupancy(ctx, precision, tile.pc, p->diffusion, kernel, &bps));
+  }
   p->grid = ctx->sm_count * bps;
-  const int TB = tile.pc.tb;
-  const int TPB = targets_per_block(tile.pc);
+  const int TB = p->sym ? kSymTile : tile.pc.tb;
+  const int TPB = p->sym ? kSymTile : targets_per_block(tile.pc);
   const double slots = (double)p->grid;
   const double target_pairs =
       std::max(p->interactions / (slots * std::max(1, tile.items_per_slot)), (double)TPB * TB);
@@ -169,8 +371,8 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
   // per system: partial slots [target tiles][chunks][6][TPB] (none with one
   // chunk), rates [6][n], one counter per target tile
   if (TPB % 8 != 0) return fail(ctx, PAWAN_ERR_INVALID, "targets per block must be a multiple of 8");
-  size_t partial_total = 0, box_total = 0, rates_total = 0, count_total = 0, slot_total = 0;
-  std::vector<size_t> partial_off(systems.size()), box_off(systems.size()), slot_off(systems.size());
+  size_t partial_total = 0, box_total = 0, rates_total = 0, count_total = 0;
+  std::vector<size_t> partial_off(systems.size()), box_off(systems.size());
   std::vector<size_t> rates_off(systems.size()), count_off(systems.size());
   std::vector<double> sys_cost(systems.size(), 0.0);
   p->nchunks.resize(systems.size());
@@ -181,13 +383,11 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
                               ? (fixed_chunk_sources + TB - 1) / TB
                               : (int)std::ceil(target_pairs / ((double)TPB * TB));
     tiles_per_chunk = std::max(1, std::min(tiles_per_chunk, src_tiles));
-    const int nch = (src_tiles + tiles_per_chunk - 1) / tiles_per_chunk;
+    const int nch = p->sym ? 1 : (src_tiles + tiles_per_chunk - 1) / tiles_per_chunk;
     p->nchunks[s] = nch;
     const size_t target_tiles = ((size_t)n + TPB - 1) / TPB;
     partial_off[s] = partial_total;
     if (nch > 1) partial_total += target_tiles * (size_t)nch * 6 * (size_t)TPB;
-    slot_off[s] = slot_total;  // item slots (target tile, chunk), for the near pass
-    slot_total += target_tiles * (size_t)nch;
     rates_off[s] = rates_total;
     rates_total += 6 * (size_t)n;
     count_off[s] = count_total;
@@ -202,7 +402,7 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
     // target-major: a target tile's chunks are consecutive, so they run at
     // about the same time and the block completing the tile finds their
     // partial slots still in L2
-    for (int t0 = t_lo; t0 < t_hi; t0 += TPB) {
+    for (int t0 = t_lo; t0 < t_hi && !p->sym; t0 += TPB) {
       const int nt = std::min(TPB, t_hi - t0);
       for (int c = 0; c < nch; ++c) {
         const int s0 = c * tiles_per_chunk * TB;
@@ -225,14 +425,17 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
     p->partial.ordered_on(ctx->stream);
     p->rates.ordered_on(ctx->stream);
     p->tile_count.ordered_on(ctx->stream);
-    p->near_partial.ordered_on(ctx->stream);
-    p->near_flag.ordered_on(ctx->stream);
     p->boxes.ordered_on(ctx->stream);
     p->items.ordered_on(ctx->stream);
     p->segs.ordered_on(ctx->stream);
     p->stage_items.ordered_on(ctx->stream);
     p->shard_items.ordered_on(ctx->stream);
     p->stage_descs.ordered_on(ctx->stream);
+    p->sym_items.ordered_on(ctx->stream);
+    p->sym_segs.ordered_on(ctx->stream);
+    p->sym_jbase.ordered_on(ctx->stream);
+    p->sym_sums.ordered_on(ctx->stream);
+    p->slots.ordered_on(ctx->stream);
   }
   PAWAN_CUDA(ctx, p->partial.alloc(partial_total));
   // the pair kernels discard the slots' L2 lines after summing them: every
@@ -242,10 +445,6 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
   PAWAN_CUDA(ctx, p->rates.alloc(rates_total));
   PAWAN_CUDA(ctx, p->tile_count.alloc(count_total));
   PAWAN_CUDA(ctx, cudaMemsetAsync(p->tile_count.p, 0, p->tile_count.bytes(), ctx->stream));
-  if (tile.pc.split > 0) {
-    PAWAN_CUDA(ctx, p->near_partial.alloc(slot_total * 6 * (size_t)TPB));
-    PAWAN_CUDA(ctx, p->near_flag.alloc(slot_total));
-  }
   PAWAN_CUDA(ctx, p->boxes.alloc(box_total));
   std::vector<WorkItem> wh(items.size());
   p->item_costs.resize(items.size());
@@ -269,8 +468,6 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
     d.partial = p->nchunks[s] > 1 ? p->partial.p + partial_off[s] : nullptr;
     d.rates = p->rates.p + rates_off[s];
     d.tile_count = p->tile_count.p + count_off[s];
-    d.near_partial = tile.pc.split > 0 ? p->near_partial.p + slot_off[s] * 6 * (size_t)TPB : nullptr;
-    d.near_flag = tile.pc.split > 0 ? p->near_flag.p + slot_off[s] : nullptr;
     d.n = (int)y->n;
     d.nchunks = p->nchunks[s];
     d.nu = y->nu;
@@ -310,12 +507,14 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
   p->n_stage_blocks = (int)sih.size();
   p->n_shard_blocks = (int)shh.size();
   p->dts.assign(systems.size(), 0.0);
+  if (p->sym) PAWAN_TRY(build_sym_work(ctx, *p, fixed_chunk_sources > 0));
   PAWAN_CUDA(ctx, p->items.alloc(wh.size()));
   PAWAN_CUDA(ctx, p->segs.alloc(sh.size()));
   PAWAN_CUDA(ctx, p->stage_items.alloc(sih.size()));
   PAWAN_CUDA(ctx, p->stage_descs.alloc(sh.size()));
-  PAWAN_CUDA(ctx, cudaMemcpyAsync(p->items.p, wh.data(), wh.size() * sizeof(WorkItem),
-                                  cudaMemcpyHostToDevice, ctx->stream));
+  if (!wh.empty())
+    PAWAN_CUDA(ctx, cudaMemcpyAsync(p->items.p, wh.data(), wh.size() * sizeof(WorkItem),
+                                    cudaMemcpyHostToDevice, ctx->stream));
   PAWAN_CUDA(ctx, cudaMemcpyAsync(p->segs.p, sh.data(), sh.size() * sizeof(SegDesc),
                                   cudaMemcpyHostToDevice, ctx->stream));
   PAWAN_CUDA(ctx, cudaMemcpyAsync(p->stage_items.p, sih.data(), sih.size() * sizeof(StageItem),
@@ -369,6 +568,29 @@ static cudaEvent_t take_event(pawan_ctx *ctx) {
   return e;
 }
 
+// Work items [first, first + count) of a plan on the symmetric engine, and the
+// slot sums of every phase whose last item is among them.
+static int launch_sym_range(pawan_ctx *ctx, Plan &p, int first, int count) {
+  int at = 0;
+  for (const Plan::Phase &ph : p.phases) {
+    for (bool group : {true, false}) {
+      const int n = group ? ph.groups : ph.tiles;
+      const int lo = std::max(first, at), hi = std::min(first + count, at + n);
+      at += n;
+      if (lo >= hi) continue;
+      double *slots = p.slots.p + (group ? 0 : p.tile_slots);
+      PAWAN_CUDA(ctx, launch_sym_f32(group, p.diffusion, p.kernel, p.sym_items.p + lo, hi - lo, p.sym_segs.p,
+                                     p.sym_jbase.p, slots, ctx->stream));
+      ctx->launches++;
+    }
+    if (at > first && at <= first + count) {
+      PAWAN_CUDA(ctx, launch_sym_sums(p.sym_sums.p + ph.sum0, ph.sums, p.sym_segs.p, p.slots.p, ctx->stream));
+      ctx->launches++;
+    }
+  }
+  return PAWAN_OK;
+}
+
 int launch_pairs(pawan_ctx *ctx, Plan &p, bool allow_events) {
   return launch_pairs_range(ctx, p, 0, p.n_items, allow_events);
 }
@@ -383,7 +605,7 @@ int launch_pairs_range(pawan_ctx *ctx, Plan &p, int first, int count, bool allow
       PAWAN_TRY(launch_stage_mode(ctx, p, STAGE_PACK));
       break;
     }
-  PAWAN_CUDA(ctx, cudaMemsetAsync(ctx->d_counter, 0, 2 * sizeof(int), ctx->stream));
+  if (!p.sym) PAWAN_CUDA(ctx, cudaMemsetAsync(ctx->d_counter, 0, sizeof(int), ctx->stream));
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (ctx->profile && allow_events) {
     e0 = take_event(ctx);
@@ -391,8 +613,10 @@ int launch_pairs_range(pawan_ctx *ctx, Plan &p, int first, int count, bool allow
     if (!e0 || !e1) return fail(ctx, PAWAN_ERR_CUDA, "cannot create profiling events");
     PAWAN_CUDA(ctx, cudaEventRecord(e0, ctx->stream));
   }
-  cudaError_t e;
-  if (p.precision == PAWAN_PREC_F32)
+  cudaError_t e = cudaSuccess;
+  if (p.sym)
+    PAWAN_TRY(launch_sym_range(ctx, p, first, count));
+  else if (p.precision == PAWAN_PREC_F32)
     e = launch_pairs_f32(p.tile.pc, p.diffusion, p.kernel, p.grid, items, count, p.segs.p,
                          ctx->d_counter, ctx->stream);
   else if (p.precision == PAWAN_PREC_F64)
@@ -402,7 +626,7 @@ int launch_pairs_range(pawan_ctx *ctx, Plan &p, int first, int count, bool allow
     e = launch_pairs_plain(p.tile.pc, p.kernel, p.grid, items, count, p.segs.p, ctx->d_counter,
                            ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "pair kernel launch");
-  ctx->launches++;
+  if (!p.sym) ctx->launches++;
   if (e0) {
     PAWAN_CUDA(ctx, cudaEventRecord(e1, ctx->stream));
     ctx->pending.push_back({e0, e1});
@@ -432,7 +656,7 @@ static double stage_bytes(const Plan &p, int mode) {
     const pawan_system *y = p.systems[s];
     const double n = (double)y->n;
     const double rates = 48.0;
-    const double pack = 16.0 + 128.0 + 32.0 / (double)p.tile.pc.tb;
+    const double pack = 16.0 + 128.0 + 32.0 / (double)p.stage_host[s].box_tile;
     double per = 0.0;
     switch (mode) {
       case STAGE_RATES: per = rates + 48.0; break;
@@ -505,6 +729,7 @@ int rk4_steps(pawan_ctx *ctx, Plan &p, size_t nsteps, bool use_graph) {
     int st = rk4_one_step(ctx, p, false);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
+    p.graph_kernels = ctx->launches.load() - before;
     ctx->launches = before;  // capture enqueues nothing; replays count below
     if (st != PAWAN_OK) {
       if (g) cudaGraphDestroy(g);
@@ -521,7 +746,7 @@ int rk4_steps(pawan_ctx *ctx, Plan &p, size_t nsteps, bool use_graph) {
         break;
       }
     PAWAN_CUDA(ctx, cudaGraphLaunch(p.graph_exec, ctx->stream));
-    ctx->launches += 8;
+    ctx->launches += p.graph_kernels;
     for (int st = 0; st < 4; ++st) note_repack(p);
   }
   return PAWAN_OK;
@@ -557,7 +782,14 @@ int autotune_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, in
     return PAWAN_OK;
   };
   // 1) tile shape at the default chunking, 2) chunking for the best shape.
-  for (const TileChoice &t : tile_candidates(precision, systems[0]->kernel)) {
+  bool sym_timed = false;
+  for (TileChoice t : tile_candidates(precision, systems[0]->kernel)) {
+    if (tile_symmetric(precision, t.pc)) {
+      // one engine behind all of them: timed once, as the default tiling
+      if (sym_timed) continue;
+      sym_timed = true;
+      t.pc = default_tile(precision).pc;
+    }
     double ms = 0;
     status = time_tile(t, &ms);
     if (status != PAWAN_OK) break;

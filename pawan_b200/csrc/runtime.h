@@ -169,8 +169,20 @@ struct Plan {
   DBuf<double> partial;   // per system [target tiles][chunks][6][tpb] (chunks > 1)
   DBuf<double> rates;     // per system [6][n]: the summed chunks
   DBuf<int> tile_count;   // per system and target tile; 0 between launches
-  DBuf<double> near_partial;        // split tilings: near sums per item slot (as partial)
-  DBuf<unsigned char> near_flag;    // split tilings: per item slot, whether it had near tiles
+  // symmetric pair engine (sym): items in launch order, by phase; the slots are
+  // reused from phase to phase, each summed into the rates at its end
+  bool sym = false;
+  struct Phase {
+    int groups = 0, tiles = 0;  // items over groups, then over single tile pairs
+    int sum0 = 0, sums = 0;     // its SymSum records
+  };
+  std::vector<Phase> phases;
+  DBuf<SymItem> sym_items;
+  DBuf<SymSeg> sym_segs;
+  DBuf<int> sym_jbase;
+  DBuf<SymSum> sym_sums;
+  DBuf<double> slots;
+  size_t tile_slots = 0;  // doubles before the slots of the single-tile items
   DBuf<float4> boxes;
   DBuf<WorkItem> items;
   DBuf<SegDesc> segs;
@@ -182,6 +194,7 @@ struct Plan {
   std::vector<double> dts;  // dt in the device stage table
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
+  unsigned long long graph_kernels = 0;  // kernels one replay launches
   ~Plan();
   bool stale() const;
 };
@@ -210,6 +223,12 @@ constexpr size_t kShardAlign = 512;
 
 // Whether a precision's kernels are compiled for a tiling and smoothing kernel.
 bool tile_supported(int precision, const PairConfig &pc, int kernel);
+
+// Whether a precision and tiling run on the symmetric pair engine (each
+// unordered pair once): the FP32 tilings with the packed far path.
+bool tile_symmetric(int precision, const PairConfig &pc);
+// Device bytes of the symmetric engine's slots for one system of n particles.
+double sym_slot_bytes(size_t n, bool serving);
 
 int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int precision,
                const TileChoice &tile, std::unique_ptr<Plan> &out, int fixed_chunk_sources = 0,

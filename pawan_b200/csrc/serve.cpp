@@ -24,9 +24,8 @@
 // turns at about one target of work per iteration.  Small requests
 // then keep their pace beside arbitrarily large ones, as with chunked
 // prefill in language-model serving.  Its result is unchanged, bit for bit:
-// every work item writes its own partial slot whichever launch runs it, and
-// a target tile's slots are summed in chunk order by the item that completes
-// the tile, in whichever launch that is.
+// every work item writes slots of its own whichever launch runs it, and the
+// slots are summed in a fixed order once the stage's last item is done.
 //
 // The engine's systems and plans take their device memory from the device's
 // memory pool in the order of the engine's stream (cudaMallocAsync /
@@ -34,9 +33,10 @@
 // device, and a request's particles are packed by the batched plan built
 // after its admission instead of a plan of its own.
 //
-// Sources are chunked in fixed-size chunks per request, so a request's
-// arithmetic does not depend on which other requests share its launches: its
-// result is the same alone and in the mix, bit for bit.
+// A request's work is decomposed by its own size alone (and, on the one-sided
+// kernels, its sources chunked in chunks of a fixed size), so its arithmetic
+// does not depend on which other requests share its launches: its result is
+// the same alone and in the mix, bit for bit.
 //
 // The engine owns its own context (stream, scheduler counter) on the device of
 // the context it was created from, so its worker never shares a stream with
@@ -87,23 +87,20 @@ struct Request {
 };
 
 // Device bytes a request holds while active: the system's buffers plus its
-// rates and partial slots in a batched plan (fixed chunk size; slots cover
-// whole target tiles of at most 512 particles).
-double request_bytes(size_t n, const TileChoice &tile) {
-  const int tb = tile.pc.tb;
+// rates and slots in a batched plan (the symmetric engine's, or partial slots
+// of a fixed chunk size that cover whole target tiles of at most 512 particles).
+double request_bytes(size_t n, int precision, const TileChoice &tile) {
   const double per = 5 * 48.0 + 16.0 + 4.0 + 64.0 + 64.0 + 1.0 + 48.0;
+  if (precision == PAWAN_PREC_F32 && tile_symmetric(precision, tile.pc))
+    return (double)n * per + sym_slot_bytes(n, true) + 4096.0;
+  const int tb = tile.pc.tb;
   const size_t chunk = ((kServeChunkSources + tb - 1) / tb) * (size_t)tb;
   const size_t nch = (n + chunk - 1) / chunk;
   const double slots = nch > 1 ? 48.0 * (double)(n + 512) * (double)nch : 0.0;
-  // a separate near pass keeps its sums in slots of its own (every chunk, one
-  // chunk included) with a flag byte each
-  const double near = tile.pc.split > 0 ? 49.0 * (double)(n + 512) * (double)nch : 0.0;
-  return (double)n * per + slots + near + 4096.0;
+  return (double)n * per + slots + 4096.0;
 }
 
-// The engine's tiling: for FP32 the packed far path with the packed near pass
-// (requests are rings of a few thousand to a few hundred thousand particles,
-// where the near tile pairs are a tenth of the work for the small ones); the
+// The engine's tiling: for FP32 one that the symmetric pair engine runs; the
 // library default otherwise.
 TileChoice serve_tile(int precision) {
   TileChoice t = default_tile(precision);
@@ -506,7 +503,7 @@ int pawan_server_submit(pawan_server *srv, size_t n_wakes, const size_t *num_par
   r->nu = nu;
   r->dt = dt;
   r->nsteps = nsteps;
-  r->bytes = request_bytes(n, srv->tile);
+  r->bytes = request_bytes(n, srv->cfg.precision, srv->tile);
   std::lock_guard<std::mutex> lk(srv->mu);
   r->id = srv->next_id++;
   r->t_submit = now_since(srv->t0);
