@@ -20,12 +20,18 @@
 // All calls share the one array, so calls whose kernels overlap on the GPU
 // (different streams, different host threads) race and must be serialised by
 // the caller.  Whatever must start at zero (the scheduler counter and the
-// per-tile counters) is cleared by the call itself; the rest is fully
-// overwritten before it is read.
+// per-tile counters) is cleared by the call itself, the count of finished
+// prepare blocks by the last of them (the array starts zeroed); the rest is
+// fully overwritten before it is read.
 //
 // The pair kernel is pawan_system_solve's in PAWAN_PREC_F32 with the
-// high-order smoothing kernel only, at a fixed tiling (128 threads, one
-// target per thread) and 4,096-source chunks.  The FP32 positions are taken
+// high-order smoothing kernel only, on the one-sided kernel (the symmetric
+// engine's slots would not fit the array).  The array holds 512 chunk slots of
+// 128 targets, so a system of t tiles is split into 512 / t source chunks, and
+// several threads share a target's sources (noalloc_config below): a few
+// thousand particles fill the device that way.  With one thread per target
+// and fixed chunks of 4,096 sources, one call at N = 4,096 ran 32 blocks for
+// 540 us, now 70 (N = 16,384: 560 us, now 513).  The FP32 positions are taken
 // relative to particle 0 (pawan_system_set_particles uses the centroid), and
 // the near-tile radius max(4 s_max, 0.03 x extent) measures the extent from
 // particle 0, so it can be up to twice the allocating path's: more tile pairs
@@ -44,10 +50,10 @@ namespace {
 
 constexpr int kNoallocMaxParticles = 16384;
 constexpr int kNaTB = 128;         // threads per block = sources per tile
-constexpr int kNaChunk = 4096;     // sources per work item
 constexpr int kNaMaxTiles = (kNoallocMaxParticles + kNaTB - 1) / kNaTB;
-constexpr int kNaMaxChunks = (kNoallocMaxParticles + kNaChunk - 1) / kNaChunk;
-constexpr int kNaMaxItems = kNaMaxTiles * kNaMaxChunks;
+constexpr int kNaSlots = 512;      // chunk slots of kNaTB targets
+constexpr int kNaMaxP = 4;         // most threads per target
+constexpr int kNaMaxItems = kNaSlots * kNaMaxP;
 constexpr int kNaPrepBlocks = (kNoallocMaxParticles + kStageThreads - 1) / kStageThreads;
 
 // Layout of the scratch array.  The kernels need 16-byte alignment of the
@@ -59,14 +65,37 @@ struct NoallocScratch {
   float4 poslo[kNoallocMaxParticles];
   float4 vorlo[kNoallocMaxParticles];
   float4 boxes[2 * kNaMaxTiles];
-  double partial[kNaMaxTiles * kNaMaxChunks * 6 * kNaTB];  // [tile][chunk][6][128]
+  double partial[kNaSlots * 6 * kNaTB];                    // [target tile][chunk][6][targets]
   double rates[6 * kNoallocMaxParticles];                  // [6][n]
   float block_max[2 * kNaPrepBlocks];  // per prepare block: max s, max |x - x0|^2
   WorkItem items[kNaMaxItems];
-  int tile_count[kNaMaxTiles];
+  int tile_count[kNaMaxTiles * kNaMaxP];
   SegDesc seg;
   int counter;
+  int prepared;  // blocks of the current call's prepare launch done; 0 between calls
 };
+
+// The tiling and the source chunk of a call.  Threads per target: 4 up to 4,096
+// particles, 2 beyond (pair kernel at N = 2,048: 27 us with 4, 30 with 2, 47
+// with 1; at 4,096: 58, 60 and 68; at 8,192: 156, 145 and 155).
+struct NoallocConfig {
+  PairConfig pc;
+  int chunk;   // sources per work item: whole tiles
+  int chunks;
+  int tiles;   // target tiles
+};
+
+NoallocConfig noalloc_config(int n) {
+  NoallocConfig c;
+  const int st = (n + kNaTB - 1) / kNaTB;
+  c.pc = PairConfig{kNaTB, n <= 4096 ? 4 : 2, 4};
+  const int most = kNaSlots / st;               // chunks that the slots hold
+  const int per = (st + most - 1) / most;       // source tiles per chunk
+  c.chunk = per * kNaTB;
+  c.chunks = (st + per - 1) / per;
+  c.tiles = (n + targets_per_block(c.pc) - 1) / targets_per_block(c.pc);
+  return c;
+}
 
 static_assert(offsetof(NoallocScratch, boxes) % 256 == 0 && offsetof(NoallocScratch, partial) % 256 == 0 &&
                   offsetof(NoallocScratch, rates) % 256 == 0,
@@ -77,10 +106,14 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoallocS
 // Pack: positions relative to particle 0 as FP32 hi/lo, strengths hi/lo,
 // s^2/2 and volume; the bounding box (with the range of s^2/2 in w) of each
 // 128-particle tile; per-block maxima of the smoothing radius and of the
-// distance from particle 0.
+// distance from particle 0.  The last block to finish then writes the
+// near-tile radius (the rule of pawan_system_set_particles, with the extent
+// measured from particle 0), the segment descriptor and the work list, and
+// clears the counters.
 __global__ void __launch_bounds__(kStageThreads)
     noalloc_prepare(NoallocScratch *S, const double *pos, const double *vor, const double *rad,
-                    const double *vol, int n) {
+                    const double *vol, int n, double nu, int tpb, int tiles, int chunk, int chunks) {
+  __shared__ int s_last;
   __shared__ float lo[4][kStageThreads], hi[4][kStageThreads];
   __shared__ float ms[kStageThreads], me[kStageThreads];
   const int t = threadIdx.x;
@@ -137,23 +170,19 @@ __global__ void __launch_bounds__(kStageThreads)
   if (t == 0) {
     S->block_max[2 * blockIdx.x] = ms[0];
     S->block_max[2 * blockIdx.x + 1] = me[0];
+    __threadfence();
+    s_last = atomicAdd(&S->prepared, 1) == (int)gridDim.x - 1;
   }
-}
-
-// One block: near-tile radius (the rule of pawan_system_set_particles, with the
-// extent measured from particle 0), the segment descriptor, the work list, and
-// the cleared scheduler counter.
-__global__ void noalloc_plan(NoallocScratch *S, int n, int nblocks, double nu) {
-  __shared__ float smax, emax;
-  if (threadIdx.x == 0) {
+  __syncthreads();
+  if (!s_last) return;  // block-uniform
+  __threadfence();
+  if (t == 0) {
     float a = 0.f, b = 0.f;
-    for (int k = 0; k < nblocks; ++k) {
-      a = fmaxf(a, S->block_max[2 * k]);
-      b = fmaxf(b, S->block_max[2 * k + 1]);
+    for (int k = 0; k < (int)gridDim.x; ++k) {
+      a = fmaxf(a, __ldcg(&S->block_max[2 * k]));
+      b = fmaxf(b, __ldcg(&S->block_max[2 * k + 1]));
     }
-    smax = a;
-    emax = b;
-    const float r_near = fmaxf(4.f * smax, 0.03f * sqrtf(emax));
+    const float r_near = fmaxf(4.f * a, 0.03f * sqrtf(b));
     SegDesc d;
     d.pos32 = S->pos32;
     d.vor32 = S->vor32;
@@ -166,25 +195,17 @@ __global__ void noalloc_plan(NoallocScratch *S, int n, int nblocks, double nu) {
     d.rates = S->rates;
     d.tile_count = S->tile_count;
     d.n = n;
-    d.nchunks = (n + kNaChunk - 1) / kNaChunk;
+    d.nchunks = chunks;
     d.nu = nu;
     d.near2 = r_near * r_near;
     S->seg = d;
     S->counter = 0;
+    S->prepared = 0;
   }
-  __syncthreads();
-  const int tiles = (n + kNaTB - 1) / kNaTB;
-  const int chunks = (n + kNaChunk - 1) / kNaChunk;
-  for (int t = threadIdx.x; t < tiles; t += blockDim.x) S->tile_count[t] = 0;
-  for (int it = threadIdx.x; it < tiles * chunks; it += blockDim.x) {
-    const int c = it / tiles, tt = it % tiles;
-    WorkItem w;
-    w.seg = 0;
-    w.t0 = tt * kNaTB;
-    w.chunk = c;
-    w.s0 = c * kNaChunk;
-    w.s1 = min(n, (c + 1) * kNaChunk);
-    S->items[it] = w;
+  for (int q = t; q < tiles; q += kStageThreads) S->tile_count[q] = 0;
+  for (int it = t; it < tiles * chunks; it += kStageThreads) {
+    const int q = it / chunks, c = it - q * chunks;
+    S->items[it] = WorkItem{0, q * tpb, c, c * chunk, min(n, (c + 1) * chunk)};
   }
 }
 
@@ -201,7 +222,7 @@ __global__ void noalloc_reduce(const NoallocScratch *S, int n, double *vel, doub
 
 struct DeviceSlot {
   NoallocScratch *scratch = nullptr;
-  int grid = 0;
+  int grid[2] = {0, 0};  // resident blocks with 2 and with 4 threads per target
 };
 constexpr int kMaxDevices = 64;
 DeviceSlot g_slots[kMaxDevices];
@@ -220,12 +241,15 @@ cudaError_t device_slot(int dev, DeviceSlot *out) {
     int sms = 0, bps = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    e = pairs_f32_occupancy(PairConfig{kNaTB, 1, 2}, true, KERNEL_HIGHORDER, &bps);
-    if (e != cudaSuccess) return e;
-    int bps0 = 0;
-    e = pairs_f32_occupancy(PairConfig{kNaTB, 1, 2}, false, KERNEL_HIGHORDER, &bps0);
-    if (e != cudaSuccess) return e;
-    s.grid = sms * (bps < bps0 ? bps : bps0);
+    for (int k = 0; k < 2; ++k) {
+      int bps0 = 0;
+      const PairConfig pc{kNaTB, k ? 4 : 2, 4};
+      e = pairs_f32_occupancy(pc, true, KERNEL_HIGHORDER, &bps);
+      if (e != cudaSuccess) return e;
+      e = pairs_f32_occupancy(pc, false, KERNEL_HIGHORDER, &bps0);
+      if (e != cudaSuccess) return e;
+      s.grid[k] = sms * (bps < bps0 ? bps : bps0);
+    }
     s.scratch = static_cast<NoallocScratch *>(ptr);
   }
   *out = s;
@@ -251,13 +275,13 @@ extern "C" int pawan_interact_noalloc(const double *position, const double *vort
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int ni = (int)n;
   const int pblocks = (ni + kStageThreads - 1) / kStageThreads;
-  noalloc_prepare<<<pblocks, kStageThreads, 0, s>>>(slot.scratch, position, vorticity, radius,
-                                                     volume, ni);
-  noalloc_plan<<<1, 256, 0, s>>>(slot.scratch, ni, pblocks, nu);
-  const int items = ((ni + kNaTB - 1) / kNaTB) * ((ni + kNaChunk - 1) / kNaChunk);
-  cudaError_t e = launch_pairs_f32(PairConfig{kNaTB, 1, 2}, nu != 0.0, KERNEL_HIGHORDER, slot.grid,
-                                   slot.scratch->items, items, &slot.scratch->seg,
-                                   &slot.scratch->counter, s);
+  const NoallocConfig c = noalloc_config(ni);
+  noalloc_prepare<<<pblocks, kStageThreads, 0, s>>>(slot.scratch, position, vorticity, radius, volume, ni, nu,
+                                                     targets_per_block(c.pc), c.tiles, c.chunk, c.chunks);
+  const int items = c.tiles * c.chunks;
+  const int resident = slot.grid[c.pc.p == 4 ? 1 : 0];
+  cudaError_t e = launch_pairs_f32(c.pc, nu != 0.0, KERNEL_HIGHORDER, items < resident ? items : resident,
+                                   slot.scratch->items, items, &slot.scratch->seg, &slot.scratch->counter, s);
   if (e != cudaSuccess) return PAWAN_ERR_CUDA;
   noalloc_reduce<<<(ni + 255) / 256, 256, 0, s>>>(slot.scratch, ni, velocity, retvorcity);
   if (cudaGetLastError() != cudaSuccess) return PAWAN_ERR_CUDA;
