@@ -407,7 +407,7 @@ static int run_diagnostics(pawan_system *sys, bool quadratic, double *out12) {
   cudaError_t e = launch_diagnostics((int)sys->n, sys->kernel, sys->pos64.p, sys->vor64.p, sys->wake_id.p,
                                      sys->diag_scratch.p, sys->diag_out.p, quadratic, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "diagnostics launch");
-  ctx->launches += quadratic ? 4 : 2;
+  ctx->launches += quadratic ? 3 : 2;
   double h[12] = {0};
   PAWAN_CUDA(ctx, cudaMemcpyAsync(h, sys->diag_out.p, 12 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   PAWAN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -17,11 +17,21 @@
 // Gaussian QSIG (:30-38): q = (phi/rho_bar - Z)/rho_bar^2 with
 // phi = erf(rho_bar/sqrt 2)/(4 pi sigma^3), Z = exp(-rho_bar^2/2)/(sigma^3 (2 pi)^1.5).
 // The reference's pair loops visit i<j and double (or, across wakes, double
-// the full cross sum); both equal one term per ordered pair, which is the
-// gather sum written here.  Per-target sums are reduced per block in a fixed
+// the full cross sum); the terms are symmetric in (i, j), so each unordered pair
+// is visited once here too.  Per-target sums are reduced per block in a fixed
 // tree and the block partials by one block in fixed order: deterministic.
+//
+// The quadratic kernel is bound by the FP64 pipe: 67 operations per unordered
+// pair.  A block takes 128 targets and a range of the sources from the targets'
+// own tile on, in ranges short enough that the device is full from about two
+// thousand particles on.  Helical wake, whole call on one B200: N = 65,536
+// 10.5 ms (28.7 when every ordered pair was visited, by one block per 128
+// targets), 0.74 of the FP64 pipe's rate; N = 16,384 0.69 ms (3.2).
+#include <algorithm>
+
 #include "device.cuh"
 #include "kernels.h"
+#include "rsqrt64.cuh"
 
 namespace pawan {
 namespace {
@@ -29,6 +39,8 @@ namespace {
 constexpr int kDiagThreads = 128;
 constexpr int kLin = 9;   // linear quantities
 constexpr int kQuad = 3;  // enstrophy, helicity, kinetic energy
+constexpr int kFinalThreads = 512;
+constexpr double kDiagBlocks = 3000.0;  // five per resident block: the last ones end together
 
 template <int K>
 __device__ void block_sum(double (&v)[K], double *smem /* [K][kDiagThreads] */, double *out) {
@@ -75,16 +87,26 @@ __global__ void __launch_bounds__(kDiagThreads)
   block_sum<kLin>(v, smem, block_out + (size_t)blockIdx.x * kLin);
 }
 
+// Block (c, I): targets of tile I against the sources j > i of
+// [128 I + c * span, 128 I + (c + 1) * span).
 template <int KERN>
 __global__ void __launch_bounds__(kDiagThreads)
-    diag_quadratic_kernel(int n, const double4 *__restrict__ pos, const double4 *__restrict__ vor,
+    diag_quadratic_kernel(int n, int tile0, int span, const double4 *__restrict__ pos, const double4 *__restrict__ vor,
                           const int *__restrict__ wake_id, double *__restrict__ block_out) {
-  __shared__ double4 sp[kDiagThreads];
+  __shared__ double4 sp[kDiagThreads];  // w: s^2 / 2
   __shared__ double4 sv[kDiagThreads];
   __shared__ int sw[kDiagThreads];
   __shared__ double smem[kQuad * kDiagThreads];
   const int tid = threadIdx.x;
-  const int i = blockIdx.x * kDiagThreads + tid;
+  const int I = tile0 + blockIdx.y;
+  const int i = I * kDiagThreads + tid;
+  double *const out = block_out + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kQuad;
+  const long long first = (long long)I * kDiagThreads + (long long)blockIdx.x * span;
+  if (first >= n) {
+    if (tid < kQuad) out[tid] = 0.0;
+    return;
+  }
+  const int s0 = (int)first, s1 = (int)min((long long)n, first + span);
   const bool valid = i < n;
   double4 ri = make_double4(0, 0, 0, 1), ai = make_double4(0, 0, 0, 0);
   int wi = -1;
@@ -93,105 +115,121 @@ __global__ void __launch_bounds__(kDiagThreads)
     ai = vor[i];
     wi = wake_id[i];
   }
-  const double A = kInv4Pi;
-  const double si = ri.w;
-  const double hi = 0.5 * si * si;
-  const double a2 = ai.x * ai.x + ai.y * ai.y + ai.z * ai.z;
-  double ens = (valid && KERN == KERNEL_HIGHORDER) ? 5.0 * kInvPi / 4.0 / (si * si * si) * a2 : 0.0;
-  double hel = 0.0;
-  double ke = valid ? 2.0 * (kInvPi * a2 / si / 8.0) : 0.0;
-
-  for (int ts = 0; ts < n; ts += kDiagThreads) {
+  const double hi = 0.5 * ri.w * ri.w;
+  double ens = 0.0, hel = 0.0, all = 0.0, same = 0.0;
+  for (int ts = s0; ts < s1; ts += kDiagThreads) {
     __syncthreads();
     const int j = ts + tid;
-    if (j < n) {
-      sp[tid] = pos[j];
+    if (j < s1) {
+      const double4 r = pos[j];
+      sp[tid] = make_double4(r.x, r.y, r.z, 0.5 * r.w * r.w);
       sv[tid] = vor[j];
       sw[tid] = wake_id[j];
     }
     __syncthreads();
-    const int cnt = min(kDiagThreads, n - ts);
+    const int cnt = min(kDiagThreads, s1 - ts);
+    const int own = i - ts;  // sources up to the target itself belong to the other order
+#pragma unroll 2
     for (int jj = 0; jj < cnt; ++jj) {
-      if (ts + jj == i) continue;
+      if (jj <= own) continue;
       const double4 rj = sp[jj], aj = sv[jj];
       const double x0 = rj.x - ri.x, x1 = rj.y - ri.y, x2 = rj.z - ri.z;
-      const double rho2 = x0 * x0 + x1 * x1 + x2 * x2;
-      const double sig2 = hi + 0.5 * rj.w * rj.w;
-      const double w = rsqrt(rho2 + sig2);
-      const double w2 = w * w, w3 = w2 * w, w4 = w2 * w2;
-      const double aa = ai.x * aj.x + ai.y * aj.y + ai.z * aj.z;
-      const double aix = ai.x * x0 + ai.y * x1 + ai.z * x2;
-      const double ajx = aj.x * x0 + aj.y * x1 + aj.z * x2;
-      const double rinv = rsqrt(rho2);
+      const double rho2 = fma(x2, x2, fma(x1, x1, x0 * x0));
+      const double sig2 = hi + rj.w;
+      const double s = rho2 + sig2;
+      const double w = rsqrt_f64(s), w2 = w * w, w3 = w2 * w, w4 = w2 * w2;
+      const double aa = fma(ai.z, aj.z, fma(ai.y, aj.y, ai.x * aj.x));
+      const double pp = fma(ai.z, x2, fma(ai.y, x1, ai.x * x0)) * fma(aj.z, x2, fma(aj.y, x1, aj.x * x0));
+      const double rinv = rsqrt_f64(rho2);
       double q;
       if (KERN == KERNEL_GAUSSIAN) {
-        // QSIG, gaussian.h:30-38
+        // QSIG, gaussian.h:30-38, in units of 1 / (4 pi)
         const double sig = sqrt(sig2);
         const double rho_bar = rho2 * rinv / sig;
-        const double sig3 = sig2 * sig;
-        const double z = exp(-0.5 * rho_bar * rho_bar) / sig3 / pow(2.0 * kPi, 1.5);
-        const double phi = 0.25 * kInvPi * erf(kSqrtHalf * rho_bar) / sig3;
-        q = (phi / rho_bar - z) / (rho_bar * rho_bar);
+        const double z = kSqrt2OverPi * exp(-0.5 * rho_bar * rho_bar);
+        q = (erf(kSqrtHalf * rho_bar) / rho_bar - z) / (rho_bar * rho_bar * sig2 * sig);
       } else {
-        // ENST: factor = (1/8pi) (rho^2 + sigma^2)^(-7/2)
-        const double factor = (kInvPi / 8.0) * (w4 * w3);
-        const double F1 = factor * (10.0 * sig2 * sig2 - 2.0 * rho2 * rho2 - 7.0 * sig2 * rho2);
-        const double F2 = factor * (-15.0 * rho2);
-        ens += F1 * aa + F2 * aix * ajx;
-        // QSIG: q = (phi/rho_bar - Z)/rho_bar^2
-        const double uu = sig2 * w2;
-        const double u2 = uu * uu;
+        // ENST in units of 1 / (8 pi): (rho^2 + sigma^2)^(-7/2) [F1 (a_i.a_j) - 15 rho^2 (a_i.x)(a_j.x)],
+        // F1 = 10 sigma^4 - 2 rho^4 - 7 sigma^2 rho^2 = 3 sigma^2 (4 sigma^2 - rho^2) - 2 (rho^2 + sigma^2)^2
+        const double f1 = fma(-2.0 * s, s, 3.0 * sig2 * fma(4.0, sig2, -rho2));
+        ens = fma(w4 * w3, fma(-15.0 * rho2, pp, f1 * aa), ens);
+        // QSIG in units of 1 / (4 pi): q = (phi/rho_bar - Z)/rho_bar^2
+        const double uu = sig2 * w2, u2 = uu * uu;
         const double zc = u2 * u2 * u2 * w3;
-        const double ph = (rho2 + 1.5 * sig2) * w4 * rinv;
-        q = A * (ph - 7.5 * zc) * sig2 * (rinv * rinv);
+        const double ph = fma(1.5, sig2, rho2) * w4 * rinv;
+        q = fma(-7.5, zc, ph) * sig2 * (rinv * rinv);
       }
-      const double c0 = ai.y * aj.z - ai.z * aj.y;
-      const double c1 = ai.z * aj.x - ai.x * aj.z;
-      const double c2 = ai.x * aj.y - ai.y * aj.x;
-      hel += q * (x0 * c0 + x1 * c1 + x2 * c2);
-      // KINETICENERGY
-      const double e = ((rho2 + 2.0 * sig2) * aa + aix * ajx) * w3 / 16.0 * kInvPi;
-      ke += (sw[jj] == wi ? 2.0 : 1.0) * e;
+      const double c0 = fma(ai.y, aj.z, -ai.z * aj.y);
+      const double c1 = fma(ai.z, aj.x, -ai.x * aj.z);
+      const double c2 = fma(ai.x, aj.y, -ai.y * aj.x);
+      hel = fma(q, fma(x2, c2, fma(x1, c1, x0 * c0)), hel);
+      // KINETICENERGY in units of 1 / (16 pi), counted once more inside a wake
+      const double e = fma(s + sig2, aa, pp) * w3;
+      all += e;
+      same += sw[jj] == wi ? e : 0.0;
     }
   }
-  double v[kQuad] = {valid ? ens : 0.0, valid ? hel : 0.0, valid ? ke : 0.0};
+  double v[kQuad] = {0.0, 0.0, 0.0};
+  if (valid) {
+    v[0] = 2.0 * (kInvPi / 8.0) * ens;
+    v[1] = 2.0 * kInv4Pi * hel;
+    v[2] = 2.0 * (kInvPi / 16.0) * (all + same);
+    if (blockIdx.x == 0) {
+      const double a2 = ai.x * ai.x + ai.y * ai.y + ai.z * ai.z;
+      if (KERN == KERNEL_HIGHORDER) v[0] += 5.0 * kInvPi / 4.0 / (ri.w * ri.w * ri.w) * a2;
+      v[2] += 2.0 * (kInvPi * a2 / ri.w / 8.0);
+    }
+  }
   __syncthreads();
-  block_sum<kQuad>(v, smem, block_out + (size_t)blockIdx.x * kQuad);
+  block_sum<kQuad>(v, smem, out);
 }
 
-// One block: sums nblk rows of width K in a fixed order.
-template <int K>
-__global__ void __launch_bounds__(kDiagThreads)
-    diag_final_kernel(int nblk, const double *__restrict__ rows, double *__restrict__ out,
-                      double scale_lin) {
-  __shared__ double smem[K * kDiagThreads];
-  double v[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) v[k] = 0.0;
-  for (int b = threadIdx.x; b < nblk; b += kDiagThreads) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] += rows[(size_t)b * K + k];
+// Block 0 sums the linear rows, block 1 the quadratic ones, in a fixed order.
+__global__ void __launch_bounds__(kFinalThreads)
+    diag_final_kernel(int lin_rows, const double *__restrict__ lin, int quad_rows,
+                      const double *__restrict__ quad, double *__restrict__ out) {
+  __shared__ double part[kLin][kFinalThreads / 32];
+  const bool linear = blockIdx.x == 0;
+  const int rows = linear ? lin_rows : quad_rows, width = linear ? kLin : kQuad;
+  const double *src = linear ? lin : quad;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int k = 0; k < width; ++k) {
+    double v = 0.0;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < rows; b += kFinalThreads) v += src[(size_t)b * width + k];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) part[k][warp] = v;
   }
-  double tot[K];
-  block_sum<K>(v, smem, tot);
-  if (threadIdx.x == 0) {
-    if (K == kLin) {
-      for (int k = 0; k < 3; ++k) {
-        out[k] = tot[k];
-        out[3 + k] = tot[3 + k] * 0.5;
-        out[6 + k] = tot[6 + k] * (1.0 / 3.0);
-      }
-    } else {
-      for (int k = 0; k < K; ++k) out[9 + k] = tot[k];
-    }
+  __syncthreads();
+  if (threadIdx.x < width) {
+    const int k = threadIdx.x;
+    double v = 0.0;
+    for (int w = 0; w < kFinalThreads / 32; ++w) v += part[k][w];
+    if (linear)
+      out[k] = k < 3 ? v : k < 6 ? v * 0.5 : v * (1.0 / 3.0);
+    else
+      out[kLin + k] = v;
   }
+}
+
+// Sources per block of the quadratic kernel: whole warps' worth, such that
+// about kDiagBlocks blocks are not empty (half of the grid is).
+int diag_span(int n) {
+  const double tiles = (double)((n + kDiagThreads - 1) / kDiagThreads);
+  const double per = std::min((double)n, 0.5 * tiles * (double)n / kDiagBlocks);
+  return 32 * std::max(1, (int)(per / 32.0));
+}
+
+int diag_chunks(int n) {
+  const int span = diag_span(n);
+  return (n + span - 1) / span;
 }
 
 }  // namespace
 
 size_t diag_scratch_doubles(int n) {
   const size_t nblk = (size_t)(n + kDiagThreads - 1) / kDiagThreads;
-  return nblk * (kLin + kQuad);
+  return nblk * (kLin + (size_t)diag_chunks(n) * kQuad);
 }
 
 cudaError_t launch_diagnostics(int n, int kernel, const double4 *pos64, const double4 *vor64,
@@ -202,14 +240,17 @@ cudaError_t launch_diagnostics(int n, int kernel, const double4 *pos64, const do
   double *lin = scratch;
   double *quad = scratch + (size_t)nblk * kLin;
   diag_linear_kernel<<<nblk, kDiagThreads, 0, s>>>(n, pos64, vor64, lin);
-  diag_final_kernel<kLin><<<1, kDiagThreads, 0, s>>>(nblk, lin, out, 0.0);
-  if (quadratic) {
+  const int span = diag_span(n), chunks = diag_chunks(n);
+  // tiles in y in slices of the grid's extent (65,535)
+  for (int t0 = 0; quadratic && t0 < nblk; t0 += 65535) {
+    const dim3 grid(chunks, std::min(65535, nblk - t0));
+    double *q = quad + (size_t)t0 * chunks * kQuad;
     if (kernel == KERNEL_GAUSSIAN)
-      diag_quadratic_kernel<KERNEL_GAUSSIAN><<<nblk, kDiagThreads, 0, s>>>(n, pos64, vor64, wake_id, quad);
+      diag_quadratic_kernel<KERNEL_GAUSSIAN><<<grid, kDiagThreads, 0, s>>>(n, t0, span, pos64, vor64, wake_id, q);
     else
-      diag_quadratic_kernel<KERNEL_HIGHORDER><<<nblk, kDiagThreads, 0, s>>>(n, pos64, vor64, wake_id, quad);
-    diag_final_kernel<kQuad><<<1, kDiagThreads, 0, s>>>(nblk, quad, out, 0.0);
+      diag_quadratic_kernel<KERNEL_HIGHORDER><<<grid, kDiagThreads, 0, s>>>(n, t0, span, pos64, vor64, wake_id, q);
   }
+  diag_final_kernel<<<quadratic ? 2 : 1, kFinalThreads, 0, s>>>(nblk, lin, nblk * chunks, quad, out);
   return cudaGetLastError();
 }
 
