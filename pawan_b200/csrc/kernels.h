@@ -46,12 +46,12 @@ cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem
 cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const SymSeg *segs, const double *slots,
                             cudaStream_t s);
 
-// FP64 with the same algebra as the FP32 kernel ("tuned FP64").
+// FP64 with the same algebra as the FP32 kernel ("tuned FP64"), on the symmetric
+// engine whatever the tiling.
 bool pairs_f64_supported(const PairConfig &c, int kernel);
-cudaError_t pairs_f64_occupancy(const PairConfig &c, bool diffusion, int kernel, int *blocks_per_sm);
-cudaError_t launch_pairs_f64(const PairConfig &c, bool diffusion, int kernel, int grid,
-                             const WorkItem *items, int n_items, const SegDesc *segs,
-                             int *next_item, cudaStream_t s);
+cudaError_t sym_f64_occupancy(bool group, bool diffusion, int kernel, int *blocks_per_sm);
+cudaError_t launch_sym_f64(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
+                           const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s);
 
 // FP64, the reference's formula term by term (pow, divisions): the plain
 // FP64 comparator.

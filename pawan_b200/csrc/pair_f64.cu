@@ -1,13 +1,11 @@
 // All-pairs interaction in FP64 with the kernel algebra of the FP32 kernel
 // (pair_f32.cu): two rsqrt per pair, no pow, no division; alpha_i x alpha_j
-// per pair as the reference forms it, and the diffusion as
-// v_i sum(Dp alpha_j) - alpha_i sum(Dp v_j), taken after the pair loop.
-// (Forming the stretching's q-term as alpha_i x sum(q alpha_j) and the triple
-// product from the velocity's cross product as well saves six more operations
-// per pair but sums nearly parallel neighbours' terms coherently before the
-// cross product: 100 times the rounding error of the per-pair form.)  This is the
-// "tuned FP64" variant, reported beside the FP32 kernel and the plain FP64
-// comparator (pair_plain.cu).  Same work items, partial layout and gather form.
+// per pair as the reference forms it.  (Forming the stretching's q-term as
+// alpha_i x sum(q alpha_j) and the triple product from the velocity's cross
+// product as well saves six more operations per pair but sums nearly parallel
+// neighbours' terms coherently before the cross product: 100 times the rounding
+// error of the per-pair form.)  This is the "tuned FP64" variant, reported
+// beside the FP32 kernel and the plain FP64 comparator (pair_plain.cu).
 //
 // Reference: INTERACT (src/interaction/interaction_utils.h:363-407), KERNEL
 // (src/interaction/highorder.h:48-60), __interaction::interact
@@ -16,27 +14,42 @@
 // e = exp(-x2/2), K = sqrt(2/pi), gq = (erf(x/sqrt 2)/x - K e)/x2 and
 // gf = (K e - 3 gq)/x2: qh = gq/sigma^3, fh = gf/(3 sigma^5),
 // dp = (2/15) K e / sigma^5 (closed forms, as the reference evaluates them).
-#include "device.cuh"
-#include "kernels.h"
+//
+// Runs on the symmetric pair engine (pair_sym.cuh), each unordered pair once:
+// q (alpha_j x d) for the target and -q (alpha_i x d) for the source, and one
+// vector s = q (alpha_i x alpha_j) + 3 F t d + 15 nu Dp (v_i alpha_j - v_j alpha_i)
+// that is added to one and taken from the other.  As in the FP32 kernel a
+// lane's targets stay in registers and 32 sources in shared memory, whose six
+// sums travel by shuffle.  Bound by the FP64 pipe: 87 operations for two
+// interactions (77 without diffusion) against 76 for one before.  One
+// right-hand side on one B200: ring pair at N = 65,536 12.2 ms (352 G
+// interactions/s, 0.83 of the pipe) against 19.3; at N = 2,048 27 us against 69.
+#include "pair_sym.cuh"
+#include "rsqrt64.cuh"
 
 namespace pawan {
 namespace {
 
-__device__ __forceinline__ void load_source_f64(const SegDesc &sg, int j, int s1, double4 &p,
-                                                double4 &v) {
-  if (j < s1) {
-    p = sg.pos64[j];
-    v = sg.vor64[j];
-  } else {
-    p = make_double4(1e150, 1e150, 1e150, 1.0);
-    v = make_double4(0.0, 0.0, 0.0, 0.0);
-  }
-}
+constexpr int kStage64 = 4 * 512;    // per warp: 4 x double2[32]
+// Targets per lane and blocks per SM: four targets in 255 registers keep the
+// FP64 pipe fullest (one right-hand side of the ring pair at N = 16,384: 0.787
+// ms, against 0.819 with two targets and three blocks, 0.865 with one and four);
+// the Gaussian kernel's exp and erf want the warps instead (1.89 ms at N =
+// 16,000 with one and four, 2.05 with two and three, 2.52 with four and two).
+template <int KERN>
+struct Shape64 {
+  static constexpr int targets = KERN == KERNEL_GAUSSIAN ? 1 : 4;
+  static constexpr int blocks = KERN == KERNEL_GAUSSIAN ? 4 : 2;
+};
+
+// Particles past the end: far away on opposite sides, with zero strength and
+// volume, so that every term they enter is exactly zero.
+constexpr double kPad64 = 1e150;
 
 // Gaussian qh, fh, dp (see the file comment) from r2, sig2 and 1/rho.
 __device__ __forceinline__ void gauss_f64(double r2, double sig2, double ri, double &qh,
                                           double &fh, double &dp) {
-  const double is = rsqrt(sig2);
+  const double is = rsqrt_f64(sig2);
   const double is2 = is * is;
   const double is3 = is2 * is;
   const double x2 = r2 * is2;
@@ -49,165 +62,194 @@ __device__ __forceinline__ void gauss_f64(double r2, double sig2, double ri, dou
   dp = (2.0 / 15.0) * kSqrt2OverPi * e * is3 * is2;
 }
 
-template <int TB, bool DIFF, int KERN>
-__global__ void __launch_bounds__(TB)
-    pairs_f64_kernel(const WorkItem *__restrict__ items, int n_items,
-                     const SegDesc *__restrict__ segs, int *__restrict__ next_item) {
-  __shared__ double4 sp[2][TB];
-  __shared__ double4 sv[2][TB];
-  __shared__ int s_item, s_last;
-  const int tid = threadIdx.x;
+struct Sums64 {
+  double ux, uy, uz, sx, sy, sz;
+};
 
-  for (;;) {
-    if (tid == 0) s_item = atomicAdd(next_item, 1);
-    __syncthreads();
-    const int it = s_item;
-    __syncthreads();
-    if (it >= n_items) break;
+__device__ __forceinline__ void rotate(Sums64 &a, int m) {
+  a.ux = __shfl_xor_sync(kFull, a.ux, m);
+  a.uy = __shfl_xor_sync(kFull, a.uy, m);
+  a.uz = __shfl_xor_sync(kFull, a.uz, m);
+  a.sx = __shfl_xor_sync(kFull, a.sx, m);
+  a.sy = __shfl_xor_sync(kFull, a.sy, m);
+  a.sz = __shfl_xor_sync(kFull, a.sz, m);
+}
 
-    const WorkItem w = items[it];
-    const SegDesc sg = segs[w.seg];
-    const int i = w.t0 + tid;
-    const bool valid = i < sg.n;
-    double4 pi = make_double4(0.0, 0.0, 0.0, 1.0);
-    double4 vi = make_double4(0.0, 0.0, 0.0, 0.0);
-    if (valid) {
-      pi = sg.pos64[i];
-      vi = sg.vor64[i];
-    }
-    const double hi = 0.5 * pi.w * pi.w;
-    // u = sum qh (alpha_j x d); q = sum qh (alpha_i x alpha_j);
-    // G = sum fh [d.(alpha_i x alpha_j)] d; E = sum Dp alpha_j, V = sum Dp v_j
-    // (the diffusion is v_i E - V alpha_i)
-    double ux = 0, uy = 0, uz = 0, qx = 0, qy = 0, qz = 0, gx = 0, gy = 0, gz = 0;
-    double ex = 0, ey = 0, ez = 0, ev = 0;
+__device__ __forceinline__ void add64(const Sums64 &s, double f, double *acc) {
+  acc[0] += f * s.ux;
+  acc[kT] += f * s.uy;
+  acc[2 * kT] += f * s.uz;
+  acc[3 * kT] += f * s.sx;
+  acc[4 * kT] += f * s.sy;
+  acc[5 * kT] += f * s.sz;
+}
 
-    const int ntiles = (w.s1 - w.s0 + TB - 1) / TB;
-    double4 rp, rv;
-    load_source_f64(sg, w.s0 + tid, w.s1, rp, rv);
-    for (int t = 0; t < ntiles; ++t) {
-      const int buf = t & 1;
-      sp[buf][tid] = rp;
-      sv[buf][tid] = rv;
-      __syncthreads();
-      const int ts = w.s0 + t * TB;
-      if (t + 1 < ntiles) load_source_f64(sg, ts + TB + tid, w.s1, rp, rv);
-      const int skip = i - ts;
-#pragma unroll 2
-      for (int jj = 0; jj < TB; ++jj) {
-        const double4 p = sp[buf][jj];
-        const double4 s = sv[buf][jj];
-        const double dx = pi.x - p.x, dy = pi.y - p.y, dz = pi.z - p.z;
-        const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-        const double sig2 = fma(0.5 * p.w, p.w, hi);
-        const double ri = rsqrt(r2);
-        double qh, fh, dp;
-        if (KERN == KERNEL_GAUSSIAN) {
-          gauss_f64(r2, sig2, ri, qh, fh, dp);
-        } else {
-          const double wr = rsqrt(r2 + sig2);
-          const double ri2 = ri * ri;
-          const double w2 = wr * wr;
-          const double w4 = w2 * w2;
-          const double uu = sig2 * w2;
-          const double u2 = uu * uu;
-          const double u4 = u2 * u2;
-          dp = u4 * uu * (w4 * wr);
-          const double zc = dp * sig2;
-          const double ph = fma(1.5, sig2, r2) * w4 * ri;
-          qh = fma(-7.5, zc, ph) * sig2 * ri2;
-          fh = fma(2.5, zc, -qh) * ri2;
-        }
-        const double cx = fma(s.y, dz, -s.z * dy);
-        const double cy = fma(s.z, dx, -s.x * dz);
-        const double cz = fma(s.x, dy, -s.y * dx);
-        const double wx = fma(vi.y, s.z, -vi.z * s.y);
-        const double wy = fma(vi.z, s.x, -vi.x * s.z);
-        const double wz = fma(vi.x, s.y, -vi.y * s.x);
-        const double tt = fma(dz, wz, fma(dy, wy, dx * wx));
-        double ft = fh * tt;
-        const bool self = (jj == skip);
-        qh = self ? 0.0 : qh;
-        ft = self ? 0.0 : ft;
-        dp = self ? 0.0 : dp;
-        ux = fma(qh, cx, ux);
-        uy = fma(qh, cy, uy);
-        uz = fma(qh, cz, uz);
-        qx = fma(qh, wx, qx);
-        qy = fma(qh, wy, qy);
-        qz = fma(qh, wz, qz);
-        gx = fma(ft, dx, gx);
-        gy = fma(ft, dy, gy);
-        gz = fma(ft, dz, gz);
-        if (DIFF) {
-          ex = fma(dp, s.x, ex);
-          ey = fma(dp, s.y, ey);
-          ez = fma(dp, s.z, ez);
-          ev = fma(dp, s.w, ev);
-        }
+// DIAG: tile I against itself; every ordered pair is visited and only the
+// targets' sums are kept.
+template <bool DIAG, bool DIFF, int KERN>
+__device__ __forceinline__ void pairs64(const SymSeg &sg, int I, int J, int k0, int k1, char *stage, int lane,
+                                        double *accI, double *accJ) {
+  constexpr int kR = Shape64<KERN>::targets;
+  double2 *const s0 = reinterpret_cast<double2 *>(stage);  // x, y
+  double2 *const s1 = s0 + 32;                             // z, s^2 / 2
+  double2 *const s2 = s1 + 32;                             // alpha x, y
+  double2 *const s3 = s2 + 32;                             // alpha z, volume
+  const int n = sg.n;
+  const double kap = 15.0 * sg.nu;
+#pragma unroll 1
+  for (int t0 = 0; t0 < kT; t0 += 32 * kR) {
+    double4 p[kR], a[kR];  // w: s^2 / 2, volume
+    Sums64 sum[kR];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      const int i = I * kT + t0 + 32 * r + lane;
+      p[r] = make_double4(-kPad64, -kPad64, -kPad64, 1.0);
+      a[r] = make_double4(0.0, 0.0, 0.0, 0.0);
+      if (i < n) {
+        p[r] = sg.pos64[i];
+        a[r] = sg.vor64[i];
+        p[r].w = 0.5 * p[r].w * p[r].w;
       }
+      sum[r] = Sums64{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     }
-
-    if (valid) {
-      const double A = kInv4Pi;
-      double dax = A * qx + 3.0 * A * gx;
-      double day = A * qy + 3.0 * A * gy;
-      double daz = A * qz + 3.0 * A * gz;
-      if (DIFF) {
-        // v_i E - V alpha_i
-        const double c = 15.0 * sg.nu * A;
-        dax += c * fma(vi.w, ex, -ev * vi.x);
-        day += c * fma(vi.w, ey, -ev * vi.y);
-        daz += c * fma(vi.w, ez, -ev * vi.z);
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k) {
+      const int j = J * kT + 32 * k + lane;
+      double4 pj = make_double4(kPad64, kPad64, kPad64, 1.0), aj = make_double4(0.0, 0.0, 0.0, 0.0);
+      if (j < n) {
+        pj = sg.pos64[j];
+        aj = sg.vor64[j];
+        pj.w = 0.5 * pj.w * pj.w;
       }
-      const ItemOut o = item_out(sg, w.t0, w.chunk, TB);
-      double *out = o.base + (i - w.t0);
-      out[0] = A * ux;
-      out[o.stride] = A * uy;
-      out[2 * o.stride] = A * uz;
-      out[3 * o.stride] = dax;
-      out[4 * o.stride] = day;
-      out[5 * o.stride] = daz;
+      s0[lane] = make_double2(pj.x, pj.y);
+      s1[lane] = make_double2(pj.z, pj.w);
+      s2[lane] = make_double2(aj.x, aj.y);
+      s3[lane] = make_double2(aj.z, aj.w);
+      __syncwarp();
+      const int self = k - t0 / 32;  // the target whose own pair falls on step 0
+      Sums64 b{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+      for (int m = 0; m < 32; ++m) {
+        const double2 q0 = s0[lane ^ m], q1 = s1[lane ^ m], q2 = s2[lane ^ m], q3 = s3[lane ^ m];
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+          const double dx = p[r].x - q0.x, dy = p[r].y - q0.y, dz = p[r].z - q1.x;
+          const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+          const double sig2 = p[r].w + q1.y;
+          const double ri = rsqrt_f64(r2);
+          double qh, fh, dp;
+          if (KERN == KERNEL_GAUSSIAN) {
+            gauss_f64(r2, sig2, ri, qh, fh, dp);
+          } else {
+            const double wr = rsqrt_f64(r2 + sig2);
+            const double ri2 = ri * ri;
+            const double w2 = wr * wr;
+            const double w4 = w2 * w2;
+            const double uu = sig2 * w2;
+            const double u2 = uu * uu;
+            const double u4 = u2 * u2;
+            dp = u4 * uu * (w4 * wr);
+            const double zc = dp * sig2;
+            const double ph = fma(1.5, sig2, r2) * w4 * ri;
+            qh = fma(-7.5, zc, ph) * sig2 * ri2;
+            fh = fma(2.5, zc, -qh) * ri2;
+          }
+          const double wx = fma(a[r].y, q3.x, -a[r].z * q2.y);
+          const double wy = fma(a[r].z, q2.x, -a[r].x * q3.x);
+          const double wz = fma(a[r].x, q2.y, -a[r].y * q2.x);
+          const double ft = 3.0 * fh * fma(dz, wz, fma(dy, wy, dx * wx));
+          double sx = fma(ft, dx, qh * wx), sy = fma(ft, dy, qh * wy), sz = fma(ft, dz, qh * wz);
+          if (DIFF) {
+            const double kd = kap * dp;
+            sx = fma(kd, fma(a[r].w, q2.x, -q3.y * a[r].x), sx);
+            sy = fma(kd, fma(a[r].w, q2.y, -q3.y * a[r].y), sy);
+            sz = fma(kd, fma(a[r].w, q3.x, -q3.y * a[r].z), sz);
+          }
+          if (DIAG) {
+            const bool own = m == 0 && r == self;
+            qh = own ? 0.0 : qh;
+            sx = own ? 0.0 : sx;
+            sy = own ? 0.0 : sy;
+            sz = own ? 0.0 : sz;
+          }
+          sum[r].ux = fma(qh, fma(q2.y, dz, -q3.x * dy), sum[r].ux);
+          sum[r].uy = fma(qh, fma(q3.x, dx, -q2.x * dz), sum[r].uy);
+          sum[r].uz = fma(qh, fma(q2.x, dy, -q2.y * dx), sum[r].uz);
+          sum[r].sx += sx;
+          sum[r].sy += sy;
+          sum[r].sz += sz;
+          if (!DIAG) {
+            // alpha_i x d and s, taken from the source's sums at the end
+            b.ux = fma(qh, fma(a[r].y, dz, -a[r].z * dy), b.ux);
+            b.uy = fma(qh, fma(a[r].z, dx, -a[r].x * dz), b.uy);
+            b.uz = fma(qh, fma(a[r].x, dy, -a[r].y * dx), b.uz);
+            b.sx += sx;
+            b.sy += sy;
+            b.sz += sz;
+          }
+        }
+        if (!DIAG) rotate(b, (m ^ (m + 1)) & 31);
+      }
+      if (!DIAG) add64(b, -kInv4Pi, accJ + 32 * k + lane);
+      __syncwarp();
     }
-    if (sg.nchunks > 1) finish_item<TB>(sg, w.t0, TB, &s_last);
+#pragma unroll
+    for (int r = 0; r < kR; ++r) add64(sum[r], kInv4Pi, accI + t0 + 32 * r + lane);
   }
 }
 
-using KernelFn = void (*)(const WorkItem *, int, const SegDesc *, int *);
+template <bool DIFF, int KERN>
+struct Pair64 {
+  static constexpr int kStageBytes = kStage64;
+  static __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, char *st,
+                                                   int lane, double *accI, double *accJ) {
+    if (I == J)
+      pairs64<true, DIFF, KERN>(sg, I, J, k0, k1, st, lane, accI, accJ);
+    else
+      pairs64<false, DIFF, KERN>(sg, I, J, k0, k1, st, lane, accI, accJ);
+  }
+};
 
-template <int KERN>
-KernelFn select_k(const PairConfig &c, bool diffusion) {
-  if (c.tb == 128)
-    return diffusion ? &pairs_f64_kernel<128, true, KERN> : &pairs_f64_kernel<128, false, KERN>;
-  if (c.tb == 256)
-    return diffusion ? &pairs_f64_kernel<256, true, KERN> : &pairs_f64_kernel<256, false, KERN>;
-  return nullptr;
+template <bool DIFF, int KERN>
+__global__ void __launch_bounds__(kThreads, Shape64<KERN>::blocks)
+    sym_f64_group_kernel(const SymItem *__restrict__ items, const SymSeg *__restrict__ segs,
+                         const int *__restrict__ jbase, double *__restrict__ slots) {
+  group_item<Pair64<DIFF, KERN>>(items, segs, jbase, slots);
 }
 
-KernelFn select(const PairConfig &c, bool diffusion, int kernel) {
-  if (c.p != 1 || c.r != 1 || c.packed != 0) return nullptr;
-  if (kernel == KERNEL_GAUSSIAN) return select_k<KERNEL_GAUSSIAN>(c, diffusion);
-  if (kernel == KERNEL_HIGHORDER) return select_k<KERNEL_HIGHORDER>(c, diffusion);
-  return nullptr;
+template <bool DIFF, int KERN>
+__global__ void __launch_bounds__(kThreads, Shape64<KERN>::blocks)
+    sym_f64_tile_kernel(const SymItem *__restrict__ items, const SymSeg *__restrict__ segs,
+                        const int *__restrict__ jbase, double *__restrict__ slots) {
+  tile_item<Pair64<DIFF, KERN>>(items, segs, jbase, slots);
+}
+
+template <int KERN>
+SymKernel select_k(bool group, bool diffusion) {
+  if (group) return diffusion ? &sym_f64_group_kernel<true, KERN> : &sym_f64_group_kernel<false, KERN>;
+  return diffusion ? &sym_f64_tile_kernel<true, KERN> : &sym_f64_tile_kernel<false, KERN>;
+}
+
+SymKernel select(bool group, bool diffusion, int kernel) {
+  return kernel == KERNEL_GAUSSIAN ? select_k<KERNEL_GAUSSIAN>(group, diffusion)
+                                   : select_k<KERNEL_HIGHORDER>(group, diffusion);
 }
 
 }  // namespace
 
-bool pairs_f64_supported(const PairConfig &c, int kernel) { return select(c, true, kernel) != nullptr; }
-
-cudaError_t pairs_f64_occupancy(const PairConfig &c, bool diffusion, int kernel, int *blocks_per_sm) {
-  KernelFn f = select(c, diffusion, kernel);
-  if (!f) return cudaErrorInvalidValue;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, c.tb, 0);
+bool pairs_f64_supported(const PairConfig &c, int kernel) {
+  return c.p == 1 && c.r == 1 && c.packed == 0 && (c.tb == 128 || c.tb == 256) &&
+         (kernel == KERNEL_HIGHORDER || kernel == KERNEL_GAUSSIAN);
 }
 
-cudaError_t launch_pairs_f64(const PairConfig &c, bool diffusion, int kernel, int grid,
-                             const WorkItem *items, int n_items, const SegDesc *segs,
-                             int *next_item, cudaStream_t s) {
-  KernelFn f = select(c, diffusion, kernel);
-  if (!f) return cudaErrorInvalidValue;
-  f<<<grid, c.tb, 0, s>>>(items, n_items, segs, next_item);
-  return cudaGetLastError();
+cudaError_t sym_f64_occupancy(bool group, bool diffusion, int kernel, int *blocks_per_sm) {
+  return sym_occupancy(select(group, diffusion, kernel), sym_smem_bytes(group, kStage64), blocks_per_sm);
+}
+
+cudaError_t launch_sym_f64(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
+                           const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
+  return sym_launch(select(group, diffusion, kernel), sym_smem_bytes(group, kStage64), items, n_items, segs, jbase,
+                    slots, s);
 }
 
 }  // namespace pawan

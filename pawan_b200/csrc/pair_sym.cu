@@ -49,23 +49,14 @@
 // once and its source-side sums per group, each to a slot of its own; a
 // separate kernel sums a particle's slots in a fixed order, so results do not
 // depend on scheduling.
-#include <mutex>
-#include <set>
-#include <utility>
-
-#include "device.cuh"
-#include "kernels.h"
 #include "pair_scalars.cuh"
+#include "pair_sym.cuh"
 
 namespace pawan {
 namespace {
 
-constexpr int kWarps = 4;
-constexpr int kThreads = 32 * kWarps;
 constexpr int kBlocks = 3;          // per SM: 168 registers, no spills (four blocks of 128 ran 4 % slower)
-constexpr int kT = kSymTile;        // particles per tile
 constexpr int kStageBytes = 1792;   // per warp: 3 x float4[32], float2[32]
-constexpr unsigned kFull = 0xffffffffu;
 
 struct Stage {
   float4 *s0, *s1, *s2;
@@ -554,86 +545,27 @@ __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0
   }
 }
 
-// Large systems: item = group a of four tiles against the groups [b0, b1).
+template <bool DIFF, int KERN>
+struct Pair32 {
+  static constexpr int kStageBytes = ::pawan::kStageBytes;
+  static __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, char *st,
+                                                   int lane, double *accI, double *accJ) {
+    ::pawan::tile_pair<DIFF, KERN>(sg, I, J, k0, k1, stage_of(st), lane, accI, accJ);
+  }
+};
+
 template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(kThreads, kBlocks)
     sym_f32_group_kernel(const SymItem *__restrict__ items, const SymSeg *__restrict__ segs,
                          const int *__restrict__ jbase, double *__restrict__ slots) {
-  extern __shared__ float4 smem_sym[];
-  double *const accI = reinterpret_cast<double *>(smem_sym);  // [4 warps][6][128]
-  double *const accJ = accI + kWarps * 6 * kT;                // [4 tiles][6][128]
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const Stage st = stage_of(reinterpret_cast<char *>(accJ + kWarps * 6 * kT) + warp * kStageBytes);
-  const SymItem it = items[blockIdx.x];
-  const SymSeg &sg = segs[it.seg];
-  const int nt = (sg.n + kT - 1) / kT;
-  for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accI[q] = 0.0;
-  for (int b = it.b0; b < it.b1; ++b) {
-    for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accJ[q] = 0.0;
-    __syncthreads();
-    for (int r = 0; r < kWarps; ++r) {
-      const int c = (warp + r) & 3;
-      const int I = it.a * kWarps + warp, J = b * kWarps + c;
-      // inside one group: each unordered tile pair once (rounds 0, 1 and half of 2)
-      const bool mine = b > it.a || r < 2 || (r == 2 && warp < 2);
-      if (mine && I < nt && J < nt)
-        tile_pair<DIFF, KERN>(sg, min(I, J), max(I, J), 0, 4, st, lane,
-                              (I <= J ? accI + warp * 6 * kT : accJ + c * 6 * kT),
-                              (I <= J ? accJ + c * 6 * kT : accI + warp * 6 * kT));
-      __syncthreads();
-    }
-    if (b == it.a) {
-      for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accI[q] += accJ[q];
-    } else {
-      const int jb = jbase[it.jb + b];
-      if (jb >= 0) {
-        double *out = slots + ((size_t)jb + it.a - it.row0) * kWarps * 6 * kT;
-        for (int q = tid; q < kWarps * 6 * kT; q += kThreads) out[q] = accJ[q];
-      }
-    }
-    __syncthreads();
-  }
-  if (it.islot >= 0) {
-    double *out = slots + (size_t)it.islot * kWarps * 6 * kT;
-    for (int q = tid; q < kWarps * 6 * kT; q += kThreads) out[q] = accI[q];
-  }
+  group_item<Pair32<DIFF, KERN>>(items, segs, jbase, slots);
 }
 
-// Small systems: item = one tile pair (a, b0); each warp 32 sources of tile b0.
 template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(kThreads, kBlocks)
     sym_f32_tile_kernel(const SymItem *__restrict__ items, const SymSeg *__restrict__ segs,
                         const int *__restrict__ jbase, double *__restrict__ slots) {
-  extern __shared__ float4 smem_sym[];
-  double *const accI = reinterpret_cast<double *>(smem_sym);  // [4 warps][6][128]
-  double *const accJ = accI + kWarps * 6 * kT;                // [6][128]
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const Stage st = stage_of(reinterpret_cast<char *>(accJ + 6 * kT) + warp * kStageBytes);
-  const SymItem it = items[blockIdx.x];
-  const SymSeg &sg = segs[it.seg];
-  double *const mine = accI + warp * 6 * kT;
-#pragma unroll
-  for (int q = 0; q < 24; ++q) mine[32 * q + lane] = 0.0;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) accJ[k * kT + tid] = 0.0;
-  tile_pair<DIFF, KERN>(sg, it.a, it.b0, warp, warp + 1, st, lane, mine, accJ);
-  if (it.b0 > it.a) {
-    const int jb = jbase[it.jb + it.b0];
-    if (jb >= 0) {
-      double *out = slots + ((size_t)jb + it.a) * 6 * kT;
-#pragma unroll
-      for (int k = 0; k < 6; ++k) out[k * kT + tid] = accJ[k * kT + tid];
-    }
-  }
-  __syncthreads();
-  if (it.islot >= 0) {
-    double *out = slots + (size_t)it.islot * 6 * kT;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      const int q = k * kT + tid;
-      out[q] = ((accI[q] + accI[6 * kT + q]) + accI[12 * kT + q]) + accI[18 * kT + q];
-    }
-  }
+  tile_item<Pair32<DIFF, KERN>>(items, segs, jbase, slots);
 }
 
 // One block per tile: thread (k, q) sums component k of particle q over the
@@ -661,9 +593,7 @@ __global__ void __launch_bounds__(6 * kT)
   *out = r;
 }
 
-using KernelFn = void (*)(const SymItem *, const SymSeg *, const int *, double *);
-
-KernelFn select(bool group, bool diffusion, int kernel) {
+SymKernel select(bool group, bool diffusion, int kernel) {
   if (kernel == KERNEL_GAUSSIAN) {
     if (group)
       return diffusion ? &sym_f32_group_kernel<true, KERNEL_GAUSSIAN> : &sym_f32_group_kernel<false, KERNEL_GAUSSIAN>;
@@ -674,45 +604,16 @@ KernelFn select(bool group, bool diffusion, int kernel) {
   return diffusion ? &sym_f32_tile_kernel<true, KERNEL_HIGHORDER> : &sym_f32_tile_kernel<false, KERNEL_HIGHORDER>;
 }
 
-size_t smem_bytes(bool group) {
-  const size_t acc = (size_t)kWarps * 6 * kT * sizeof(double);
-  return acc + (group ? acc : acc / kWarps) + (size_t)kWarps * kStageBytes;
-}
-
-// Opts a kernel in to its dynamic shared memory beyond the default 48 KB (once
-// per kernel and device).
-cudaError_t prepare(KernelFn f, size_t bytes) {
-  static std::mutex mu;
-  static std::set<std::pair<int, KernelFn>> done;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> lk(mu);
-  if (done.count({dev, f})) return cudaSuccess;
-  e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) done.insert({dev, f});
-  return e;
-}
-
 }  // namespace
 
 cudaError_t sym_f32_occupancy(bool group, bool diffusion, int kernel, int *blocks_per_sm) {
-  KernelFn f = select(group, diffusion, kernel);
-  const size_t bytes = smem_bytes(group);
-  cudaError_t e = prepare(f, bytes);
-  if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, kThreads, bytes);
+  return sym_occupancy(select(group, diffusion, kernel), sym_smem_bytes(group, kStageBytes), blocks_per_sm);
 }
 
 cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
                            const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
-  if (n_items <= 0) return cudaSuccess;
-  KernelFn f = select(group, diffusion, kernel);
-  const size_t bytes = smem_bytes(group);
-  cudaError_t e = prepare(f, bytes);
-  if (e != cudaSuccess) return e;
-  f<<<n_items, kThreads, bytes, s>>>(items, segs, jbase, slots);
-  return cudaGetLastError();
+  return sym_launch(select(group, diffusion, kernel), sym_smem_bytes(group, kStageBytes), items, n_items, segs,
+                    jbase, slots, s);
 }
 
 cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const SymSeg *segs, const double *slots,

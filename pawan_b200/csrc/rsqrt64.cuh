@@ -2,7 +2,8 @@
 // (rsqrt.approx.ftz.f64) and one step of Halley's third-order iteration,
 //   e = 1 - x y^2,   y <- y + y e (1/2 + 3/8 e),
 // whose error is 5/16 e^3: from an estimate good to 2^-20 full FP64 precision
-// in five FMA-pipe operations.  For 0, subnormal, infinite or NaN x the result
+// in five FMA-pipe operations.  The estimate's lower 32 bits are zero, so y^2
+// is exact and e carries one rounding, of its own small size.  For 0, subnormal, infinite or NaN x the result
 // is NaN (a pair at distance 0 has no finite rates either way).
 #pragma once
 
@@ -11,7 +12,7 @@ namespace pawan {
 __device__ __forceinline__ double rsqrt_f64(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x * y, y, 1.0);
+  const double e = fma(-x, y * y, 1.0);
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
 

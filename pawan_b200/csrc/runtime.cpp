@@ -86,7 +86,7 @@ bool Plan::stale() const {
 }
 
 bool tile_symmetric(int precision, const PairConfig &pc) {
-  return precision == PAWAN_PREC_F32 && pc.packed > 0;
+  return precision == PAWAN_PREC_F64 || (precision == PAWAN_PREC_F32 && pc.packed > 0);
 }
 
 static int occupancy(pawan_ctx *ctx, int precision, const PairConfig &pc, bool diffusion,
@@ -94,8 +94,6 @@ static int occupancy(pawan_ctx *ctx, int precision, const PairConfig &pc, bool d
   cudaError_t e;
   if (precision == PAWAN_PREC_F32)
     e = pairs_f32_occupancy(pc, diffusion, kernel, bps);
-  else if (precision == PAWAN_PREC_F64)
-    e = pairs_f64_occupancy(pc, diffusion, kernel, bps);
   else
     e = pairs_plain_occupancy(pc, kernel, bps);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy query");
@@ -351,7 +349,8 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
   int bps = 0;
   p->sym = tile_symmetric(precision, tile.pc);
   if (p->sym) {
-    cudaError_t e = sym_f32_occupancy(true, p->diffusion, kernel, &bps);
+    cudaError_t e = precision == PAWAN_PREC_F64 ? sym_f64_occupancy(true, p->diffusion, kernel, &bps)
+                                                : sym_f32_occupancy(true, p->diffusion, kernel, &bps);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy query");
   } else {
     PAWAN_TRY(occupancy(ctx, precision, tile.pc, p->diffusion, kernel, &bps));
@@ -579,8 +578,9 @@ static int launch_sym_range(pawan_ctx *ctx, Plan &p, int first, int count) {
       at += n;
       if (lo >= hi) continue;
       double *slots = p.slots.p + (group ? 0 : p.tile_slots);
-      PAWAN_CUDA(ctx, launch_sym_f32(group, p.diffusion, p.kernel, p.sym_items.p + lo, hi - lo, p.sym_segs.p,
-                                     p.sym_jbase.p, slots, ctx->stream));
+      const auto launch = p.precision == PAWAN_PREC_F64 ? launch_sym_f64 : launch_sym_f32;
+      PAWAN_CUDA(ctx, launch(group, p.diffusion, p.kernel, p.sym_items.p + lo, hi - lo, p.sym_segs.p,
+                             p.sym_jbase.p, slots, ctx->stream));
       ctx->launches++;
     }
     if (at > first && at <= first + count) {
@@ -618,9 +618,6 @@ int launch_pairs_range(pawan_ctx *ctx, Plan &p, int first, int count, bool allow
     PAWAN_TRY(launch_sym_range(ctx, p, first, count));
   else if (p.precision == PAWAN_PREC_F32)
     e = launch_pairs_f32(p.tile.pc, p.diffusion, p.kernel, p.grid, items, count, p.segs.p,
-                         ctx->d_counter, ctx->stream);
-  else if (p.precision == PAWAN_PREC_F64)
-    e = launch_pairs_f64(p.tile.pc, p.diffusion, p.kernel, p.grid, items, count, p.segs.p,
                          ctx->d_counter, ctx->stream);
   else
     e = launch_pairs_plain(p.tile.pc, p.kernel, p.grid, items, count, p.segs.p, ctx->d_counter,

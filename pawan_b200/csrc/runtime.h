@@ -225,7 +225,7 @@ constexpr size_t kShardAlign = 512;
 bool tile_supported(int precision, const PairConfig &pc, int kernel);
 
 // Whether a precision and tiling run on the symmetric pair engine (each
-// unordered pair once): the FP32 tilings with the packed far path.
+// unordered pair once): the packed FP32 tilings and FP64.
 bool tile_symmetric(int precision, const PairConfig &pc);
 // Device bytes of the symmetric engine's slots for one system of n particles.
 double sym_slot_bytes(size_t n, bool serving);

@@ -91,7 +91,7 @@ struct Request {
 // of a fixed chunk size that cover whole target tiles of at most 512 particles).
 double request_bytes(size_t n, int precision, const TileChoice &tile) {
   const double per = 5 * 48.0 + 16.0 + 4.0 + 64.0 + 64.0 + 1.0 + 48.0;
-  if (precision == PAWAN_PREC_F32 && tile_symmetric(precision, tile.pc))
+  if (tile_symmetric(precision, tile.pc))
     return (double)n * per + sym_slot_bytes(n, true) + 4096.0;
   const int tb = tile.pc.tb;
   const size_t chunk = ((kServeChunkSources + tb - 1) / tb) * (size_t)tb;
