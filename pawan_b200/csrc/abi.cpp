@@ -16,7 +16,7 @@ size_t pawan_system::device_bytes() const {
   return X.bytes() + Xs.bytes() + K1.bytes() + K2.bytes() + R.bytes() + rad.bytes() +
          vol.bytes() + wake_id.bytes() + pos32.bytes() + vor32.bytes() + poslo.bytes() +
          vorlo.bytes() + pos64.bytes() +
-         vor64.bytes() + diag_scratch.bytes() + diag_out.bytes() + Xc.bytes() + field.bytes() +
+         vor64.bytes() + diag_scratch.bytes() + diag_out.bytes() + Xc.bytes() + field.bytes() + columns.bytes() +
          (plan ? plan->partial.bytes() + plan->rates.bytes() + plan->tile_count.bytes() + plan->slots.bytes() : 0);
 }
 
@@ -439,38 +439,46 @@ int pawan_system_influence(pawan_system *sys, double *field, size_t size) {
   pawan_ctx *ctx = sys->ctx;
   if (!field || size != 3 * sys->n) return fail(ctx, PAWAN_ERR_INVALID, "field size must be 3*N");
   if (!sys->has_particles) return fail(ctx, PAWAN_ERR_STATE, "particles not set");
-  if (!sys->field.p) PAWAN_CUDA(ctx, sys->field.alloc(3 * sys->n));
+  // the field and, where the sources are split, the chunks' partial fields
+  const size_t chunks = (size_t)influence_chunks((int)sys->n);
+  if (!sys->field.p) PAWAN_CUDA(ctx, sys->field.alloc(3 * sys->n * (chunks > 1 ? 1 + chunks : 1)));
   // pos64 / vor64 hold pack(X) between API calls
-  PAWAN_CUDA(ctx, launch_influence((int)sys->n, sys->kernel, sys->pos64.p, sys->vor64.p, sys->field.p,
-                                   ctx->stream));
-  ctx->launches++;
+  PAWAN_CUDA(ctx, launch_influence((int)sys->n, sys->kernel, sys->pos64.p, sys->vor64.p,
+                                   sys->field.p + 3 * sys->n, sys->field.p, ctx->stream));
+  ctx->launches += chunks > 1 ? 2 : 1;
   PAWAN_CUDA(ctx, cudaMemcpyAsync(field, sys->field.p, 3 * sys->n * sizeof(double),
                                   cudaMemcpyDeviceToHost, ctx->stream));
   PAWAN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return PAWAN_OK;
 }
 
-// Device scratch bound of pawan_system_influence_columns (strength columns
-// plus their fields): larger requests run in several launches.
+// Device scratch bound of pawan_system_influence_columns (strength columns,
+// their fields and the source chunks' partial fields): larger requests run in
+// several launches.
 constexpr size_t kInfluenceColumnBytes = size_t(256) << 20;
 constexpr size_t kMaxInfluenceColumnsPerLaunch = size_t(65535) * kInfluenceColumnGroup;
 
-static int influence_columns(pawan_system *sys, size_t ncols, const double *alpha, double *field,
-                             DBuf<double> &cols, DBuf<double> &out) {
+// Scratch up to this size stays with the system for the next call (an
+// allocation and its free cost more than a launch at the usual sizes).
+constexpr size_t kInfluenceKeepBytes = size_t(64) << 20;
+
+static int influence_columns(pawan_system *sys, size_t ncols, const double *alpha, double *field) {
   pawan_ctx *ctx = sys->ctx;
   const size_t per = 3 * sys->n;
-  const size_t fit = std::max<size_t>(1, kInfluenceColumnBytes / (2 * per * sizeof(double)));
+  const size_t chunks = (size_t)influence_chunks((int)sys->n), parts = chunks > 1 ? chunks : 0;
+  const size_t fit = std::max<size_t>(1, kInfluenceColumnBytes / ((2 + parts) * per * sizeof(double)));
   const size_t chunk = std::min(ncols, std::min(fit, kMaxInfluenceColumnsPerLaunch));
-  PAWAN_CUDA(ctx, cols.alloc(chunk * per));
-  PAWAN_CUDA(ctx, out.alloc(chunk * per));
+  // strengths, fields, partial fields
+  if (sys->columns.n < (2 + parts) * chunk * per) PAWAN_CUDA(ctx, sys->columns.alloc((2 + parts) * chunk * per));
+  double *cols = sys->columns.p, *out = cols + chunk * per, *part = out + chunk * per;
   for (size_t c0 = 0; c0 < ncols; c0 += chunk) {
     const size_t nc = std::min(chunk, ncols - c0);
-    PAWAN_CUDA(ctx, cudaMemcpyAsync(cols.p, alpha + c0 * per, nc * per * sizeof(double),
+    PAWAN_CUDA(ctx, cudaMemcpyAsync(cols, alpha + c0 * per, nc * per * sizeof(double),
                                     cudaMemcpyHostToDevice, ctx->stream));
-    PAWAN_CUDA(ctx, launch_influence_columns((int)sys->n, (int)nc, sys->kernel, sys->pos64.p, cols.p,
-                                             out.p, ctx->stream));
-    ctx->launches++;
-    PAWAN_CUDA(ctx, cudaMemcpyAsync(field + c0 * per, out.p, nc * per * sizeof(double),
+    PAWAN_CUDA(ctx, launch_influence_columns((int)sys->n, (int)nc, sys->kernel, sys->pos64.p, cols, part, out,
+                                             ctx->stream));
+    ctx->launches += parts ? 2 : 1;
+    PAWAN_CUDA(ctx, cudaMemcpyAsync(field + c0 * per, out, nc * per * sizeof(double),
                                     cudaMemcpyDeviceToHost, ctx->stream));
   }
   return PAWAN_OK;
@@ -484,10 +492,10 @@ int pawan_system_influence_columns(pawan_system *sys, size_t ncols, const double
   if (!alpha || !field || size / ncols != 3 * sys->n || size % ncols != 0)
     return fail(ctx, PAWAN_ERR_INVALID, "alpha and field must hold ncols * 3N doubles");
   if (!sys->has_particles) return fail(ctx, PAWAN_ERR_STATE, "particles not set");
-  DBuf<double> cols, out;
-  const int st = influence_columns(sys, ncols, alpha, field, cols, out);
-  // the scratch is freed on return: wait for the copies and launches first
+  const int st = influence_columns(sys, ncols, alpha, field);
+  // large scratch is freed on return: wait for the copies and launches first
   const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+  if (sys->columns.bytes() > kInfluenceKeepBytes) sys->columns.reset();
   if (st != PAWAN_OK) return st;
   if (e != cudaSuccess) return cuda_fail(ctx, e, "influence columns");
   return PAWAN_OK;

@@ -819,7 +819,7 @@ int system_alloc(pawan_system *sys) {
   const size_t n = sys->n;
   if (sys->ordered_alloc) {
     for (auto *b : {&sys->X, &sys->Xs, &sys->K1, &sys->K2, &sys->R, &sys->rad, &sys->vol,
-                    &sys->diag_scratch, &sys->diag_out, &sys->Xc, &sys->field})
+                    &sys->diag_scratch, &sys->diag_out, &sys->Xc, &sys->field, &sys->columns})
       b->ordered_on(ctx->stream);
     sys->wake_id.ordered_on(ctx->stream);
     for (auto *b : {&sys->pos32, &sys->vor32, &sys->poslo, &sys->vorlo}) b->ordered_on(ctx->stream);
