@@ -117,7 +117,6 @@ struct SymSeg {
   const float4 *pos32, *vor32, *poslo, *vorlo;
   const double4 *pos64, *vor64;
   const float4 *boxes;  // (lo, hi) per tile
-  double *rates;        // [6][n]
   int n;
   double nu;
   float near2;          // squared box distance below which a tile pair is near
@@ -132,8 +131,8 @@ struct SymItem {
 };
 
 // One tile of the slot sums: `count` slots `stride` doubles apart from
-// slots[first], in that order, into rates[.][128 t ..] (added to what is there
-// when `add`).
+// slots[first], the quarters of them in order, added to the rates of an earlier
+// phase when `add`.
 struct SymSum {
   long long first;
   int stride, count, seg, t, add;

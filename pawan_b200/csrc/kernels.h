@@ -43,7 +43,7 @@ cudaError_t sym_f32_occupancy(bool group, bool diffusion, int kernel, int *block
 cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
                            const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s);
 // Sums the slots of each listed tile into its rates.
-cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const SymSeg *segs, const double *slots,
+cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const StageDesc *descs, const double *slots,
                             cudaStream_t s);
 
 // FP64 with the same algebra as the FP32 kernel ("tuned FP64"), on the symmetric
@@ -63,6 +63,11 @@ cudaError_t launch_pairs_plain(const PairConfig &c, int kernel, int grid, const 
 // Per-particle stage kernel (RK4 stage update from the summed rates, pack).
 cudaError_t launch_stage(int mode, int n_blocks, const StageItem *items, const StageDesc *descs,
                          cudaStream_t s);
+
+// The same for a symmetric plan whose slots one phase wrote: sums each listed
+// tile's slots and applies the stage (every mode but STAGE_PACK, STAGE_SHARD).
+cudaError_t launch_sum_stage(int mode, int n_sums, const SymSum *sums, const StageDesc *descs,
+                             const double *slots, cudaStream_t s);
 
 // Diagnostics of one system.  `scratch` holds at least diag_scratch_doubles(n)
 // doubles; out[0..10] = total vorticity (3), linear impulse (3), angular

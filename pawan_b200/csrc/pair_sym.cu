@@ -568,31 +568,6 @@ __global__ void __launch_bounds__(kThreads, kBlocks)
   tile_item<Pair32<DIFF, KERN>>(items, segs, jbase, slots);
 }
 
-// One block per tile: thread (k, q) sums component k of particle q over the
-// tile's slots in slot order.  HBM- or L2-bound reads of 6 KB rows, eight in
-// flight per thread.
-__global__ void __launch_bounds__(6 * kT)
-    sym_sums_kernel(const SymSum *__restrict__ sums, const SymSeg *__restrict__ segs,
-                    const double *__restrict__ slots) {
-  const SymSum s = sums[blockIdx.x];
-  const SymSeg &sg = segs[s.seg];
-  const int k = threadIdx.x / kT, i = s.t * kT + threadIdx.x % kT;
-  if (i >= sg.n) return;
-  const double *p = slots + s.first + threadIdx.x;
-  double *out = sg.rates + (size_t)k * sg.n + i;
-  double r = s.add ? *out : 0.0;
-  int c = 0;
-  for (; c + 8 <= s.count; c += 8) {
-    double v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = __ldcs(p + (size_t)(c + u) * s.stride);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) r += v[u];
-  }
-  for (; c < s.count; ++c) r += __ldcs(p + (size_t)c * s.stride);
-  *out = r;
-}
-
 SymKernel select(bool group, bool diffusion, int kernel) {
   if (kernel == KERNEL_GAUSSIAN) {
     if (group)
@@ -614,13 +589,6 @@ cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem
                            const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
   return sym_launch(select(group, diffusion, kernel), sym_smem_bytes(group, kStageBytes), items, n_items, segs,
                     jbase, slots, s);
-}
-
-cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const SymSeg *segs, const double *slots,
-                            cudaStream_t s) {
-  if (n_sums <= 0) return cudaSuccess;
-  sym_sums_kernel<<<n_sums, 6 * kT, 0, s>>>(sums, segs, slots);
-  return cudaGetLastError();
 }
 
 }  // namespace pawan

@@ -291,6 +291,10 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, bool serving) {
     for (size_t q = 0; q < k; ++q) sums[at + q].first += (long long)group_slots;
   }
   p.tile_slots = group_slots;
+  p.fused_sums = n_phases == 1;
+  for (auto *y : p.systems)
+    if (y->shard.active) p.fused_sums = false;
+  for (const SymSum &s : sums) p.slot_bytes += (double)s.count * 48.0 * kSymTile;
   if (items.size() > (size_t)INT32_MAX) return fail(ctx, PAWAN_ERR_INVALID, "too many work items");
   p.n_items = (int)items.size();
   std::vector<SymSeg> segs;
@@ -298,7 +302,7 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, bool serving) {
     const pawan_system *y = p.systems[s];
     const StageDesc &g = p.stage_host[s];
     segs.push_back(SymSeg{g.pos32, g.vor32, g.poslo, g.vorlo, g.pos64, g.vor64, g.boxes,
-                          const_cast<double *>(g.rates), (int)y->n, y->nu, (float)(y->r_near * y->r_near)});
+                          (int)y->n, y->nu, (float)(y->r_near * y->r_near)});
   }
   PAWAN_CUDA(ctx, p.slots.alloc(group_slots + tile_slots));
   PAWAN_CUDA(ctx, p.sym_items.alloc(items.size()));
@@ -583,8 +587,8 @@ static int launch_sym_range(pawan_ctx *ctx, Plan &p, int first, int count) {
                              p.sym_jbase.p, slots, ctx->stream));
       ctx->launches++;
     }
-    if (at > first && at <= first + count) {
-      PAWAN_CUDA(ctx, launch_sym_sums(p.sym_sums.p + ph.sum0, ph.sums, p.sym_segs.p, p.slots.p, ctx->stream));
+    if (!p.fused_sums && at > first && at <= first + count) {
+      PAWAN_CUDA(ctx, launch_sym_sums(p.sym_sums.p + ph.sum0, ph.sums, p.stage_descs.p, p.slots.p, ctx->stream));
       ctx->launches++;
     }
   }
@@ -644,7 +648,7 @@ static void note_repack(Plan &p) {
 
 // Algorithmic HBM bytes of one stage launch: per particle the rates (48
 // bytes: the pair kernel's summed chunks, or the gathered rates of a sharded
-// system), the FP64 state vectors the mode reads and writes, radius and
+// system; the slots themselves where the stage sums them), the FP64 state vectors the mode reads and writes, radius and
 // volume, and the 128 bytes of packed FP32 / FP64 tile data; 32 bytes of
 // bounding box per tile.  An RK4 stage is 336-384 bytes per particle.
 static double stage_bytes(const Plan &p, int mode) {
@@ -666,6 +670,10 @@ static double stage_bytes(const Plan &p, int mode) {
     }
     total += n * per;
   }
+  if (p.fused_sums && mode != STAGE_PACK) {
+    for (const pawan_system *y : p.systems) total -= 48.0 * (double)y->n;
+    total += p.slot_bytes;
+  }
   return total;
 }
 
@@ -677,7 +685,9 @@ int launch_stage_mode(pawan_ctx *ctx, Plan &p, int mode) {
     if (!e0 || !e1) return fail(ctx, PAWAN_ERR_CUDA, "cannot create profiling events");
     PAWAN_CUDA(ctx, cudaEventRecord(e0, ctx->stream));
   }
-  cudaError_t e = launch_stage(mode, p.n_stage_blocks, p.stage_items.p, p.stage_descs.p, ctx->stream);
+  cudaError_t e = p.fused_sums && mode != STAGE_PACK
+                      ? launch_sum_stage(mode, p.phases[0].sums, p.sym_sums.p, p.stage_descs.p, p.slots.p, ctx->stream)
+                      : launch_stage(mode, p.n_stage_blocks, p.stage_items.p, p.stage_descs.p, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "stage kernel launch");
   ctx->launches++;
   if (e0) {

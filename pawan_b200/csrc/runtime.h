@@ -183,6 +183,10 @@ struct Plan {
   DBuf<int> sym_jbase;
   DBuf<SymSum> sym_sums;
   DBuf<double> slots;
+  // the stage kernel sums the slots itself (one phase, not sharded): no
+  // launch for the sums, `rates` not used
+  bool fused_sums = false;
+  double slot_bytes = 0.0;  // bytes of all slots that one right-hand side sums
   size_t tile_slots = 0;  // doubles before the slots of the single-tile items
   DBuf<float4> boxes;
   DBuf<WorkItem> items;
