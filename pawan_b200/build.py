@@ -5,9 +5,9 @@
 Compiles every source under pawan_b200/csrc for sm_100a only
 (-gencode arch=compute_100a,code=sm_100a) into pawan_b200/_build/*.o and links
 pawan_b200/_lib/libpawan_b200.so (CUDA runtime linked statically).  Per-file
-flags: the FP32 pair kernel flushes denormals (--ftz=true); the plain FP64
-kernel does not contract multiply-adds (--fmad=false), like the reference's
-x86-64 build.  Rebuilds only what changed (sources or any header).
+flags: the FP32 pair kernels flush denormals (--ftz=true); the plain FP64 kernel
+does not contract multiply-adds (--fmad=false), like the reference's x86-64
+build, nor does the symmetric FP32 one, whose kernels must round alike.  Rebuilds only what changed (sources or any header).
 """
 from __future__ import annotations
 
@@ -31,7 +31,7 @@ COMMON = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-Wall",
                  "-I" + INCLUDE, "-I" + CSRC]
 PER_FILE = {
     "pair_f32.cu": ["--ftz=true"],
-    "pair_sym.cu": ["--ftz=true"],
+    "pair_sym.cu": ["--ftz=true", "--fmad=false"],
     "noalloc.cu": ["--ftz=true"],
     "pair_plain.cu": ["--fmad=false"],
 }

@@ -159,6 +159,23 @@ constexpr int kStageThreads = 256;
 
 
 #ifdef __CUDACC__
+// ---- programmatic dependent launch ----
+// A kernel launched with launch_dependent() (kernels.h) may start while the
+// kernel before it in the stream is still running.  It passes the pointer that
+// leads to everything that kernel writes through wait_previous(), which waits
+// for that kernel's end; only loads made through the returned pointer are sure
+// to come after it (the compiler may move others up).  Data written by earlier
+// kernels is read with plain loads, never through the read-only cache.
+// start_next() lets the kernel after it start as soon as every block has come
+// this far.
+template <class T>
+__device__ __forceinline__ T *wait_previous(T *p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("" : "+l"(p) : : "memory");
+  return p;
+}
+__device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- per-item partial sums and their in-launch reduction -------------------
 //
 // A work item (target tile x source chunk) of a segment with nchunks > 1

@@ -23,6 +23,23 @@ struct PairConfig {
   int split = 0;
 };
 
+// Launches f on s as a programmatic dependent of the kernel before it (its
+// launch overlaps that kernel's end; see wait_previous in device.cuh).
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*f)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, f, static_cast<P>(args)...);
+}
+
 inline int targets_per_block(const PairConfig &c) { return c.tb / c.p * c.r; }
 
 // `kernel` below is a SmoothingKernel (device.cuh).
@@ -39,9 +56,9 @@ cudaError_t launch_pairs_f32(const PairConfig &c, bool diffusion, int kernel, in
 // The symmetric pair engine (FP32): each unordered pair once, sums into the
 // items' slots; one block per item.  group: items over groups of kSymGroup
 // tiles, else over single tile pairs.
-cudaError_t sym_f32_occupancy(bool group, bool diffusion, int kernel, int *blocks_per_sm);
+cudaError_t sym_f32_occupancy(bool diffusion, int kernel, int *blocks_per_sm);
 cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
-                           const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s);
+                           int sm_count, const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s);
 // Sums the slots of each listed tile into its rates.
 cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const StageDesc *descs, const double *slots,
                             cudaStream_t s);
@@ -49,9 +66,9 @@ cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const StageDesc *des
 // FP64 with the same algebra as the FP32 kernel ("tuned FP64"), on the symmetric
 // engine whatever the tiling.
 bool pairs_f64_supported(const PairConfig &c, int kernel);
-cudaError_t sym_f64_occupancy(bool group, bool diffusion, int kernel, int *blocks_per_sm);
+cudaError_t sym_f64_occupancy(bool diffusion, int kernel, int *blocks_per_sm);
 cudaError_t launch_sym_f64(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
-                           const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s);
+                           int sm_count, const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s);
 
 // FP64, the reference's formula term by term (pow, divisions): the plain
 // FP64 comparator.

@@ -201,7 +201,7 @@ __device__ __forceinline__ void pairs64(const SymSeg &sg, int I, int J, int k0, 
 template <bool DIFF, int KERN>
 struct Pair64 {
   static constexpr int kStageBytes = kStage64;
-  static __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, char *st,
+  static __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, int, int, char *st,
                                                    int lane, double *accI, double *accJ) {
     if (I == J)
       pairs64<true, DIFF, KERN>(sg, I, J, k0, k1, st, lane, accI, accJ);
@@ -212,16 +212,16 @@ struct Pair64 {
 
 template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(kThreads, Shape64<KERN>::blocks)
-    sym_f64_group_kernel(const SymItem *__restrict__ items, const SymSeg *__restrict__ segs,
+    sym_f64_group_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
                          const int *__restrict__ jbase, double *__restrict__ slots) {
   group_item<Pair64<DIFF, KERN>>(items, segs, jbase, slots);
 }
 
 template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(kThreads, Shape64<KERN>::blocks)
-    sym_f64_tile_kernel(const SymItem *__restrict__ items, const SymSeg *__restrict__ segs,
+    sym_f64_tile_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
                         const int *__restrict__ jbase, double *__restrict__ slots) {
-  tile_item<Pair64<DIFF, KERN>>(items, segs, jbase, slots);
+  tile_item<Pair64<DIFF, KERN>, 1>(items, segs, jbase, slots);
 }
 
 template <int KERN>
@@ -242,14 +242,14 @@ bool pairs_f64_supported(const PairConfig &c, int kernel) {
          (kernel == KERNEL_HIGHORDER || kernel == KERNEL_GAUSSIAN);
 }
 
-cudaError_t sym_f64_occupancy(bool group, bool diffusion, int kernel, int *blocks_per_sm) {
-  return sym_occupancy(select(group, diffusion, kernel), sym_smem_bytes(group, kStage64), blocks_per_sm);
+cudaError_t sym_f64_occupancy(bool diffusion, int kernel, int *blocks_per_sm) {
+  return sym_occupancy(select(true, diffusion, kernel), sym_smem_bytes(SYM_GROUP, kStage64), blocks_per_sm);
 }
 
-cudaError_t launch_sym_f64(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
+cudaError_t launch_sym_f64(bool group, bool diffusion, int kernel, const SymItem *items, int n_items, int,
                            const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
-  return sym_launch(select(group, diffusion, kernel), sym_smem_bytes(group, kStage64), items, n_items, segs, jbase,
-                    slots, s);
+  return sym_launch(select(group, diffusion, kernel), kThreads,
+                    sym_smem_bytes(group ? SYM_GROUP : SYM_TILE, kStage64), items, n_items, segs, jbase, slots, s);
 }
 
 }  // namespace pawan

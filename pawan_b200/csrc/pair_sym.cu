@@ -41,6 +41,10 @@
 // one-sided; 20,011 unordered particles (near tile pairs only, mixed radii)
 // 0.87 ms against 1.48.
 //
+// Compiled without contraction of multiply-adds (every FMA is written out), so
+// that the kernels of the launch shapes below round alike and a system's result
+// does not depend on which of them runs it.
+//
 // Work items.  Large systems: a block of four warps takes a group of 4 tiles
 // (512 particles) against a run of groups; in round r warp w computes tile w
 // against tile (w + r) % 4 of the group, so no two warps add to one source's
@@ -151,20 +155,26 @@ __device__ __forceinline__ void far_block_z(const Stage &st, int lane, const Far
         else
           kernel_scalars(T[r].h + p.w, rsqrtf(r2 + (T[r].h + p.w)), ri, m, fh, dp);
         const float g = -fh * far_t(T[r], s, e);
-        float gx = g * dx, gy = g * dy, gz = g * dz;
+        add_wq(T[r], s, e, m, a[r], b);
         if (DIFF) {
           const float kd = kap * dp;
-          gx = fmaf(kd, fmaf(T[r].v, s.x, -s.w * T[r].ax), gx);
-          gy = fmaf(kd, fmaf(T[r].v, s.y, -s.w * T[r].ay), gy);
-          gz = fmaf(kd, fmaf(T[r].v, s.z, -s.w * T[r].az), gz);
+          const float gx = fmaf(kd, fmaf(T[r].v, s.x, -s.w * T[r].ax), g * dx);
+          const float gy = fmaf(kd, fmaf(T[r].v, s.y, -s.w * T[r].ay), g * dy);
+          const float gz = fmaf(kd, fmaf(T[r].v, s.z, -s.w * T[r].az), g * dz);
+          a[r].gx += gx;
+          a[r].gy += gy;
+          a[r].gz += gz;
+          b.gx += gx;
+          b.gy += gy;
+          b.gz += gz;
+        } else {
+          a[r].gx = fmaf(g, dx, a[r].gx);
+          a[r].gy = fmaf(g, dy, a[r].gy);
+          a[r].gz = fmaf(g, dz, a[r].gz);
+          b.gx = fmaf(g, dx, b.gx);
+          b.gy = fmaf(g, dy, b.gy);
+          b.gz = fmaf(g, dz, b.gz);
         }
-        add_wq(T[r], s, e, m, a[r], b);
-        a[r].gx += gx;
-        a[r].gy += gy;
-        a[r].gz += gz;
-        b.gx += gx;
-        b.gy += gy;
-        b.gz += gz;
       }
       // lane l holds the sums of source l ^ k and next takes l ^ (k + 1)
       const int k = kk + u;
@@ -246,29 +256,33 @@ __device__ __forceinline__ void fold_far(const Sums9 &s, float x, float y, float
   const double Qx = As2 * s.qx, Qy = As2 * s.qy, Qz = As2 * s.qz;
   const double xp = x, yp = y, zp = z;
   const double px = (double)ax + (double)lx, py = (double)ay + (double)ly, pz = (double)az + (double)lz;
-  acc[0] += (Qy * zp - Qz * yp) - As2 * s.wx;
-  acc[stride] += (Qz * xp - Qx * zp) - As2 * s.wy;
-  acc[2 * stride] += (Qx * yp - Qy * xp) - As2 * s.wz;
-  acc[3 * stride] += (py * Qz - pz * Qy) + g3 * s.gx;
-  acc[4 * stride] += (pz * Qx - px * Qz) + g3 * s.gy;
-  acc[5 * stride] += (px * Qy - py * Qx) + g3 * s.gz;
+  acc[0] += fma(-As2, (double)s.wx, fma(Qy, zp, -Qz * yp));
+  acc[stride] += fma(-As2, (double)s.wy, fma(Qz, xp, -Qx * zp));
+  acc[2 * stride] += fma(-As2, (double)s.wz, fma(Qx, yp, -Qy * xp));
+  acc[3 * stride] += fma(g3, (double)s.gx, fma(py, Qz, -pz * Qy));
+  acc[4 * stride] += fma(g3, (double)s.gy, fma(pz, Qx, -px * Qz));
+  acc[5 * stride] += fma(g3, (double)s.gz, fma(px, Qy, -py * Qx));
 }
 
 // A far tile pair: sub-blocks [k0, k1) of 32 sources of tile J against all
 // targets of tile I, R per lane and pass.  accI: the warp's [6][128] target
 // sums; accJ: [6][128] source sums of tile J.
 template <int CLS, bool UNI, bool DIFF, int KERN, int R>
-__device__ __forceinline__ void far_pair(const SymSeg &sg, int I, int J, int k0, int k1, float cx,
-                                         float cy, float cz, float hu, const Stage &st, int lane,
+__device__ __forceinline__ void far_pair(const SymSeg &sg, int I, int J, int k0, int k1, int ta, int tb,
+                                         float cx, float cy, float cz, float hu, const Stage &st, int lane,
                                          double *accI, double *accJ) {
+  if (R == 4) {  // one pass over all targets
+    if (ta > 0) return;
+    tb = kT;
+  }
   const double As2 = UNI ? kInv4Pi * 2.0 * (double)hu : kInv4Pi;
   const float kap = (CLS == FAR_Z && DIFF) ? (float)(UNI ? 80.0 * sg.nu / (double)hu : 5.0 * sg.nu) : 0.f;
-  const float4 *__restrict__ pos = sg.pos32;
-  const float4 *__restrict__ vor = sg.vor32;
-  const float4 *__restrict__ vlo = sg.vorlo;
+  const float4 *pos = sg.pos32;
+  const float4 *vor = sg.vor32;
+  const float4 *vlo = sg.vorlo;
   const int n = sg.n;
 #pragma unroll 1
-  for (int t0 = 0; t0 < kT; t0 += 32 * R) {
+  for (int t0 = ta; t0 < tb; t0 += 32 * R) {
     FarTarget T[R];
     Sums9 a[R];
 #pragma unroll
@@ -276,7 +290,7 @@ __device__ __forceinline__ void far_pair(const SymSeg &sg, int I, int J, int k0,
       const int i = I * kT + t0 + 32 * r + lane;
       T[r] = FarTarget{kPadTarget, kPadTarget, kPadTarget, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 1.f, 0.f};
       if (i < n) {
-        const float4 p = __ldg(pos + i), q = __ldg(vor + i);
+        const float4 p = pos[i], q = vor[i];
         const float x = p.x - cx, y = p.y - cy, z = p.z - cz;
         T[r] = FarTarget{x, y, z, q.x, q.y, q.z, fmaf(q.y, z, -q.z * y), fmaf(q.z, x, -q.x * z),
                          fmaf(q.x, y, -q.y * x), p.w, q.w};
@@ -289,9 +303,9 @@ __device__ __forceinline__ void far_pair(const SymSeg &sg, int I, int J, int k0,
       float4 p = make_float4(kPadSource, kPadSource, kPadSource, 1.f), q = make_float4(0.f, 0.f, 0.f, 0.f);
       float4 l = q, e = q;
       if (j < n) {
-        p = __ldg(pos + j);
-        q = __ldg(vor + j);
-        l = __ldg(vlo + j);
+        p = pos[j];
+        q = vor[j];
+        l = vlo[j];
         p.x -= cx;
         p.y -= cy;
         p.z -= cz;
@@ -317,7 +331,7 @@ __device__ __forceinline__ void far_pair(const SymSeg &sg, int I, int J, int k0,
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int i = I * kT + t0 + 32 * r + lane;
-      const float4 l = i < n ? __ldg(vlo + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 l = i < n ? vlo[i] : make_float4(0.f, 0.f, 0.f, 0.f);
       fold_far(a[r], T[r].x, T[r].y, T[r].z, T[r].ax, T[r].ay, T[r].az, l.x, l.y, l.z, As2, 3.0 * As2,
                accI + t0 + 32 * r + lane, kT);
     }
@@ -426,6 +440,8 @@ __device__ __forceinline__ void near_block(const Stage &st, int lane, const Near
   }
 }
 
+// (product and sum rounded apart: two passes over the targets add up alike
+// whether one warp or two make them)
 __device__ __forceinline__ void fold_near(const Sums6 &s, double As2, double *acc, int stride) {
   acc[0] += As2 * s.ux;
   acc[stride] += As2 * s.uy;
@@ -436,25 +452,25 @@ __device__ __forceinline__ void fold_near(const Sums6 &s, double As2, double *ac
 }
 
 template <bool UNI, bool DIAG, bool DIFF, int KERN>
-__device__ __forceinline__ void near_pair(const SymSeg &sg, int I, int J, int k0, int k1, float hu,
-                                          const Stage &st, int lane, double *accI, double *accJ) {
+__device__ __forceinline__ void near_pair(const SymSeg &sg, int I, int J, int k0, int k1, int ta, int tb,
+                                          float hu, const Stage &st, int lane, double *accI, double *accJ) {
   constexpr int R = 2;
   const double As2 = UNI ? kInv4Pi * 2.0 * (double)hu : kInv4Pi;
   const float kap = DIFF ? (float)(UNI ? 240.0 * sg.nu / (double)hu : 15.0 * sg.nu) : 0.f;
   const int n = sg.n;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
-  for (int t0 = 0; t0 < kT; t0 += 32 * R) {
+  for (int t0 = ta; t0 < tb; t0 += 32 * R) {
     NearTarget T[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int i = I * kT + t0 + 32 * r + lane;
       float4 p = make_float4(kPadTarget, kPadTarget, kPadTarget, 1.f), pl = zero, q = zero, l = zero;
       if (i < n) {
-        p = __ldg(sg.pos32 + i);
-        pl = __ldg(sg.poslo + i);
-        q = __ldg(sg.vor32 + i);
-        l = __ldg(sg.vorlo + i);
+        p = sg.pos32[i];
+        pl = sg.poslo[i];
+        q = sg.vor32[i];
+        l = sg.vorlo[i];
       }
       const float aa = fmaf(q.z, q.z, fmaf(q.y, q.y, q.x * q.x));
       T[r] = NearTarget{p.x, p.y, p.z, pl.x, pl.y, pl.z, q.x, q.y, q.z, l.x, l.y, l.z,
@@ -466,10 +482,10 @@ __device__ __forceinline__ void near_pair(const SymSeg &sg, int I, int J, int k0
       const int j = J * kT + 32 * k + lane;
       float4 p = make_float4(kPadSource, kPadSource, kPadSource, 1.f), pl = zero, q = zero, l = zero;
       if (j < n) {
-        p = __ldg(sg.pos32 + j);
-        pl = __ldg(sg.poslo + j);
-        q = __ldg(sg.vor32 + j);
-        l = __ldg(sg.vorlo + j);
+        p = sg.pos32[j];
+        pl = sg.poslo[j];
+        q = sg.vor32[j];
+        l = sg.vorlo[j];
       }
       st.s0[lane] = p;
       st.s1[lane] = make_float4(pl.x, pl.y, pl.z, q.w);
@@ -488,22 +504,23 @@ __device__ __forceinline__ void near_pair(const SymSeg &sg, int I, int J, int k0
   }
 }
 
-// One tile pair (I <= J), sub-blocks [k0, k1) of J's sources, in the class that
+// One tile pair (I <= J), sub-blocks [k0, k1) of J's sources and the targets [ta,
+// tb) of I (all of them, when ta is 0, in the classes of one pass), in the class that
 // the two tiles' boxes allow.  The classes and their bounds are pair_f32.cu's;
 // the far formulation is centred on the smaller of the two boxes, whose
 // half-diagonal bounds |x'_i| + |x'_j| by 3 |d| for every pair.
 template <bool DIFF, int KERN>
-__device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, const Stage &st,
-                                          int lane, double *accI, double *accJ) {
-  const float4 alo = __ldg(sg.boxes + 2 * I), ahi = __ldg(sg.boxes + 2 * I + 1);
-  const float4 blo = __ldg(sg.boxes + 2 * J), bhi = __ldg(sg.boxes + 2 * J + 1);
+__device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, int ta, int tb,
+                                          const Stage &st, int lane, double *accI, double *accJ) {
+  const float4 alo = sg.boxes[2 * I], ahi = sg.boxes[2 * I + 1];
+  const float4 blo = sg.boxes[2 * J], bhi = sg.boxes[2 * J + 1];
   const bool uni = KERN == KERNEL_HIGHORDER && alo.w == ahi.w && blo.w == bhi.w && alo.w == blo.w;
   const float hu = alo.w;
   if (I == J) {
     if (uni)
-      near_pair<true, true, DIFF, KERN>(sg, I, J, k0, k1, hu, st, lane, accI, accJ);
+      near_pair<true, true, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
     else
-      near_pair<false, true, DIFF, KERN>(sg, I, J, k0, k1, hu, st, lane, accI, accJ);
+      near_pair<false, true, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
     return;
   }
   const float gap2 = box_gap2(alo, ahi, blo, bhi);
@@ -512,9 +529,9 @@ __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0
   const bool far = gap2 > 0.f && gap2 >= sg.near2 && gap2 >= (first ? da : db);
   if (!far) {
     if (uni)
-      near_pair<true, false, DIFF, KERN>(sg, I, J, k0, k1, hu, st, lane, accI, accJ);
+      near_pair<true, false, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
     else
-      near_pair<false, false, DIFF, KERN>(sg, I, J, k0, k1, hu, st, lane, accI, accJ);
+      near_pair<false, false, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
     return;
   }
   const float4 lo = first ? alo : blo, hi = first ? ahi : bhi;
@@ -522,73 +539,83 @@ __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0
   const float sig2max = ahi.w + bhi.w;
   if (KERN == KERNEL_GAUSSIAN) {
     if (gap2 >= 49.f * sig2max)
-      far_pair<FAR_SER, false, DIFF, KERN, 4>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_SER, false, DIFF, KERN, 4>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_Z, false, DIFF, KERN, 2>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_Z, false, DIFF, KERN, 2>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     return;
   }
   if (gap2 >= 256.f * sig2max) {
     if (uni)
-      far_pair<FAR_SER, true, DIFF, KERN, 4>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_SER, true, DIFF, KERN, 4>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_SER, false, DIFF, KERN, 4>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_SER, false, DIFF, KERN, 4>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
   } else if (gap2 >= 36.f * sig2max) {
     if (uni)
-      far_pair<FAR_NZ, true, DIFF, KERN, 4>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_NZ, true, DIFF, KERN, 4>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_NZ, false, DIFF, KERN, 4>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_NZ, false, DIFF, KERN, 4>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
   } else {
     if (uni)
-      far_pair<FAR_Z, true, DIFF, KERN, 2>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_Z, true, DIFF, KERN, 2>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_Z, false, DIFF, KERN, 2>(sg, I, J, k0, k1, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_Z, false, DIFF, KERN, 2>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
   }
 }
 
 template <bool DIFF, int KERN>
 struct Pair32 {
   static constexpr int kStageBytes = ::pawan::kStageBytes;
-  static __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, char *st,
-                                                   int lane, double *accI, double *accJ) {
-    ::pawan::tile_pair<DIFF, KERN>(sg, I, J, k0, k1, stage_of(st), lane, accI, accJ);
+  static __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, int ta, int tb,
+                                                   char *st, int lane, double *accI, double *accJ) {
+    ::pawan::tile_pair<DIFF, KERN>(sg, I, J, k0, k1, ta, tb, stage_of(st), lane, accI, accJ);
   }
 };
 
 template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(kThreads, kBlocks)
-    sym_f32_group_kernel(const SymItem *__restrict__ items, const SymSeg *__restrict__ segs,
+    sym_f32_group_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
                          const int *__restrict__ jbase, double *__restrict__ slots) {
   group_item<Pair32<DIFF, KERN>>(items, segs, jbase, slots);
 }
 
 template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(kThreads, kBlocks)
-    sym_f32_tile_kernel(const SymItem *__restrict__ items, const SymSeg *__restrict__ segs,
+    sym_f32_tile_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
                         const int *__restrict__ jbase, double *__restrict__ slots) {
-  tile_item<Pair32<DIFF, KERN>>(items, segs, jbase, slots);
+  tile_item<Pair32<DIFF, KERN>, 1>(items, segs, jbase, slots);
 }
 
-SymKernel select(bool group, bool diffusion, int kernel) {
-  if (kernel == KERNEL_GAUSSIAN) {
-    if (group)
-      return diffusion ? &sym_f32_group_kernel<true, KERNEL_GAUSSIAN> : &sym_f32_group_kernel<false, KERNEL_GAUSSIAN>;
-    return diffusion ? &sym_f32_tile_kernel<true, KERNEL_GAUSSIAN> : &sym_f32_tile_kernel<false, KERNEL_GAUSSIAN>;
-  }
-  if (group)
-    return diffusion ? &sym_f32_group_kernel<true, KERNEL_HIGHORDER> : &sym_f32_group_kernel<false, KERNEL_HIGHORDER>;
-  return diffusion ? &sym_f32_tile_kernel<true, KERNEL_HIGHORDER> : &sym_f32_tile_kernel<false, KERNEL_HIGHORDER>;
+template <bool DIFF, int KERN>
+__global__ void __launch_bounds__(2 * kThreads, 1)
+    sym_f32_halves_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
+                          const int *__restrict__ jbase, double *__restrict__ slots) {
+  tile_item<Pair32<DIFF, KERN>, 2>(items, segs, jbase, slots);
+}
+
+template <bool DIFF, int KERN>
+SymKernel select_k(int shape) {
+  return shape == SYM_GROUP  ? &sym_f32_group_kernel<DIFF, KERN>
+         : shape == SYM_TILE ? &sym_f32_tile_kernel<DIFF, KERN>
+                             : &sym_f32_halves_kernel<DIFF, KERN>;
+}
+
+SymKernel select(int shape, bool diffusion, int kernel) {
+  if (kernel == KERNEL_GAUSSIAN)
+    return diffusion ? select_k<true, KERNEL_GAUSSIAN>(shape) : select_k<false, KERNEL_GAUSSIAN>(shape);
+  return diffusion ? select_k<true, KERNEL_HIGHORDER>(shape) : select_k<false, KERNEL_HIGHORDER>(shape);
 }
 
 }  // namespace
 
-cudaError_t sym_f32_occupancy(bool group, bool diffusion, int kernel, int *blocks_per_sm) {
-  return sym_occupancy(select(group, diffusion, kernel), sym_smem_bytes(group, kStageBytes), blocks_per_sm);
+cudaError_t sym_f32_occupancy(bool diffusion, int kernel, int *blocks_per_sm) {
+  return sym_occupancy(select(SYM_GROUP, diffusion, kernel), sym_smem_bytes(SYM_GROUP, kStageBytes), blocks_per_sm);
 }
 
-cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
+cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem *items, int n_items, int sm_count,
                            const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
-  return sym_launch(select(group, diffusion, kernel), sym_smem_bytes(group, kStageBytes), items, n_items, segs,
-                    jbase, slots, s);
+  const int shape = group ? SYM_GROUP : n_items <= sm_count ? SYM_TILE_HALVES : SYM_TILE;
+  return sym_launch(select(shape, diffusion, kernel), sym_threads(shape), sym_smem_bytes(shape, kStageBytes), items,
+                    n_items, segs, jbase, slots, s);
 }
 
 }  // namespace pawan

@@ -353,8 +353,8 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
   int bps = 0;
   p->sym = tile_symmetric(precision, tile.pc);
   if (p->sym) {
-    cudaError_t e = precision == PAWAN_PREC_F64 ? sym_f64_occupancy(true, p->diffusion, kernel, &bps)
-                                                : sym_f32_occupancy(true, p->diffusion, kernel, &bps);
+    cudaError_t e = precision == PAWAN_PREC_F64 ? sym_f64_occupancy(p->diffusion, kernel, &bps)
+                                                : sym_f32_occupancy(p->diffusion, kernel, &bps);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy query");
   } else {
     PAWAN_TRY(occupancy(ctx, precision, tile.pc, p->diffusion, kernel, &bps));
@@ -583,8 +583,8 @@ static int launch_sym_range(pawan_ctx *ctx, Plan &p, int first, int count) {
       if (lo >= hi) continue;
       double *slots = p.slots.p + (group ? 0 : p.tile_slots);
       const auto launch = p.precision == PAWAN_PREC_F64 ? launch_sym_f64 : launch_sym_f32;
-      PAWAN_CUDA(ctx, launch(group, p.diffusion, p.kernel, p.sym_items.p + lo, hi - lo, p.sym_segs.p,
-                             p.sym_jbase.p, slots, ctx->stream));
+      PAWAN_CUDA(ctx, launch(group, p.diffusion, p.kernel, p.sym_items.p + lo, hi - lo, ctx->sm_count,
+                             p.sym_segs.p, p.sym_jbase.p, slots, ctx->stream));
       ctx->launches++;
     }
     if (!p.fused_sums && at > first && at <= first + count) {

@@ -208,12 +208,11 @@ __global__ void __launch_bounds__(kStageThreads, kStageMinBlocks)
 constexpr int kSumThreads = 4 * kSymTile;
 
 // A block's quarter sums of a tile's slots: part[quarter][component][particle].
-__device__ __forceinline__ void sum_slots(const SymSum &s, const double *__restrict__ slots,
-                                          double (*part)[6][kSymTile]) {
+__device__ __forceinline__ void sum_slots(const SymSum &s, const double *slots, double (*part)[6][kSymTile]) {
   const int q = threadIdx.x & (kSymTile - 1), g = threadIdx.x / kSymTile;
   const int c0 = s.count * g / 4, c1 = s.count * (g + 1) / 4;
-  const double *p = slots + s.first + q;
   double a[6] = {0, 0, 0, 0, 0, 0};
+  const double *p = slots + s.first + q;
 #pragma unroll 4
   for (int c = c0; c < c1; ++c) {
 #pragma unroll
@@ -231,11 +230,12 @@ __device__ __forceinline__ double slot_sum(const double (*part)[6][kSymTile], in
 // The sums alone, into rates[.][128 t ..] (added to what is there when `add`):
 // sharded systems, whose rates are exchanged, and plans of several phases.
 __global__ void __launch_bounds__(kSumThreads)
-    sum_slots_kernel(const SymSum *__restrict__ sums, const StageDesc *__restrict__ descs,
-                     const double *__restrict__ slots) {
+    sum_slots_kernel(const SymSum *__restrict__ sums, const StageDesc *descs, const double *slots) {
   __shared__ double part[4][6][kSymTile];
   const SymSum s = sums[blockIdx.x];
-  const StageDesc &d = descs[s.seg];
+  start_next();
+  slots = wait_previous(slots);
+  const StageDesc &d = wait_previous(descs)[s.seg];
   sum_slots(s, slots, part);
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
@@ -249,14 +249,15 @@ __global__ void __launch_bounds__(kSumThreads)
 
 template <int MODE>
 __global__ void __launch_bounds__(kSumThreads)
-    sum_stage_kernel(const SymSum *__restrict__ sums, const StageDesc *__restrict__ descs,
-                     const double *__restrict__ slots) {
+    sum_stage_kernel(const SymSum *__restrict__ sums, const StageDesc *descs, const double *slots) {
   constexpr int kT = kSymTile, kC = 6 * kSymTile;
   __shared__ double part[4][6][kT];
   __shared__ double xs[kC];  // the new state: [x (128 x 3) | alpha (128 x 3)]
   __shared__ float box[8][kT / 32];
   const SymSum s = sums[blockIdx.x];
-  const StageDesc &d = descs[s.seg];
+  start_next();
+  slots = wait_previous(slots);
+  const StageDesc &d = wait_previous(descs)[s.seg];
   const int tid = threadIdx.x, q = tid & (kT - 1), g = tid / kT;
   const int l0 = s.t * kT;
   sum_slots(s, slots, part);
@@ -334,8 +335,7 @@ __global__ void __launch_bounds__(kSumThreads)
 cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const StageDesc *descs, const double *slots,
                             cudaStream_t s) {
   if (n_sums <= 0) return cudaSuccess;
-  sum_slots_kernel<<<n_sums, kSumThreads, 0, s>>>(sums, descs, slots);
-  return cudaGetLastError();
+  return launch_dependent(sum_slots_kernel, dim3(n_sums), kSumThreads, 0, s, sums, descs, slots);
 }
 
 cudaError_t launch_sum_stage(int mode, int n_sums, const SymSum *sums, const StageDesc *descs,
@@ -343,27 +343,20 @@ cudaError_t launch_sum_stage(int mode, int n_sums, const SymSum *sums, const Sta
   if (n_sums <= 0) return cudaSuccess;
   switch (mode) {
     case STAGE_RATES:
-      sum_stage_kernel<STAGE_RATES><<<n_sums, kSumThreads, 0, s>>>(sums, descs, slots);
-      break;
+      return launch_dependent(sum_stage_kernel<STAGE_RATES>, dim3(n_sums), kSumThreads, 0, s, sums, descs, slots);
     case STAGE_K1:
-      sum_stage_kernel<STAGE_K1><<<n_sums, kSumThreads, 0, s>>>(sums, descs, slots);
-      break;
+      return launch_dependent(sum_stage_kernel<STAGE_K1>, dim3(n_sums), kSumThreads, 0, s, sums, descs, slots);
     case STAGE_K2:
-      sum_stage_kernel<STAGE_K2><<<n_sums, kSumThreads, 0, s>>>(sums, descs, slots);
-      break;
+      return launch_dependent(sum_stage_kernel<STAGE_K2>, dim3(n_sums), kSumThreads, 0, s, sums, descs, slots);
     case STAGE_K3:
-      sum_stage_kernel<STAGE_K3><<<n_sums, kSumThreads, 0, s>>>(sums, descs, slots);
-      break;
+      return launch_dependent(sum_stage_kernel<STAGE_K3>, dim3(n_sums), kSumThreads, 0, s, sums, descs, slots);
     case STAGE_FINAL:
-      sum_stage_kernel<STAGE_FINAL><<<n_sums, kSumThreads, 0, s>>>(sums, descs, slots);
-      break;
+      return launch_dependent(sum_stage_kernel<STAGE_FINAL>, dim3(n_sums), kSumThreads, 0, s, sums, descs, slots);
     case STAGE_EULER:
-      sum_stage_kernel<STAGE_EULER><<<n_sums, kSumThreads, 0, s>>>(sums, descs, slots);
-      break;
+      return launch_dependent(sum_stage_kernel<STAGE_EULER>, dim3(n_sums), kSumThreads, 0, s, sums, descs, slots);
     default:
       return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 cudaError_t launch_stage(int mode, int n_blocks, const StageItem *items, const StageDesc *descs,
