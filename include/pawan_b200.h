@@ -249,9 +249,13 @@ int pawan_ctx_stream(pawan_ctx *ctx, void **stream);
 /* Many independent systems in one persistent pair launch per RK4 stage
  * (ragged segments), the four stages optionally captured in a CUDA graph.
  * No reference counterpart (the reference integrates one system at a time).
- * Each system's result matches its own pawan_system_rk4 result up to the
- * FP64 rounding of how its source chunks are grouped; graph and non-graph
- * runs of one batch agree bit for bit. */
+ * Graph and non-graph runs of one batch agree bit for bit.  Each system's
+ * result matches its own pawan_system_rk4 result up to the FP64 rounding of how
+ * its sums are grouped -- except that an FP32 batch whose tiling was neither
+ * set nor tuned keeps the one-sided pair kernel for its systems of more than
+ * 8,192 particles (high-order smoothing), which then agree within the FP32
+ * tolerance; pawan_batch_set_tiling with packed > 0 or pawan_batch_autotune
+ * takes them to the faster symmetric engine. */
 int pawan_batch_create(pawan_ctx *ctx, size_t n, pawan_system *const *systems, pawan_batch **out);
 void pawan_batch_destroy(pawan_batch *batch);
 /* dt[i] for system i (NULL: every system uses dt0). */

@@ -21,6 +21,7 @@ struct PairConfig {
   int minb = 0;
   int packed = 0;
   int split = 0;
+  bool onesided = false;  // {128, 1, 4, 1, 0, 2} on the one-sided packed kernel
 };
 
 // Launches f on s as a programmatic dependent of the kernel before it (its

@@ -1,8 +1,9 @@
 // All-pairs vortex-particle interaction, FP32 pair math with FP64
 // accumulation of per-tile partial sums, one side of each pair at a time: the
-// scalar tilings of the autotuner and the allocation-free solve.  The packed
-// tilings, the default among them, run on the symmetric engine (pair_sym.cu),
-// which shares the algebra and the tile classes derived here.
+// scalar tilings of the autotuner, the allocation-free solve and the larger
+// systems of a batch.  The packed tilings, the default among them, run on the
+// symmetric engine (pair_sym.cu), which shares the algebra and the tile classes
+// derived here.
 //
 // Reference: the pair physics of INTERACT (src/interaction/interaction_utils.h:363-407)
 // with KERNEL (src/interaction/highorder.h:48-60), summed over all pairs of a
@@ -222,6 +223,148 @@ __device__ __forceinline__ void tile_far(const float4 *__restrict__ sa,
   }
 }
 
+// ---- packed far path: two sources per FP32x2 instruction -----------------
+// For the larger systems of a batch, which keep this kernel (and its rounding;
+// batch_tile in abi.cpp says why).
+// The far formulation above with every FP32 operation on a pair of sources
+// (FFMA2/FMUL2/FADD2 issue once for two lanes' worth of work, halving the
+// issue slots the FMA pipe needs).  Shared-memory layout of a far tile, per
+// source pair k = (a, b) = (2k, 2k+1):
+//   f0[k] = (-x'_a, -x'_b, -y'_a, -y'_b)   f1[k] = (-z'_a, -z'_b, h_a, h_b)
+//   f2[k] = (ax_a, ax_b, ay_a, ay_b)       f3[k] = (az_a, az_b, v_a, v_b)
+//   f4[k] = (bx_a, bx_b, by_a, by_b)       f5[k] = (bz_a, bz_b)   (beta = alpha x x')
+// so every load yields operand pairs and the target enters each instruction
+// as a broadcast pair held in registers.  Signs are arranged so that no
+// operand needs negating in the loop (a negated pair costs two scalar
+// instructions): positions are stored negated, the target's strength is held
+// negated, and the loop accumulates -fh.
+
+struct Acc2 {
+  float2 wx, wy, wz;  // sum qh beta_j
+  float2 qx, qy, qz;  // sum qh alpha_j
+  float2 gx, gy, gz;  // sum -fh t d
+  float2 ex, ey, ez;  // sum Dp alpha_j
+  float2 ev;          // sum Dp v_j
+};
+
+struct Target2 {
+  float2 x, y, z;     // x'_i, broadcast
+  float2 h;           // h_i, broadcast
+  float2 na, nb, nc;  // -alpha_i (hi), broadcast
+  float2 gx, gy, gz;  // gamma_i = x'_i x alpha_i, broadcast
+};
+
+__device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
+
+template <bool DIFF, bool UNI, int NSRC, int U, bool NZ, bool SER = false>
+__device__ __forceinline__ void tile_far_packed(const float4 *__restrict__ f0,
+                                                const float4 *__restrict__ f1,
+                                                const float4 *__restrict__ f2,
+                                                const float4 *__restrict__ f3,
+                                                const float4 *__restrict__ f4,
+                                                const float2 *__restrict__ f5, const Target2 &T,
+                                                float hu, Acc2 &a) {
+  const float2 s2u = bc2(2.f * hu), h2 = bc2(hu), c240 = bc2(-480.f * hu);
+  const float2 nh2 = bc2(-hu), one2 = bc2(1.0f), nhalf2 = bc2(-0.5f);
+#pragma unroll U
+  for (int k = 0; k < NSRC / 2; ++k) {
+    const float4 A0 = f0[k], A1 = f1[k], A2 = f2[k], A3 = f3[k], A4 = f4[k];
+    const float2 bz = f5[k];
+    const float2 npx = make_float2(A0.x, A0.y), npy = make_float2(A0.z, A0.w);
+    const float2 npz = make_float2(A1.x, A1.y), hj = make_float2(A1.z, A1.w);
+    const float2 sx = make_float2(A2.x, A2.y), sy = make_float2(A2.z, A2.w);
+    const float2 sz = make_float2(A3.x, A3.y), sv = make_float2(A3.z, A3.w);
+    const float2 bx = make_float2(A4.x, A4.y), by = make_float2(A4.z, A4.w);
+    const float2 dx = __fadd2_rn(T.x, npx);
+    const float2 dy = __fadd2_rn(T.y, npy);
+    const float2 dz = __fadd2_rn(T.z, npz);
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    float2 qh, nfh, dp;
+    if (NZ && SER) {
+      // Z-free far field by the series in pairs (kernel_scalars_series):
+      // one MUFU rsqrt per source, 6 FP32x2 operations with one radius
+      const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+      const float2 ri2 = __fmul2_rn(ri, ri);
+      if (UNI) {
+        qh = __fmul2_rn(__fmul2_rn(__fmul2_rn(ri, ri2), __ffma2_rn(nh2, ri2, one2)), ri2);
+      } else {
+        const float2 e = __fmul2_rn(__fadd2_rn(T.h, hj), ri2);
+        qh = __fmul2_rn(__fmul2_rn(__fmul2_rn(e, ri), ri2), __ffma2_rn(nhalf2, e, one2));
+      }
+      nfh = __fmul2_rn(qh, ri2);
+      dp = make_float2(0.f, 0.f);
+    } else if (NZ) {
+      // Z-free far field in pairs (kernel_scalars_nz), no diffusion sums
+      if (UNI) {
+        const float2 sr = __fadd2_rn(r2, s2u);
+        const float2 y = make_float2(rcp_approx(sr.x), rcp_approx(sr.y));
+        const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+        const float2 ri2 = __fmul2_rn(ri, ri);
+        const float2 ph = __ffma2_rn(__fmul2_rn(h2, y), y, y);
+        qh = __fmul2_rn(__fmul2_rn(ph, ri), ri2);
+        nfh = __fmul2_rn(qh, ri2);
+      } else {
+        const float2 sig2 = __fadd2_rn(T.h, hj);
+        float qa, fa, qb, fb;
+        kernel_scalars_nz(sig2.x, r2.x, qa, fa);
+        kernel_scalars_nz(sig2.y, r2.y, qb, fb);
+        qh = make_float2(qa, qb);
+        nfh = make_float2(fa, fb);
+      }
+      dp = make_float2(0.f, 0.f);
+    } else if (UNI) {
+      // kernel_scalars_uniform in pairs, returning -fs
+      const float2 sr = __fadd2_rn(r2, s2u);
+      const float2 w = make_float2(rsqrtf(sr.x), rsqrtf(sr.y));
+      const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+      const float2 ri2 = __fmul2_rn(ri, ri);
+      const float2 y = __fmul2_rn(w, w);
+      const float2 u = __fmul2_rn(h2, y);
+      const float2 v = __fmul2_rn(u, w);
+      const float2 v2 = __fmul2_rn(v, v);
+      dp = __fmul2_rn(__fmul2_rn(v2, v2), v);
+      const float2 ph = __fmul2_rn(__ffma2_rn(u, y, y), ri);
+      qh = __fmul2_rn(__ffma2_rn(c240, dp, ph), ri2);
+      nfh = __fmul2_rn(__ffma2_rn(bc2(-80.f), dp, qh), ri2);
+    } else {
+      // kernel_scalars in pairs, returning -fh
+      const float2 sig2 = __fadd2_rn(T.h, hj);
+      const float2 sr = __fadd2_rn(r2, sig2);
+      const float2 w = make_float2(rsqrtf(sr.x), rsqrtf(sr.y));
+      const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+      const float2 w2 = __fmul2_rn(w, w);
+      const float2 uu = __fmul2_rn(sig2, w2);
+      const float2 v = __fmul2_rn(uu, w);
+      const float2 v2 = __fmul2_rn(v, v);
+      dp = __fmul2_rn(__fmul2_rn(v2, v2), v);
+      const float2 zc = __fmul2_rn(dp, sig2);
+      const float2 ph = __fmul2_rn(__fmul2_rn(__ffma2_rn(bc2(0.5f), uu, bc2(1.0f)), w2), ri);
+      const float2 ri2 = __fmul2_rn(ri, ri);
+      qh = __fmul2_rn(__fmul2_rn(__ffma2_rn(bc2(-7.5f), zc, ph), sig2), ri2);
+      nfh = __fmul2_rn(__ffma2_rn(bc2(-2.5f), zc, qh), ri2);
+    }
+    // alpha_i.(alpha_j x d) = alpha_j.gamma_i - alpha_i.beta_j
+    const float2 t = __ffma2_rn(T.nc, bz, __ffma2_rn(T.nb, by, __ffma2_rn(T.na, bx,
+                     __ffma2_rn(sz, T.gz, __ffma2_rn(sy, T.gy, __fmul2_rn(sx, T.gx))))));
+    const float2 nft = __fmul2_rn(nfh, t);
+    a.wx = __ffma2_rn(qh, bx, a.wx);
+    a.wy = __ffma2_rn(qh, by, a.wy);
+    a.wz = __ffma2_rn(qh, bz, a.wz);
+    a.qx = __ffma2_rn(qh, sx, a.qx);
+    a.qy = __ffma2_rn(qh, sy, a.qy);
+    a.qz = __ffma2_rn(qh, sz, a.qz);
+    a.gx = __ffma2_rn(nft, dx, a.gx);
+    a.gy = __ffma2_rn(nft, dy, a.gy);
+    a.gz = __ffma2_rn(nft, dz, a.gz);
+    if (DIFF && !NZ) {
+      a.ex = __ffma2_rn(dp, sx, a.ex);
+      a.ey = __ffma2_rn(dp, sy, a.ey);
+      a.ez = __ffma2_rn(dp, sz, a.ez);
+      a.ev = __ffma2_rn(dp, sv, a.ev);
+    }
+  }
+}
+
 // a*d - b*c to within 1.5 ulp of the result (Kahan's FMA algorithm): the
 // rounding error of b*c is recovered exactly by the second FMA.
 __device__ __forceinline__ float det2(float a, float b, float c, float d) {
@@ -326,19 +469,25 @@ __device__ __forceinline__ bool far_tiles(float gap2, float4 slo, float4 shi, fl
 // MINB: blocks per SM the register allocation is bounded for (occupancy).
 // KERN: the smoothing kernel (SmoothingKernel); the uniform-radius
 // specialisation exists for the high-order kernel only.
-template <int TB, int P, int R, int U, bool DIFF, int MINB, int KERN>
+// PK: the far path two sources per FP32x2 instruction (P = R = 1, high-order).
+template <int TB, int P, int R, int U, bool DIFF, int MINB, int KERN, bool PK = false>
 __global__ void __launch_bounds__(TB, MINB)
     pairs_f32_kernel(const WorkItem *__restrict__ items, int n_items,
                      const SegDesc *__restrict__ segs, int *__restrict__ next_item) {
+  static_assert(!PK || (P == 1 && R == 1 && KERN == KERNEL_HIGHORDER), "the packed far path's shape");
   constexpr int TG = TB / P;   // targets per block and per target row r
   constexpr int TPB = TG * R;  // targets per block
+  constexpr int FQ = PK ? TB / 2 : 1;
   // two-stage tile ring in dynamic shared memory (pair_f32_smem_bytes):
-  // sp, sv, spl, svl [2][TB] (pos32, vor32, poslo, vorlo as staged)
+  // sp, sv, spl, svl [2][TB] (pos32, vor32, poslo, vorlo as staged), then
+  // the packed far format fq [5][2][FQ] float4 and fz [2][FQ] float2
   extern __shared__ float4 smem_f32[];
   float4 *const sp = smem_f32;
   float4 *const sv = sp + 2 * TB;
   float4 *const spl = sv + 2 * TB;
   float4 *const svl = spl + 2 * TB;
+  float4 *const fq = svl + 2 * TB;
+  float2 *const fz = reinterpret_cast<float2 *>(fq + 10 * FQ);
   __shared__ int s_item, s_last;
   const int tid = threadIdx.x;
   const int g = tid % P;
@@ -424,8 +573,29 @@ __global__ void __launch_bounds__(TB, MINB)
         const float px = p0.x - cx, py = p0.y - cy, pz = p0.z - cz;
         const float bx = fmaf(p1.y, pz, -p1.z * py), by = fmaf(p1.z, px, -p1.x * pz),
                     bz = fmaf(p1.x, py, -p1.y * px);
-        sp[buf * TB + tid] = make_float4(px, py, pz, p0.w);
-        spl[buf * TB + tid] = make_float4(bx, by, bz, 0.f);
+        if (PK) {
+          const int k = tid >> 1, hf = tid & 1;
+          float *q0 = reinterpret_cast<float *>(fq + (0 * 2 + buf) * FQ + k);
+          float *q1 = reinterpret_cast<float *>(fq + (1 * 2 + buf) * FQ + k);
+          float *q2 = reinterpret_cast<float *>(fq + (2 * 2 + buf) * FQ + k);
+          float *q3 = reinterpret_cast<float *>(fq + (3 * 2 + buf) * FQ + k);
+          float *q4 = reinterpret_cast<float *>(fq + (4 * 2 + buf) * FQ + k);
+          float *q5 = reinterpret_cast<float *>(fz + buf * FQ + k);
+          q0[hf] = -px;
+          q0[2 + hf] = -py;
+          q1[hf] = -pz;
+          q1[2 + hf] = p0.w;
+          q2[hf] = p1.x;
+          q2[2 + hf] = p1.y;
+          q3[hf] = p1.z;
+          q3[2 + hf] = p1.w;
+          q4[hf] = bx;
+          q4[2 + hf] = by;
+          q5[hf] = bz;
+        } else {
+          sp[buf * TB + tid] = make_float4(px, py, pz, p0.w);
+          spl[buf * TB + tid] = make_float4(bx, by, bz, 0.f);
+        }
       }
       __syncthreads();
       if (t + 1 < ntiles)
@@ -441,7 +611,56 @@ __global__ void __launch_bounds__(TB, MINB)
         ay[r] = (double)T[r].bh + (double)bl[r];
         az[r] = (double)T[r].ch + (double)cl[r];
       }
-      if (!near) {
+      if (!near && PK) {
+        Target2 T2;
+        const float fx = T[0].xh - cx, fy = T[0].yh - cy, fzz = T[0].zh - cz;
+        T2.x = bc2(fx);
+        T2.y = bc2(fy);
+        T2.z = bc2(fzz);
+        T2.h = bc2(T[0].h);
+        T2.na = bc2(-T[0].ah);
+        T2.nb = bc2(-T[0].bh);
+        T2.nc = bc2(-T[0].ch);
+        T2.gx = bc2(fmaf(fy, T[0].ch, -fzz * T[0].bh));
+        T2.gy = bc2(fmaf(fzz, T[0].ah, -fx * T[0].ch));
+        T2.gz = bc2(fmaf(fx, T[0].bh, -fy * T[0].ah));
+        Acc2 b;
+        b.wx = b.wy = b.wz = b.qx = b.qy = b.qz = b.gx = b.gy = b.gz = make_float2(0.f, 0.f);
+        b.ex = b.ey = b.ez = b.ev = make_float2(0.f, 0.f);
+        const float4 *f0 = fq + buf * FQ, *f1 = fq + (2 + buf) * FQ, *f2 = fq + (4 + buf) * FQ,
+                     *f3 = fq + (6 + buf) * FQ, *f4 = fq + (8 + buf) * FQ;
+        const float2 *f5 = fz + buf * FQ;
+        if (ser && uni)
+          tile_far_packed<DIFF, true, TB, U, true, true>(f0, f1, f2, f3, f4, f5, T2, slo.w, b);
+        else if (ser)
+          tile_far_packed<DIFF, false, TB, U, true, true>(f0, f1, f2, f3, f4, f5, T2, 0.f, b);
+        else if (nz && uni)
+          tile_far_packed<DIFF, true, TB, U, true>(f0, f1, f2, f3, f4, f5, T2, slo.w, b);
+        else if (nz)
+          tile_far_packed<DIFF, false, TB, U, true>(f0, f1, f2, f3, f4, f5, T2, 0.f, b);
+        else if (uni)
+          tile_far_packed<DIFF, true, TB, U, false>(f0, f1, f2, f3, f4, f5, T2, slo.w, b);
+        else
+          tile_far_packed<DIFF, false, TB, U, false>(f0, f1, f2, f3, f4, f5, T2, 0.f, b);
+        const double s2 = uni ? 2.0 * (double)slo.w : 1.0;
+        const double As2 = A * s2;
+        const double cd = uni ? 32.0 * cnu : cnu;
+        const double Qx = As2 * (b.qx.x + b.qx.y), Qy = As2 * (b.qy.x + b.qy.y),
+                     Qz = As2 * (b.qz.x + b.qz.y);
+        const double xp = fx, yp = fy, zp = fzz;
+        ou[0][0] += (Qy * zp - Qz * yp) - As2 * (b.wx.x + b.wx.y);
+        ou[0][1] += (Qz * xp - Qx * zp) - As2 * (b.wy.x + b.wy.y);
+        ou[0][2] += (Qx * yp - Qy * xp) - As2 * (b.wz.x + b.wz.y);
+        oa[0][0] += (ay[0] * Qz - az[0] * Qy) - 3.0 * As2 * (b.gx.x + b.gx.y);
+        oa[0][1] += (az[0] * Qx - ax[0] * Qz) - 3.0 * As2 * (b.gy.x + b.gy.y);
+        oa[0][2] += (ax[0] * Qy - ay[0] * Qx) - 3.0 * As2 * (b.gz.x + b.gz.y);
+        if (DIFF && !nz) {
+          const double v = T[0].v, ev = b.ev.x + b.ev.y;
+          oa[0][0] += cd * (v * (b.ex.x + b.ex.y) - ev * ax[0]);
+          oa[0][1] += cd * (v * (b.ey.x + b.ey.y) - ev * ay[0]);
+          oa[0][2] += cd * (v * (b.ez.x + b.ez.y) - ev * az[0]);
+        }
+      } else if (!near) {
         FarTarget F[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -589,6 +808,9 @@ KernelFn select_gaussian(const PairConfig &c) {
 #undef PAWAN_F32_CASE_K
 
 KernelFn select(const PairConfig &c, bool diffusion, int kernel) {
+  if (c.onesided && c.packed == 2 && kernel == KERNEL_HIGHORDER && c.tb == 128 && c.p == 1 && c.r == 1)
+    return diffusion ? &pairs_f32_kernel<128, 1, 1, 4, true, 4, KERNEL_HIGHORDER, true>
+                     : &pairs_f32_kernel<128, 1, 1, 4, false, 4, KERNEL_HIGHORDER, true>;
   if (c.packed != 0 || c.split != 0) return nullptr;
   if (kernel == KERNEL_GAUSSIAN) return diffusion ? select_gaussian<true>(c) : select_gaussian<false>(c);
   if (kernel == KERNEL_HIGHORDER)
@@ -615,8 +837,11 @@ bool symmetric_tiling(const PairConfig &c, int kernel) {
   return false;
 }
 
-// Dynamic shared memory of a tiling: the staged ring.
-size_t smem_bytes(const PairConfig &c) { return 8 * (size_t)c.tb * sizeof(float4); }
+// Dynamic shared memory of a tiling: the staged ring plus the packed far format.
+size_t smem_bytes(const PairConfig &c) {
+  const size_t fq = c.packed ? (size_t)c.tb / 2 : 1;
+  return 8 * (size_t)c.tb * sizeof(float4) + 10 * fq * sizeof(float4) + 2 * fq * sizeof(float2);
+}
 
 // Opts a kernel in to its dynamic shared memory beyond the default 48 KB (once
 // per kernel and device).
@@ -636,7 +861,7 @@ cudaError_t prepare(KernelFn f, size_t bytes) {
 }  // namespace
 
 bool pairs_f32_supported(const PairConfig &c, int kernel) {
-  return c.packed != 0 ? symmetric_tiling(c, kernel) : select(c, true, kernel) != nullptr;
+  return c.packed != 0 && !c.onesided ? symmetric_tiling(c, kernel) : select(c, true, kernel) != nullptr;
 }
 
 cudaError_t pairs_f32_occupancy(const PairConfig &c, bool diffusion, int kernel, int *blocks_per_sm) {

@@ -86,7 +86,7 @@ bool Plan::stale() const {
 }
 
 bool tile_symmetric(int precision, const PairConfig &pc) {
-  return precision == PAWAN_PREC_F64 || (precision == PAWAN_PREC_F32 && pc.packed > 0);
+  return precision == PAWAN_PREC_F64 || (precision == PAWAN_PREC_F32 && pc.packed > 0 && !pc.onesided);
 }
 
 static int occupancy(pawan_ctx *ctx, int precision, const PairConfig &pc, bool diffusion,

@@ -67,7 +67,7 @@ struct TileChoice {
   int items_per_slot = 16;
   bool operator==(const TileChoice &o) const {
     return pc.tb == o.pc.tb && pc.p == o.pc.p && pc.r == o.pc.r && pc.unroll == o.pc.unroll &&
-           pc.minb == o.pc.minb && pc.packed == o.pc.packed && pc.split == o.pc.split &&
+           pc.minb == o.pc.minb && pc.packed == o.pc.packed && pc.split == o.pc.split && pc.onesided == o.pc.onesided &&
            items_per_slot == o.items_per_slot;
   }
 };

@@ -56,8 +56,10 @@ def test_against_restatement(ctx, n, mixed, kernel):
 
 
 def test_batch_of_both_decompositions_matches_alone(ctx):
-    """Systems on either side of the edge in one launch sequence."""
-    sizes = [EDGE + 1, 129, EDGE, 2000]
+    """Systems on either side of the edge in one launch sequence: with a packed
+    tiling set, all on the symmetric engine; untuned, those of more than 8,192
+    particles on the one-sided kernel."""
+    sizes = [EDGE + 1, 129, 2000, 8192, 8193]
     alone, systems = [], []
     for k, n in enumerate(sizes):
         arrays = particles(n, seed=90 + k)
@@ -66,8 +68,31 @@ def test_batch_of_both_decompositions_matches_alone(ctx):
         systems.append(s)
     b = Batch(ctx, systems)
     b.solve()
+    for n, s, r in zip(sizes, systems, alone):
+        got = s.get_rates()
+        assert np.array_equal(got, r) == (n <= 8192)
+        assert rms_rel(got, r) <= TOL_F32_RMS
+    b.set_config(128, unroll=4, packed=2)
+    b.solve()
     for s, r in zip(systems, alone):
         assert np.array_equal(s.get_rates(), r)  # a system's slots and their order are its own
+
+
+def test_untuned_batch_steps_both_kinds_of_system(ctx):
+    """Per-system dt, graph and eager, over the two plans of an untuned batch."""
+    scs = [g.single_ring(n_stations=k, seed=95 + k, nu=1e-3) for k in (1100, 40, 1030)]  # N = 8,800, 320, 8,240
+    dts = np.array([0.001, 0.002, 0.003])
+    runs = []
+    for graph in (False, True):
+        systems = [System.from_scenario(ctx, sc, "f32") for sc in scs]
+        Batch(ctx, systems).rk4(dts, 2, use_graph=graph)
+        runs.append([s.get_states() for s in systems])
+    for sc, dt, a, b in zip(scs, dts, *runs):
+        assert np.array_equal(a, b)
+        solo = System.from_scenario(ctx, sc, "f32")
+        solo.rk4(dt, 2)
+        st0 = sc.state()
+        assert rms_rel(a - st0, solo.get_states() - st0) <= TOL_F32_RMS
 
 
 def test_sharded_groups_match_unsharded(ctx):
