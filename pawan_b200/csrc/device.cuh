@@ -166,13 +166,26 @@ constexpr int kStageThreads = 256;
 // for that kernel's end; only loads made through the returned pointer are sure
 // to come after it (the compiler may move others up).  Data written by earlier
 // kernels is read with plain loads, never through the read-only cache.
+// Work tables (items, segments, stage descriptions) are written by copies alone,
+// which no kernel after them overtakes, and may be read before the wait: their
+// latency is then hidden in it.
 // start_next() lets the kernel after it start as soon as every block has come
 // this far.
 template <class T>
-__device__ __forceinline__ T *wait_previous(T *p) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+__device__ __forceinline__ T *launder_pointer(T *p) {
   asm volatile("" : "+l"(p) : : "memory");
   return p;
+}
+template <class T>
+__device__ __forceinline__ T *wait_previous(T *p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  return launder_pointer(p);
+}
+// The same for several pointers.
+template <class... T>
+__device__ __forceinline__ void wait_previous_for(T *&...p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  ((p = launder_pointer(p)), ...);
 }
 __device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -15,6 +15,8 @@
 // stage modes read every particle's rates from the gathered buffer.
 // Products and sums use __dmul_rn/__dadd_rn so no multiply-add is contracted,
 // keeping the update bit-identical to the reference's for equal rates.
+#include <cuda_pipeline.h>
+
 #include "device.cuh"
 #include "kernels.h"
 
@@ -204,7 +206,17 @@ __global__ void __launch_bounds__(kStageThreads, kStageMinBlocks)
 // the state vectors, where one thread per particle strides by three -- and
 // packs the tile.  In place of a launch for the sums and one for the stage: a
 // right-hand side at N = 2,048 20.6 us against 24.6, at 512 20.6 against 24.6
-// (eager RK4 on one B200).
+// (eager RK4 on one B200, before launches overlapped).
+//
+// What bounds it: the latency of its chain of loads (small systems) and the L2's
+// bytes in flight (a tile of N = 16,384 has 128 slots of 6 KB).  The state is
+// loaded beside the slots, by copies to shared memory that hold no registers,
+// and the registers are left unbounded (some 95): more slot loads in flight, and
+// one block to an SM -- with 40 registers the blocks, which start while the pair
+// kernel's last ones run, gather three to an SM on the SMs that are free first.
+// One RK4 right-hand side, 40 registers / unbounded: N = 2,048 17.3 / 14.7 us,
+// 8,192 84.0 / 79.2, 16,384 285 / 265.  (8-byte copies of the slots to shared
+// memory, three or four slots deep: 18.1, 88.2, 283.)
 constexpr int kSumThreads = 4 * kSymTile;
 
 // A block's quarter sums of a tile's slots: part[quarter][component][particle].
@@ -229,7 +241,7 @@ __device__ __forceinline__ double slot_sum(const double (*part)[6][kSymTile], in
 
 // The sums alone, into rates[.][128 t ..] (added to what is there when `add`):
 // sharded systems, whose rates are exchanged, and plans of several phases.
-__global__ void __launch_bounds__(kSumThreads)
+__global__ void __launch_bounds__(kSumThreads, 1)
     sum_slots_kernel(const SymSum *__restrict__ sums, const StageDesc *descs, const double *slots) {
   __shared__ double part[4][6][kSymTile];
   const SymSum s = sums[blockIdx.x];
@@ -248,50 +260,69 @@ __global__ void __launch_bounds__(kSumThreads)
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kSumThreads)
+__global__ void __launch_bounds__(kSumThreads, 1)
     sum_stage_kernel(const SymSum *__restrict__ sums, const StageDesc *descs, const double *slots) {
   constexpr int kT = kSymTile, kC = 6 * kSymTile;
+  constexpr bool kOne = MODE == STAGE_FINAL, kTwo = MODE == STAGE_FINAL || MODE == STAGE_K3;
   __shared__ double part[4][6][kT];
-  __shared__ double xs[kC];  // the new state: [x (128 x 3) | alpha (128 x 3)]
+  __shared__ double xs[kC];  // the state, then the new one: [x (128 x 3) | alpha (128 x 3)]
+  __shared__ double k1[kOne ? kC : 1], k2[kTwo ? kC : 1];
   __shared__ float box[8][kT / 32];
   const SymSum s = sums[blockIdx.x];
+  const StageDesc *const desc = descs + s.seg;
+  const int n = desc->n;
+  const double *X = desc->X, *K1 = desc->K1, *K2 = desc->K2;
   start_next();
-  slots = wait_previous(slots);
-  const StageDesc &d = wait_previous(descs)[s.seg];
+  wait_previous_for(slots, X, K1, K2);
   const int tid = threadIdx.x, q = tid & (kT - 1), g = tid / kT;
   const int l0 = s.t * kT;
+  // the values the update starts from, in flight beside the slots and held by no register
+  if (MODE != STAGE_RATES) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int e = tid + u * kSumThreads;
+      const int h = e >= kC / 2 ? 1 : 0, f = e - h * (kC / 2);  // x or alpha, component within it
+      if (e >= kC || l0 + f / 3 >= n) continue;
+      const size_t at = (size_t)h * 3 * n + 3 * (size_t)l0 + f;
+      __pipeline_memcpy_async(xs + e, X + at, sizeof(double));
+      if (kOne) __pipeline_memcpy_async(k1 + e, K1 + at, sizeof(double));
+      if (kTwo) __pipeline_memcpy_async(k2 + e, K2 + at, sizeof(double));
+    }
+    __pipeline_commit();
+  }
   sum_slots(s, slots, part);
+  if (MODE != STAGE_RATES) __pipeline_wait_prior(0);  // (each thread reads its own copies)
+  const StageDesc &d = *launder_pointer(desc);
   const double dt = d.dt;
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     const int e = tid + u * kSumThreads;
     if (e >= kC) break;
-    const int h = e >= kC / 2 ? 1 : 0, f = e - h * (kC / 2);  // x or alpha, component within it
-    const int i = f / 3, k = 3 * h + (f - 3 * i);
-    if (l0 + i >= d.n) continue;
-    const size_t at = (size_t)h * 3 * d.n + 3 * (size_t)l0 + f;
-    const double r = slot_sum(part, k, i);
+    const int h = e >= kC / 2 ? 1 : 0, f = e - h * (kC / 2);
+    const int i = f / 3;
+    if (l0 + i >= n) continue;
+    const size_t at = (size_t)h * 3 * n + 3 * (size_t)l0 + f;
+    const double r = slot_sum(part, 3 * h + (f - 3 * i), i);
+    double x = 0.0;
     if (MODE == STAGE_RATES) {
       d.R[at] = r;
       continue;
     }
-    double x = 0.0;
     if (MODE == STAGE_K1 || MODE == STAGE_K2) {
-      double *K = (MODE == STAGE_K1) ? d.K1 : d.K2;
-      K[at] = r;
-      x = __dadd_rn(__dmul_rn(r, 0.5 * dt), d.X[at]);
+      (MODE == STAGE_K1 ? d.K1 : d.K2)[at] = r;
+      x = __dadd_rn(__dmul_rn(r, 0.5 * dt), xs[e]);
       d.Xs[at] = x;
     } else if (MODE == STAGE_K3) {
-      d.K2[at] = __dadd_rn(d.K2[at], r);
-      x = __dadd_rn(__dmul_rn(r, dt), d.X[at]);
+      d.K2[at] = __dadd_rn(k2[e], r);
+      x = __dadd_rn(__dmul_rn(r, dt), xs[e]);
       d.Xs[at] = x;
     } else if (MODE == STAGE_FINAL) {
-      const double a = __dmul_rn(__dadd_rn(d.K1[at], r), dt / 6.);
-      const double b = __dmul_rn(d.K2[at], dt / 3.);
-      x = __dadd_rn(d.X[at], __dadd_rn(a, b));
+      const double a = __dmul_rn(__dadd_rn(k1[e], r), dt / 6.);
+      const double b = __dmul_rn(k2[e], dt / 3.);
+      x = __dadd_rn(xs[e], __dadd_rn(a, b));
       d.X[at] = x;
     } else {  // STAGE_EULER
-      x = __dadd_rn(d.X[at], __dmul_rn(r, dt));
+      x = __dadd_rn(xs[e], __dmul_rn(r, dt));
       d.X[at] = x;
     }
     xs[e] = x;
@@ -300,7 +331,7 @@ __global__ void __launch_bounds__(kSumThreads)
   __syncthreads();
   // pack: each quarter of the block writes one pair of arrays
   const int l = l0 + q;
-  const bool has = l < d.n;
+  const bool has = l < n;
   const double x0 = xs[3 * q], x1 = xs[3 * q + 1], x2 = xs[3 * q + 2];
   const double a0 = xs[kC / 2 + 3 * q], a1 = xs[kC / 2 + 3 * q + 1], a2 = xs[kC / 2 + 3 * q + 2];
   if (g == 0) {
