@@ -3,6 +3,10 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
+#include <set>
+#include <utility>
+
 #include "device.cuh"
 
 namespace pawan {
@@ -24,21 +28,46 @@ struct PairConfig {
   bool onesided = false;  // {128, 1, 4, 1, 0, 2} on the one-sided packed kernel
 };
 
+// Opts a kernel in to its dynamic shared memory beyond the default 48 KB (once
+// per kernel and device).
+inline cudaError_t allow_dynamic_smem(const void *f, size_t bytes) {
+  static std::mutex mu;
+  static std::set<std::pair<int, const void *>> done;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(mu);
+  if (done.count({dev, f})) return cudaSuccess;
+  e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) done.insert({dev, f});
+  return e;
+}
+
 // Launches f on s as a programmatic dependent of the kernel before it (its
-// launch overlaps that kernel's end; see wait_previous in device.cuh).
+// launch overlaps that kernel's end; see wait_previous in device.cuh), in
+// clusters of `cluster` blocks.
 template <class... P, class... A>
-inline cudaError_t launch_dependent(void (*f)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
-  cudaLaunchAttribute at[1];
+inline cudaError_t launch_dependent_clusters(void (*f)(P...), int cluster, dim3 grid, int threads, size_t smem,
+                                             cudaStream_t s, A... args) {
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t c = {};
   c.gridDim = grid;
   c.blockDim = dim3(threads);
   c.dynamicSmemBytes = smem;
   c.stream = s;
   c.attrs = at;
-  c.numAttrs = 1;
+  c.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&c, f, static_cast<P>(args)...);
+}
+
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*f)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  return launch_dependent_clusters(f, 1, grid, threads, smem, s, args...);
 }
 
 inline int targets_per_block(const PairConfig &c) { return c.tb / c.p * c.r; }

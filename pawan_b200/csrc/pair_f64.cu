@@ -221,7 +221,7 @@ template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(kThreads, Shape64<KERN>::blocks)
     sym_f64_tile_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
                         const int *__restrict__ jbase, double *__restrict__ slots) {
-  tile_item<Pair64<DIFF, KERN>, 1>(items, segs, jbase, slots);
+  tile_item<Pair64<DIFF, KERN>>(items, segs, jbase, slots);
 }
 
 template <int KERN>
@@ -248,8 +248,8 @@ cudaError_t sym_f64_occupancy(bool diffusion, int kernel, int *blocks_per_sm) {
 
 cudaError_t launch_sym_f64(bool group, bool diffusion, int kernel, const SymItem *items, int n_items, int,
                            const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
-  return sym_launch(select(group, diffusion, kernel), kThreads,
-                    sym_smem_bytes(group ? SYM_GROUP : SYM_TILE, kStage64), items, n_items, segs, jbase, slots, s);
+  return sym_launch(select(group, diffusion, kernel), group ? SYM_GROUP : SYM_TILE, kStage64, items, n_items, segs,
+                    jbase, slots, s);
 }
 
 }  // namespace pawan

@@ -49,7 +49,8 @@
 // (512 particles) against a run of groups; in round r warp w computes tile w
 // against tile (w + r) % 4 of the group, so no two warps add to one source's
 // FP64 sums at a time and their order is fixed.  Small systems: one tile pair
-// per block, each warp 32 of its sources.  An item writes its target-side sums
+// per block, each warp 32 of its sources (launches of few tile pairs: eight warps,
+// in one block or a cluster of two).  An item writes its target-side sums
 // once and its source-side sums per group, each to a slot of its own; a
 // separate kernel sums a particle's slots in a fixed order, so results do not
 // depend on scheduling.
@@ -582,21 +583,29 @@ template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(kThreads, kBlocks)
     sym_f32_tile_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
                         const int *__restrict__ jbase, double *__restrict__ slots) {
-  tile_item<Pair32<DIFF, KERN>, 1>(items, segs, jbase, slots);
+  tile_item<Pair32<DIFF, KERN>>(items, segs, jbase, slots);
 }
 
 template <bool DIFF, int KERN>
-__global__ void __launch_bounds__(2 * kThreads, 1)
-    sym_f32_halves_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
+__global__ void __launch_bounds__(Spread<1>::threads, 1)
+    sym_f32_wide_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
+                        const int *__restrict__ jbase, double *__restrict__ slots) {
+  spread_item<Pair32<DIFF, KERN>, 1>(items, segs, jbase, slots);
+}
+
+template <bool DIFF, int KERN>
+__global__ void __launch_bounds__(Spread<2>::threads, 2)
+    sym_f32_spread_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
                           const int *__restrict__ jbase, double *__restrict__ slots) {
-  tile_item<Pair32<DIFF, KERN>, 2>(items, segs, jbase, slots);
+  spread_item<Pair32<DIFF, KERN>, 2>(items, segs, jbase, slots);
 }
 
 template <bool DIFF, int KERN>
 SymKernel select_k(int shape) {
   return shape == SYM_GROUP  ? &sym_f32_group_kernel<DIFF, KERN>
          : shape == SYM_TILE ? &sym_f32_tile_kernel<DIFF, KERN>
-                             : &sym_f32_halves_kernel<DIFF, KERN>;
+         : shape == SYM_WIDE ? &sym_f32_wide_kernel<DIFF, KERN>
+                             : &sym_f32_spread_kernel<DIFF, KERN>;
 }
 
 SymKernel select(int shape, bool diffusion, int kernel) {
@@ -613,9 +622,17 @@ cudaError_t sym_f32_occupancy(bool diffusion, int kernel, int *blocks_per_sm) {
 
 cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem *items, int n_items, int sm_count,
                            const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
-  const int shape = group ? SYM_GROUP : n_items <= sm_count ? SYM_TILE_HALVES : SYM_TILE;
-  return sym_launch(select(shape, diffusion, kernel), sym_threads(shape), sym_smem_bytes(shape, kStageBytes), items,
-                    n_items, segs, jbase, slots, s);
+  // Up to one tile pair per SM a launch lasts as long as one tile pair's chain of
+  // steps: eight warps take it in less time than four, and two SMs in less than
+  // one (two warps a scheduler issue at 0.8 per cycle, one alone at 0.6).  One
+  // right-hand side as an RK4 stage runs it, wide / spread: n = 64 13.5 / 10.9 us,
+  // 512 16.2 / 13.0, 1,408 17.5 / 14.5.  With more than two blocks per SM-pair the
+  // clusters are not placed evenly: 2,048 19.1 / 21.8 (four warps: 24.6).
+  const int shape = group                     ? SYM_GROUP
+                    : 2 * n_items <= sm_count ? SYM_SPREAD
+                    : n_items <= sm_count     ? SYM_WIDE
+                                              : SYM_TILE;
+  return sym_launch(select(shape, diffusion, kernel), shape, kStageBytes, items, n_items, segs, jbase, slots, s);
 }
 
 }  // namespace pawan

@@ -7,9 +7,7 @@
 // memory.
 #pragma once
 
-#include <mutex>
-#include <set>
-#include <utility>
+#include <cooperative_groups.h>
 
 #include "device.cuh"
 #include "kernels.h"
@@ -67,103 +65,141 @@ __device__ __forceinline__ void group_item(const SymItem *__restrict__ items, co
   }
 }
 
-// Small systems: item = one tile pair (a, b0); each warp 32 sources of tile b0.
-// HALVES = 2: eight warps, the second four taking the upper 64 targets where
-// the tile pair's class visits the targets in passes of 64 (the same sums, bit
-// for bit): for launches of no more blocks than SMs, which wait for one tile
-// pair's chain of steps.
-template <class F, int HALVES>
+// Small systems: item = one tile pair (a, b0); each warp 32 of its sources.
+template <class F>
 __device__ __forceinline__ void tile_item(const SymItem *__restrict__ items, const SymSeg *segs,
                                           const int *__restrict__ jbase, double *__restrict__ slots) {
   extern __shared__ float4 smem_sym[];
   double *const accI = reinterpret_cast<double *>(smem_sym);  // [4 sub-blocks][6][128]
-  double *const accJ = accI + kWarps * 6 * kT;                // [HALVES][6][128]
+  double *const accJ = accI + kWarps * 6 * kT;                // [6][128]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int sub = warp & 3, half = HALVES == 1 ? 0 : warp >> 2;
-  char *const st = reinterpret_cast<char *>(accJ + HALVES * 6 * kT) + warp * F::kStageBytes;
+  char *const st = reinterpret_cast<char *>(accJ + 6 * kT) + warp * F::kStageBytes;
   const SymItem it = items[blockIdx.x];
-  double *const mine = accI + sub * 6 * kT;
+  double *const mine = accI + warp * 6 * kT;
   start_next();
-  if (HALVES == 1) {
-    // each lane clears what it will add to
+  // each lane clears what it will add to
 #pragma unroll
-    for (int q = 0; q < 24; ++q) mine[32 * q + lane] = 0.0;
+  for (int q = 0; q < 24; ++q) mine[32 * q + lane] = 0.0;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) accJ[k * kT + tid] = 0.0;
-  } else {
-    for (int q = tid; q < (kWarps + HALVES) * 6 * kT; q += HALVES * kThreads) accI[q] = 0.0;
-    __syncthreads();
-  }
+  for (int k = 0; k < 6; ++k) accJ[k * kT + tid] = 0.0;
   const SymSeg &sg = wait_previous(segs)[it.seg];
-  F::tile_pair(sg, it.a, it.b0, sub, sub + 1, half * (kT / HALVES), (half + 1) * (kT / HALVES), st, lane, mine,
-               accJ + half * 6 * kT);
+  F::tile_pair(sg, it.a, it.b0, warp, warp + 1, 0, kT, st, lane, mine, accJ);
   const int jb = it.b0 > it.a ? jbase[it.jb + it.b0] : -1;
-  if (HALVES == 1 && jb >= 0) {
+  if (jb >= 0) {
     // this thread's own source
     double *out = slots + ((size_t)jb + it.a) * 6 * kT;
 #pragma unroll
     for (int k = 0; k < 6; ++k) out[k * kT + tid] = accJ[k * kT + tid];
   }
   __syncthreads();
-  if (HALVES == 2 && jb >= 0) {
-    double *out = slots + ((size_t)jb + it.a) * 6 * kT;
-#pragma unroll
-    for (int k = 0; k < 6 / HALVES; ++k) {
-      const int q = k * HALVES * kThreads + tid;
-      out[q] = accJ[q] + accJ[6 * kT + q];
-    }
-  }
   if (it.islot >= 0) {
     double *out = slots + (size_t)it.islot * 6 * kT;
 #pragma unroll
-    for (int k = 0; k < 6 / HALVES; ++k) {
-      const int q = k * HALVES * kThreads + tid;
+    for (int k = 0; k < 6; ++k) {
+      const int q = k * kThreads + tid;
       out[q] = ((accI[q] + accI[6 * kT + q]) + accI[12 * kT + q]) + accI[18 * kT + q];
     }
+  }
+}
+
+// The same sums, bit for bit, from eight warps: C blocks (a cluster) per tile
+// pair, block c computing kSubs runs of 32 sources, each in two warps, the second
+// taking the upper 64 targets where the tile pair's class visits the targets in
+// passes of 64; the runs' target sums are added through distributed shared
+// memory.  For launches that last as long as one tile pair's chain of steps.
+template <int C>
+struct Spread {
+  static constexpr int subs = 4 / C;  // runs of 32 sources per block
+  static constexpr int threads = 64 * subs;
+};
+
+template <class F, int C>
+__device__ __forceinline__ void spread_item(const SymItem *__restrict__ items, const SymSeg *segs,
+                                            const int *__restrict__ jbase, double *__restrict__ slots) {
+  namespace cg = cooperative_groups;
+  constexpr int kSubs = Spread<C>::subs, kN = Spread<C>::threads, kC = 6 * kT;
+  extern __shared__ float4 smem_sym[];
+  double *const accI = reinterpret_cast<double *>(smem_sym);  // [kSubs][6][128]
+  double *const accJ = accI + kSubs * kC;                     // [2 halves][6][128], the block's sources used
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int half = warp / kSubs, own = warp % kSubs;  // (the warps of one half on different schedulers)
+  char *const st = reinterpret_cast<char *>(accJ + 2 * kC) + warp * F::kStageBytes;
+  const int rank = C > 1 ? (int)blockIdx.x % C : 0, sub = kSubs * rank + own;
+  const SymItem it = items[blockIdx.x / C];
+  SymSeg sg = segs[it.seg];
+  start_next();
+#pragma unroll
+  for (int q = tid; q < (kSubs + 2) * kC; q += kN) accI[q] = 0.0;
+  __syncthreads();
+  wait_previous_for(sg.pos32, sg.vor32, sg.poslo, sg.vorlo, sg.pos64, sg.vor64, sg.boxes);
+  F::tile_pair(sg, it.a, it.b0, sub, sub + 1, half * (kT / 2), (half + 1) * (kT / 2), st, lane, accI + own * kC,
+               accJ + half * kC);
+  if constexpr (C > 1)
+    cg::this_cluster().sync();
+  else
+    __syncthreads();
+  const int jb = it.b0 > it.a ? jbase[it.jb + it.b0] : -1;
+  if (jb >= 0) {
+    // thread: one of the block's 32 kSubs sources, three of its six sums
+    const int at = 3 * (tid / (32 * kSubs)) * kT + 32 * kSubs * rank + tid % (32 * kSubs);
+    double *out = slots + ((size_t)jb + it.a) * kC;
+#pragma unroll
+    for (int u = 0; u < 3; ++u) out[at + u * kT] = accJ[at + u * kT] + accJ[kC + at + u * kT];
+  }
+  if (it.islot >= 0) {
+    const double *c[4];  // the runs of sources in order
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      c[k] = accI + (k % kSubs) * kC;
+      if constexpr (C > 1) c[k] = cg::this_cluster().map_shared_rank(c[k], k / kSubs);
+    }
+    double *out = slots + (size_t)it.islot * kC;
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      const int q = rank * (kC / C) + u * kN + tid;
+      out[q] = ((c[0][q] + c[1][q]) + c[2][q]) + c[3][q];
+    }
+  }
+  if constexpr (C > 1) {
+    // no block leaves while another reads its sums (which the stores above have
+    // waited for; nothing else is to be ordered)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
   }
 }
 
 using SymKernel = void (*)(const SymItem *, const SymSeg *, const int *, double *);
 
 // How a launch's blocks are shaped: groups of tiles, single tile pairs, or
-// single tile pairs with the targets in halves.
-enum SymShape { SYM_GROUP = 0, SYM_TILE = 1, SYM_TILE_HALVES = 2 };
+// single tile pairs over eight warps of one block or of a cluster of two.
+enum SymShape { SYM_GROUP = 0, SYM_TILE = 1, SYM_WIDE = 2, SYM_SPREAD = 3 };
 
-inline int sym_threads(int shape) { return shape == SYM_TILE_HALVES ? 2 * kThreads : kThreads; }
+inline int sym_cluster(int shape) { return shape == SYM_SPREAD ? 2 : 1; }
+inline int sym_threads(int shape) { return shape == SYM_WIDE ? Spread<1>::threads : kThreads; }
 
 inline size_t sym_smem_bytes(int shape, size_t stage) {
   const size_t tile = (size_t)6 * kT * sizeof(double);
-  const size_t source_sums = shape == SYM_GROUP ? kWarps : shape == SYM_TILE ? 1 : 2;
-  return (kWarps + source_sums) * tile + (size_t)(sym_threads(shape) / 32) * stage;
-}
-
-// Opts a kernel in to its dynamic shared memory beyond the default 48 KB (once
-// per kernel and device).
-inline cudaError_t sym_prepare(SymKernel f, size_t bytes) {
-  static std::mutex mu;
-  static std::set<std::pair<int, SymKernel>> done;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> lk(mu);
-  if (done.count({dev, f})) return cudaSuccess;
-  e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) done.insert({dev, f});
-  return e;
+  const size_t sums = shape == SYM_GROUP  ? 2 * kWarps
+                      : shape == SYM_TILE ? kWarps + 1
+                                          : 2 + (shape == SYM_WIDE ? Spread<1>::subs : Spread<2>::subs);
+  return sums * tile + (size_t)(sym_threads(shape) / 32) * stage;
 }
 
 inline cudaError_t sym_occupancy(SymKernel f, size_t bytes, int *blocks_per_sm) {
-  cudaError_t e = sym_prepare(f, bytes);
+  cudaError_t e = allow_dynamic_smem((const void *)f, bytes);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, kThreads, bytes);
 }
 
-inline cudaError_t sym_launch(SymKernel f, int threads, size_t bytes, const SymItem *items, int n_items, const SymSeg *segs,
-                              const int *jbase, double *slots, cudaStream_t s) {
+inline cudaError_t sym_launch(SymKernel f, int shape, size_t stage, const SymItem *items, int n_items,
+                              const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
   if (n_items <= 0) return cudaSuccess;
-  cudaError_t e = sym_prepare(f, bytes);
+  const size_t bytes = sym_smem_bytes(shape, stage);
+  cudaError_t e = allow_dynamic_smem((const void *)f, bytes);
   if (e != cudaSuccess) return e;
-  return launch_dependent(f, dim3(n_items), threads, bytes, s, items, segs, jbase, slots);
+  const int cluster = sym_cluster(shape);
+  return launch_dependent_clusters(f, cluster, dim3(n_items * cluster), sym_threads(shape), bytes, s, items, segs,
+                                   jbase, slots);
 }
 
 }  // namespace

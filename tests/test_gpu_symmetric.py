@@ -35,6 +35,24 @@ def solved(ctx, arrays, nu, kernel="highorder"):
     return s
 
 
+@pytest.mark.parametrize("n", [64, 129, 1408, 1409, 2048])
+@pytest.mark.parametrize("kernel", ["highorder", "gaussian"])
+def test_launch_shapes_agree(ctx, n, kernel):
+    """Tile pairs in a cluster of two blocks (alone, up to 74 of them), in one
+    block of eight warps (up to 148) and in one of four (in a batch of more):
+    bit for bit."""
+    alone, systems = [], []
+    for k in range(4):
+        s = solved(ctx, particles(n, mixed=k % 2 == 1, seed=96 + k), 1e-3, kernel)
+        alone.append(s.get_rates())
+        systems.append(s)
+    systems.append(solved(ctx, particles(3000, seed=95), 1e-3, kernel))  # 300 tile pairs
+    alone.append(systems[-1].get_rates())
+    Batch(ctx, systems).solve()
+    for s, r in zip(systems, alone):
+        assert np.array_equal(s.get_rates(), r)
+
+
 @pytest.mark.parametrize("kernel", ["highorder", "gaussian"])
 @pytest.mark.parametrize("mixed", [False, True])
 @pytest.mark.parametrize("n", [383, 385, EDGE, EDGE + 1, EDGE + 511, EDGE + 512])
