@@ -180,14 +180,15 @@ __device__ __forceinline__ void gauss_scalars(float sig2, float r2, float ri, fl
 // a x (v + b_lo) has no cancellation; and a_lo x b = mu (a_lo x a) + a_lo x v,
 // the last term eps |a||v| relative to |a x v| = |a||v|.  iaa = 1/|a|^2 (0
 // for a = 0) and (lx, ly, lz) = a_lo x a are per target.
+// Also returns mu and v + b_lo: b + b_lo = mu a + (v + b_lo).
 __device__ __forceinline__ void projection_cross(float ax, float ay, float az, float iaa, float lx,
                                                  float ly, float lz, float bx, float by, float bz,
                                                  float mx, float my, float mz, float &wx, float &wy,
-                                                 float &wz) {
-  const float mu = fmaf(az, bz, fmaf(ay, by, ax * bx)) * iaa;
-  const float vx = fmaf(-mu, ax, bx) + mx;
-  const float vy = fmaf(-mu, ay, by) + my;
-  const float vz = fmaf(-mu, az, bz) + mz;
+                                                 float &wz, float &mu, float &vx, float &vy, float &vz) {
+  mu = fmaf(az, bz, fmaf(ay, by, ax * bx)) * iaa;
+  vx = fmaf(-mu, ax, bx) + mx;
+  vy = fmaf(-mu, ay, by) + my;
+  vz = fmaf(-mu, az, bz) + mz;
   wx = fmaf(mu, lx, fmaf(ay, vz, -az * vy));
   wy = fmaf(mu, ly, fmaf(az, vx, -ax * vz));
   wz = fmaf(mu, lz, fmaf(ax, vy, -ay * vx));
