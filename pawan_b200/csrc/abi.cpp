@@ -167,6 +167,9 @@ void pawan_ctx_destroy(pawan_ctx *ctx) {
   for (auto e : ctx->event_pool) cudaEventDestroy(e);
   for (auto e : ctx->marks)
     if (e) cudaEventDestroy(e);
+  for (auto e : ctx->staging_events)
+    if (e) cudaEventDestroy(e);
+  if (ctx->staging) cudaFreeHost(ctx->staging);
   if (ctx->flush_buf) cudaFree(ctx->flush_buf);
   if (ctx->d_counter) cudaFree(ctx->d_counter);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -365,12 +368,8 @@ int pawan_system_get_wake_rates(pawan_system *sys, size_t wake, double *velocity
   if (wake >= sys->counts.size() || !velocity || !retvorcity)
     return fail(ctx, PAWAN_ERR_INVALID, "bad wake index or null output");
   const size_t o = sys->offsets[wake], c = sys->counts[wake], N = sys->n;
-  PAWAN_CUDA(ctx, cudaMemcpyAsync(velocity, sys->R.p + 3 * o, 3 * c * sizeof(double),
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-  PAWAN_CUDA(ctx, cudaMemcpyAsync(retvorcity, sys->R.p + 3 * N + 3 * o, 3 * c * sizeof(double),
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-  PAWAN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return PAWAN_OK;
+  return copy_to_host(ctx, {{sys->R.p + 3 * o, velocity, 3 * c * sizeof(double)},
+                            {sys->R.p + 3 * N + 3 * o, retvorcity, 3 * c * sizeof(double)}});
 }
 
 int pawan_system_rk4(pawan_system *sys, double dt, size_t nsteps) {

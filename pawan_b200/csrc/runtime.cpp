@@ -875,35 +875,24 @@ int system_ensure_plan(pawan_system *sys) {
   return build_plan(sys->ctx, {sys}, sys->precision, sys->tile, sys->plan);
 }
 
-// Reference layout (per wake [x | alpha]) -> device union layout [x | alpha].
-int state_to_device(pawan_system *sys, const double *state) {
-  pawan_ctx *ctx = sys->ctx;
-  const size_t N = sys->n;
+static std::vector<HostCopy> state_copies(const pawan_system *sys, double *dev, double *host) {
+  std::vector<HostCopy> v;
   for (size_t w = 0; w < sys->counts.size(); ++w) {
     const size_t o = sys->offsets[w], c = sys->counts[w];
-    const double *src = state + 6 * o;
-    PAWAN_CUDA(ctx, cudaMemcpyAsync(sys->X.p + 3 * o, src, 3 * c * sizeof(double),
-                                    cudaMemcpyHostToDevice, ctx->stream));
-    PAWAN_CUDA(ctx, cudaMemcpyAsync(sys->X.p + 3 * N + 3 * o, src + 3 * c, 3 * c * sizeof(double),
-                                    cudaMemcpyHostToDevice, ctx->stream));
+    v.push_back({dev + 3 * o, host + 6 * o, 3 * c * sizeof(double)});
+    v.push_back({dev + 3 * sys->n + 3 * o, host + 6 * o + 3 * c, 3 * c * sizeof(double)});
   }
-  return PAWAN_OK;
+  return v;
+}
+
+// Reference layout (per wake [x | alpha]) -> device union layout [x | alpha].
+int state_to_device(pawan_system *sys, const double *state) {
+  return copy_to_device(sys->ctx, state_copies(sys, sys->X.p, const_cast<double *>(state)));
 }
 
 // Device union layout -> reference layout; synchronous.
 int state_from_device(pawan_system *sys, const double *dev_union, double *state) {
-  pawan_ctx *ctx = sys->ctx;
-  const size_t N = sys->n;
-  for (size_t w = 0; w < sys->counts.size(); ++w) {
-    const size_t o = sys->offsets[w], c = sys->counts[w];
-    double *dst = state + 6 * o;
-    PAWAN_CUDA(ctx, cudaMemcpyAsync(dst, dev_union + 3 * o, 3 * c * sizeof(double),
-                                    cudaMemcpyDeviceToHost, ctx->stream));
-    PAWAN_CUDA(ctx, cudaMemcpyAsync(dst + 3 * c, dev_union + 3 * N + 3 * o, 3 * c * sizeof(double),
-                                    cudaMemcpyDeviceToHost, ctx->stream));
-  }
-  PAWAN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return PAWAN_OK;
+  return copy_to_host(sys->ctx, state_copies(sys, const_cast<double *>(dev_union), state));
 }
 
 }  // namespace pawan

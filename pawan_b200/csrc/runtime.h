@@ -104,6 +104,11 @@ struct pawan_ctx {
   unsigned long long stage_launches = 0;
   double stage_bytes = 0.0;
   cudaEvent_t marks[16] = {};
+  // pinned staging of the copies to the host (host_copy.cpp): allocated on first
+  // use, at most 1 MB, released with the context
+  char *staging = nullptr;
+  size_t staging_bytes = 0;
+  cudaEvent_t staging_events[4] = {};
   void *flush_buf = nullptr;
   size_t flush_bytes = 0;
   // autotune results: (precision, diffusion, log2 sum n^2, log2 segments) -> tile
@@ -258,6 +263,16 @@ int system_upload(pawan_system *sys, const double *position, const double *vorti
                   const double *radius, const double *volume);
 int system_ensure_plan(pawan_system *sys);
 int state_to_device(pawan_system *sys, const double *state);
+// Copies between the device and the caller's memory, in order, on the context's
+// stream.  copy_to_host returns when the data has arrived; copy_to_device when the
+// caller's memory may be reused.
+struct HostCopy {
+  double *dev;
+  double *host;
+  size_t bytes;
+};
+int copy_to_host(pawan_ctx *ctx, std::vector<HostCopy> v);
+int copy_to_device(pawan_ctx *ctx, std::vector<HostCopy> v);
 int state_from_device(pawan_system *sys, const double *dev_union, double *state);
 
 }  // namespace pawan
