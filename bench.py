@@ -224,11 +224,11 @@ def state_update_roofline(prof_stage: dict) -> dict:
     n = max(1, prof_stage["stage_launches"])
     ms = prof_stage["stage_ms"] / n
     gbs = prof_stage["stage_bytes"] / n / (ms * 1e-3) / 1e9 if ms > 0 else None
-    return {"kernel": "stage_kernel", "bound": "hbm", "launches": prof_stage["stage_launches"],
+    return {"kernel": "sum_stage_kernel", "bound": "hbm", "launches": prof_stage["stage_launches"],
             "ms_per_launch": ms, "bytes_per_launch": prof_stage["stage_bytes"] / n,
             "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": (gbs / peak) if gbs else None,
             "peak_source": src,
-            "bytes": "per particle: the 48-byte rates the pair kernel summed, the FP64 state vectors "
+            "bytes": "per particle: the 48-byte slots of the pair kernel's sums (or rates), the FP64 state vectors "
                      "the stage reads and writes, radius and volume, and 128 bytes of packed tile data "
                      "(336-384 bytes for an RK4 stage)"}
 
@@ -697,7 +697,7 @@ def run_pawan(args, rk: Ranks):
             "roofline": {"bound": "fp32", "achieved": achieved_tflops, "peak": peak_tflops,
                          "unit": "TFLOP/s", "frac": achieved_tflops / peak_tflops,
                          "traffic": traffic_from_profiles(tuned),
-                         "kernel": "pairs_f32_kernel", "flops_per_interaction": flops,
+                         "kernel": "sym_f32_group_kernel", "flops_per_interaction": flops,
                          "pair_launch_ms": pair_avg_s * 1e3,
                          "peak_source": "measured: FFMA-chain probe (pawan_peak_fp32) in this run",
                          "note": "achieved counts the reference formula's 96 flops per interaction; the "
@@ -879,7 +879,7 @@ def run_strong(args, rk: Ranks):
                        "tile": tuned},
             "gpu_launches": int(launches), "clocks": clk,
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                         "frac": achieved / peak, "traffic": None, "kernel": "pairs_f32_kernel",
+                         "frac": achieved / peak, "traffic": None, "kernel": "sym_f32 kernels",
                          "flops_per_interaction": flops, "pair_launch_ms": pair_avg_s * 1e3,
                          "peak_source": "measured: FFMA-chain probe (pawan_peak_fp32) in this run"}}
     sh.close()

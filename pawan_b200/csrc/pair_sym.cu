@@ -21,8 +21,7 @@
 // diffusion vector is formed as v_i w + (v_i mu - v_j) alpha_i - v_j lo_i from
 // the w = alpha_j - mu alpha_i that alpha_i x alpha_j is formed from, accurate for
 // nearly equal strengths and volumes whatever mu's rounding (14 operations; from
-// alpha_j - alpha_i in hi and lo 20: 20,011 unordered particles 871
-// -> 846 us).
+// alpha_j - alpha_i in hi and lo 20: 20,011 unordered particles 846 us, 871).
 //
 // Layout.  A warp computes a 128 x 128 tile pair (I, J): each lane holds R
 // targets of I (4 on far tiles, 2 on near ones) and their sums in registers,
@@ -40,9 +39,9 @@
 // registers, at about two reads per cycle and lane.  The step's 3 loads, 9
 // shuffles and address are shared by four targets; with two the shared-memory
 // pipe (21 of its cycles per step) would be the limit.  One right-hand side of
-// the ring pair at N = 131,072: 14.2 ms (1,210 G interactions/s) against 18.4 ms
+// the ring pair at N = 131,072: 13.9 ms (1,236 G interactions/s) against 18.4 ms
 // one-sided; 20,011 unordered particles (near tile pairs only, mixed radii)
-// 0.87 ms against 1.48.
+// 0.85 ms against 1.48.
 //
 // Compiled without contraction of multiply-adds (every FMA is written out), so
 // that the kernels of the launch shapes below round alike and a system's result
