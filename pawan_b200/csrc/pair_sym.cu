@@ -193,16 +193,16 @@ __device__ __forceinline__ void far_block_z(const Stage &st, int lane, const Far
 // half -- which is what the packing saves: 1,435 G interactions/s against 1,340
 // of the scalar loop in a loop of its own on one B200, 1,210 against 1,150 in
 // this kernel on the ring pair at N = 131,072.
-template <int CLS, bool UNI, int KERN, int R>
+template <int CLS, bool UNI, int KERN, int R, int UNROLL>
 __device__ __forceinline__ void far_block(const Stage &st, int lane, const FarTarget (&T)[R], float hu,
                                           Sums9 (&a)[R], Sums9 &b) {
   const float2 one2 = make_float2(1.f, 1.f), half2 = make_float2(0.5f, 0.5f), nhalf2 = make_float2(-0.5f, -0.5f);
   const float2 h2 = make_float2(hu, hu), nh2 = make_float2(-hu, -hu), s2u2 = make_float2(2.f * hu, 2.f * hu);
 #pragma unroll 1
-  for (int kk = 0; kk < 32; kk += 2) {
+  for (int kk = 0; kk < 32; kk += UNROLL) {
     const int base = lane ^ kk;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < UNROLL; ++u) {
       const float4 p = st.s0[base ^ u], s = st.s1[base ^ u], e = st.s2[base ^ u];
 #pragma unroll
       for (int r = 0; r < R; r += 2) {
@@ -270,7 +270,7 @@ __device__ __forceinline__ void fold_far(const Sums9 &s, float x, float y, float
 // A far tile pair: sub-blocks [k0, k1) of 32 sources of tile J against all
 // targets of tile I, R per lane and pass.  accI: the warp's [6][128] target
 // sums; accJ: [6][128] source sums of tile J.
-template <int CLS, bool UNI, bool DIFF, int KERN, int R>
+template <int CLS, bool UNI, bool DIFF, int KERN, int R, int UNROLL>
 __device__ __forceinline__ void far_pair(const SymSeg &sg, int I, int J, int k0, int k1, int ta, int tb,
                                          float cx, float cy, float cz, float hu, const Stage &st, int lane,
                                          double *accI, double *accJ) {
@@ -324,7 +324,7 @@ __device__ __forceinline__ void far_pair(const SymSeg &sg, int I, int J, int k0,
       if constexpr (CLS == FAR_Z)
         far_block_z<UNI, DIFF, KERN, R>(st, lane, T, hu, kap, a, b);
       else
-        far_block<CLS, UNI, KERN, R>(st, lane, T, hu, a, b);
+        far_block<CLS, UNI, KERN, R, UNROLL>(st, lane, T, hu, a, b);
       const float4 pj = st.s0[lane], qj = st.s1[lane], ej = st.s2[lane];
       const float2 lj = st.s3[lane];
       fold_far(b, pj.x, pj.y, pj.z, qj.x, qj.y, qj.z, ej.w, lj.x, lj.y, As2, -3.0 * As2,
@@ -370,12 +370,15 @@ __device__ __forceinline__ void rotate(Sums6 &a, int m) {
 template <bool UNI, bool DIAG, bool DIFF, int KERN, int R>
 __device__ __forceinline__ void near_block(const Stage &st, int lane, const NearTarget (&T)[R], int self,
                                            float hu, float kap, Sums6 (&a)[R], Sums6 &b) {
+  // steps per iteration (the Gaussian scalars' code is four times as long): 20,011
+  // unordered particles 844 us with two, 835 with four, 842 with eight
+  constexpr int kUnroll = KERN == KERNEL_GAUSSIAN ? 2 : 4;
   const float s2u = 2.f * hu, c240 = -480.f * hu;
 #pragma unroll 1
-  for (int kk = 0; kk < 32; kk += 2) {
+  for (int kk = 0; kk < 32; kk += kUnroll) {
     const int base = lane ^ kk;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < kUnroll; ++u) {
       // (hi position, h), (lo position, volume), (strength, lo.x), (lo.y, lo.z)
       const float4 p = st.s0[base ^ u], pl = st.s1[base ^ u], s = st.s2[base ^ u];
       const float2 l = st.s3[base ^ u];
@@ -509,7 +512,7 @@ __device__ __forceinline__ void near_pair(const SymSeg &sg, int I, int J, int k0
 // the two tiles' boxes allow.  The classes and their bounds are pair_f32.cu's;
 // the far formulation is centred on the smaller of the two boxes, whose
 // half-diagonal bounds |x'_i| + |x'_j| by 3 |d| for every pair.
-template <bool DIFF, int KERN>
+template <bool DIFF, int KERN, int UNROLL>
 __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, int ta, int tb,
                                           const Stage &st, int lane, double *accI, double *accJ) {
   const float4 alo = sg.boxes[2 * I], ahi = sg.boxes[2 * I + 1];
@@ -539,64 +542,72 @@ __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0
   const float sig2max = ahi.w + bhi.w;
   if (KERN == KERNEL_GAUSSIAN) {
     if (gap2 >= 49.f * sig2max)
-      far_pair<FAR_SER, false, DIFF, KERN, 4>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_SER, false, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_Z, false, DIFF, KERN, 2>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_Z, false, DIFF, KERN, 2, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     return;
   }
   if (gap2 >= 256.f * sig2max) {
     if (uni)
-      far_pair<FAR_SER, true, DIFF, KERN, 4>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_SER, true, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_SER, false, DIFF, KERN, 4>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_SER, false, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
   } else if (gap2 >= 36.f * sig2max) {
     if (uni)
-      far_pair<FAR_NZ, true, DIFF, KERN, 4>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_NZ, true, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_NZ, false, DIFF, KERN, 4>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_NZ, false, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
   } else {
     if (uni)
-      far_pair<FAR_Z, true, DIFF, KERN, 2>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_Z, true, DIFF, KERN, 2, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_Z, false, DIFF, KERN, 2>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<FAR_Z, false, DIFF, KERN, 2, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
   }
 }
 
-template <bool DIFF, int KERN>
+template <bool DIFF, int KERN, int UNROLL>
 struct Pair32 {
   static constexpr int kStageBytes = ::pawan::kStageBytes;
   static __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, int ta, int tb,
                                                    char *st, int lane, double *accI, double *accJ) {
-    ::pawan::tile_pair<DIFF, KERN>(sg, I, J, k0, k1, ta, tb, stage_of(st), lane, accI, accJ);
+    ::pawan::tile_pair<DIFF, KERN, UNROLL>(sg, I, J, k0, k1, ta, tb, stage_of(st), lane, accI, accJ);
   }
 };
+
+// Steps of the far loop per iteration: four where the registers and the code
+// (two far classes instead of six) leave room, the Gaussian kernel's single tile
+// pairs (N = 32,000 1,021 -> 993 us).  In groups four spill (65,536 particles 3.69
+// -> 3.98 ms), and with the default kernel's classes they gain 1 % at 32,768 and
+// lose 2-5 % at 2,100 to 4,096.
+template <bool DIFF, int KERN>
+using TilePair32 = Pair32<DIFF, KERN, KERN == KERNEL_GAUSSIAN ? 4 : 2>;
 
 template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(kThreads, kBlocks)
     sym_f32_group_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
                          const int *__restrict__ jbase, double *__restrict__ slots) {
-  group_item<Pair32<DIFF, KERN>>(items, segs, jbase, slots);
+  group_item<Pair32<DIFF, KERN, 2>>(items, segs, jbase, slots);
 }
 
 template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(kThreads, kBlocks)
     sym_f32_tile_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
                         const int *__restrict__ jbase, double *__restrict__ slots) {
-  tile_item<Pair32<DIFF, KERN>>(items, segs, jbase, slots);
+  tile_item<TilePair32<DIFF, KERN>>(items, segs, jbase, slots);
 }
 
 template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(Spread<1>::threads, 1)
     sym_f32_wide_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
                         const int *__restrict__ jbase, double *__restrict__ slots) {
-  spread_item<Pair32<DIFF, KERN>, 1>(items, segs, jbase, slots);
+  spread_item<TilePair32<DIFF, KERN>, 1>(items, segs, jbase, slots);
 }
 
 template <bool DIFF, int KERN>
 __global__ void __launch_bounds__(Spread<2>::threads, 2)
     sym_f32_spread_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
                           const int *__restrict__ jbase, double *__restrict__ slots) {
-  spread_item<Pair32<DIFF, KERN>, 2>(items, segs, jbase, slots);
+  spread_item<TilePair32<DIFF, KERN>, 2>(items, segs, jbase, slots);
 }
 
 template <bool DIFF, int KERN>
