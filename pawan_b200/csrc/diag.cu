@@ -21,12 +21,12 @@
 // is visited once here too.  Per-target sums are reduced per block in a fixed
 // tree and the block partials by one block in fixed order: deterministic.
 //
-// The quadratic kernel is bound by the FP64 pipe: 67 operations per unordered
+// The quadratic kernel is bound by the FP64 pipe: 68 operations per unordered
 // pair.  A block takes 128 targets and a range of the sources from the targets'
 // own tile on, in ranges short enough that the device is full from about two
 // thousand particles on.  Helical wake, whole call on one B200: N = 65,536
-// 10.5 ms (28.7 when every ordered pair was visited, by one block per 128
-// targets), 0.74 of the FP64 pipe's rate; N = 16,384 0.69 ms (3.2).
+// 10.3 ms (28.7 when every ordered pair was visited, by one block per 128
+// targets), 0.76 of the FP64 pipe's rate; N = 16,384 0.67 ms (3.2).
 #include <algorithm>
 
 #include "device.cuh"
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kDiagThreads)
     __syncthreads();
     const int cnt = min(kDiagThreads, s1 - ts);
     const int own = i - ts;  // sources up to the target itself belong to the other order
-#pragma unroll 2
+#pragma unroll 1  // (two: 10.45 ms, eight: 10.29)
     for (int jj = 0; jj < cnt; ++jj) {
       if (jj <= own) continue;
       const double4 rj = sp[jj], aj = sv[jj];
