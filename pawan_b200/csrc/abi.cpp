@@ -838,6 +838,7 @@ void pawan_batch_destroy(pawan_batch *b) {
 int pawan_batch_rk4(pawan_batch *b, const double *dt, double dt0, size_t nsteps, int use_graph) {
   if (!b) return PAWAN_ERR_INVALID;
   PAWAN_TRY(batch_ensure_plan(b));
+  PAWAN_TRY(check_dts(b->ctx, b->systems.size(), dt, dt0));  // before either plan takes a step size
   std::vector<double> dts;
   for (size_t k = 0; k < b->plans.size(); ++k) {
     dts.clear();

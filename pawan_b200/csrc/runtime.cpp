@@ -540,22 +540,29 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
   return PAWAN_OK;
 }
 
-// Puts each system's dt into the device stage table (only when it changed).
+int check_dts(pawan_ctx *ctx, size_t n, const double *dt, double dt0) {
+  for (size_t s = 0; s < n; ++s) {
+    const double v = dt ? dt[s] : dt0;
+    if (!(v > 0.0) || !std::isfinite(v)) return fail(ctx, PAWAN_ERR_INVALID, "dt must be positive");
+  }
+  return PAWAN_OK;
+}
+
+// Puts each system's dt into the device stage table (only when it changed).  A
+// rejected call changes nothing: what p.dts holds is always what the table holds.
 int set_plan_dt(pawan_ctx *ctx, Plan &p, const double *dt, double dt0) {
+  PAWAN_TRY(check_dts(ctx, p.systems.size(), dt, dt0));
   bool changed = false;
   for (size_t s = 0; s < p.systems.size(); ++s) {
     const double v = dt ? dt[s] : dt0;
-    if (!(v > 0.0) || !std::isfinite(v)) return fail(ctx, PAWAN_ERR_INVALID, "dt must be positive");
-    if (p.dts[s] != v) {
-      p.dts[s] = v;
-      p.stage_host[s].dt = v;
-      changed = true;
-    }
+    p.stage_host[s].dt = v;
+    changed = changed || p.dts[s] != v;
   }
   if (changed) {
     PAWAN_CUDA(ctx, cudaMemcpyAsync(p.stage_descs.p, p.stage_host.data(),
                                     p.stage_host.size() * sizeof(StageDesc),
                                     cudaMemcpyHostToDevice, ctx->stream));
+    for (size_t s = 0; s < p.systems.size(); ++s) p.dts[s] = p.stage_host[s].dt;
   }
   return PAWAN_OK;
 }

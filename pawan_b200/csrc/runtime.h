@@ -243,6 +243,8 @@ double sym_slot_bytes(size_t n, bool serving);
 int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int precision,
                const TileChoice &tile, std::unique_ptr<Plan> &out, int fixed_chunk_sources = 0,
                bool ordered_alloc = false);
+// Whether n steps (dt[i], or dt0 for all when dt is null) are all valid.
+int check_dts(pawan_ctx *ctx, size_t n, const double *dt, double dt0);
 int set_plan_dt(pawan_ctx *ctx, Plan &p, const double *dt, double dt0);
 int launch_pairs(pawan_ctx *ctx, Plan &p, bool allow_events = true);
 // The pair kernel over the plan's work items [first, first + count) only (the
