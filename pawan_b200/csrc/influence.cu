@@ -61,12 +61,12 @@ __device__ __forceinline__ double pair_z(const double4 ri, double hi, const doub
   const double sig2 = __fma_rn(0.5 * rj.w, rj.w, hi);
   if (KERN == KERNEL_GAUSSIAN) {
     const double cg = 0.06349363593424096978;  // (2 pi)^-1.5
-    const double is = rsqrt_f64(sig2);
+    const double is = rsqrt_f64_full(sig2);
     const double is2 = __dmul_rn(is, is);
     return __dmul_rn(__dmul_rn(exp(-0.5 * __dmul_rn(rho2, is2)), __dmul_rn(is2, is)), cg);
   } else {
     const double c = 1.875 * kInvPi;  // 15 / (8 pi)
-    const double w = rsqrt_f64(__dadd_rn(rho2, sig2));
+    const double w = rsqrt_f64_full(__dadd_rn(rho2, sig2));
     const double w2 = __dmul_rn(w, w);
     const double u = __dmul_rn(sig2, w2);
     const double u2 = __dmul_rn(u, u);
