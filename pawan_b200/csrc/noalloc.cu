@@ -21,8 +21,9 @@
 // (different streams, different host threads) race and must be serialised by
 // the caller.  Whatever must start at zero (the scheduler counter and the
 // per-tile counters) is cleared by the call itself, the count of finished
-// prepare blocks by the last of them (the array starts zeroed); the rest is
-// fully overwritten before it is read.
+// prepare blocks by the last of them (the array starts zeroed) and once more by
+// the call's last kernel, so that calls that raced leave nothing wrong for the
+// calls after them; the rest is fully overwritten before it is read.
 //
 // The pair kernel is pawan_system_solve's in PAWAN_PREC_F32 with the
 // high-order smoothing kernel only, on the one-sided kernel (the symmetric
@@ -210,9 +211,10 @@ __global__ void __launch_bounds__(kStageThreads)
 }
 
 // The pair kernel's rates ([6][n], chunks summed in chunk order) into the
-// caller's N x 3 outputs.
-__global__ void noalloc_reduce(const NoallocScratch *S, int n, double *vel, double *dvor) {
+// caller's N x 3 outputs.  Clears the count of prepare blocks for the next call.
+__global__ void noalloc_reduce(NoallocScratch *S, int n, double *vel, double *dvor) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l == 0) S->prepared = 0;
   if (l >= n) return;
   for (int k = 0; k < 3; ++k) {
     vel[3 * (size_t)l + k] = S->rates[(size_t)k * n + l];
