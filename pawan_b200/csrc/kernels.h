@@ -85,9 +85,10 @@ cudaError_t launch_pairs_f32(const PairConfig &c, bool diffusion, int kernel, in
 
 // The symmetric pair engine (FP32): each unordered pair once, sums into the
 // items' slots; one block per item.  group: items over groups of kSymGroup
-// tiles, else over single tile pairs.
+// tiles, else over single tile pairs.  sided: some items form one side's sums
+// only (sharded systems).
 cudaError_t sym_f32_occupancy(bool diffusion, int kernel, int *blocks_per_sm);
-cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
+cudaError_t launch_sym_f32(bool group, bool sided, bool diffusion, int kernel, const SymItem *items, int n_items,
                            int sm_count, const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s);
 // Sums the slots of each listed tile into its rates.
 cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const StageDesc *descs, const double *slots,
@@ -97,7 +98,7 @@ cudaError_t launch_sym_sums(const SymSum *sums, int n_sums, const StageDesc *des
 // engine whatever the tiling.
 bool pairs_f64_supported(const PairConfig &c, int kernel);
 cudaError_t sym_f64_occupancy(bool diffusion, int kernel, int *blocks_per_sm);
-cudaError_t launch_sym_f64(bool group, bool diffusion, int kernel, const SymItem *items, int n_items,
+cudaError_t launch_sym_f64(bool group, bool sided, bool diffusion, int kernel, const SymItem *items, int n_items,
                            int sm_count, const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s);
 
 // FP64, the reference's formula term by term (pow, divisions): the plain

@@ -86,7 +86,7 @@ __device__ __forceinline__ void add64(const Sums64 &s, double f, double *acc) {
 
 // DIAG: tile I against itself; every ordered pair is visited and only the
 // targets' sums are kept.
-template <bool DIAG, bool DIFF, int KERN>
+template <int SIDE, bool DIAG, bool DIFF, int KERN>
 __device__ __forceinline__ void pairs64(const SymSeg &sg, int I, int J, int k0, int k1, char *stage, int lane,
                                         double *accI, double *accJ) {
   constexpr int kR = Shape64<KERN>::targets;
@@ -172,13 +172,15 @@ __device__ __forceinline__ void pairs64(const SymSeg &sg, int I, int J, int k0, 
             sy = own ? 0.0 : sy;
             sz = own ? 0.0 : sz;
           }
-          sum[r].ux = fma(qh, fma(q2.y, dz, -q3.x * dy), sum[r].ux);
-          sum[r].uy = fma(qh, fma(q3.x, dx, -q2.x * dz), sum[r].uy);
-          sum[r].uz = fma(qh, fma(q2.x, dy, -q2.y * dx), sum[r].uz);
-          sum[r].sx += sx;
-          sum[r].sy += sy;
-          sum[r].sz += sz;
-          if (!DIAG) {
+          if (SIDE != SIDE_J) {
+            sum[r].ux = fma(qh, fma(q2.y, dz, -q3.x * dy), sum[r].ux);
+            sum[r].uy = fma(qh, fma(q3.x, dx, -q2.x * dz), sum[r].uy);
+            sum[r].uz = fma(qh, fma(q2.x, dy, -q2.y * dx), sum[r].uz);
+            sum[r].sx += sx;
+            sum[r].sy += sy;
+            sum[r].sz += sz;
+          }
+          if (!DIAG && SIDE != SIDE_I) {
             // alpha_i x d and s, taken from the source's sums at the end
             b.ux = fma(qh, fma(a[r].y, dz, -a[r].z * dy), b.ux);
             b.uy = fma(qh, fma(a[r].z, dx, -a[r].x * dz), b.uy);
@@ -188,11 +190,12 @@ __device__ __forceinline__ void pairs64(const SymSeg &sg, int I, int J, int k0, 
             b.sz += sz;
           }
         }
-        if (!DIAG) rotate(b, (m ^ (m + 1)) & 31);
+        if (!DIAG && SIDE != SIDE_I) rotate(b, (m ^ (m + 1)) & 31);
       }
-      if (!DIAG) add64(b, -kInv4Pi, accJ + 32 * k + lane);
+      if (!DIAG && SIDE != SIDE_I) add64(b, -kInv4Pi, accJ + 32 * k + lane);
       __syncwarp();
     }
+    if (SIDE == SIDE_J) continue;
 #pragma unroll
     for (int r = 0; r < kR; ++r) add64(sum[r], kInv4Pi, accI + t0 + 32 * r + lane);
   }
@@ -201,12 +204,13 @@ __device__ __forceinline__ void pairs64(const SymSeg &sg, int I, int J, int k0, 
 template <bool DIFF, int KERN>
 struct Pair64 {
   static constexpr int kStageBytes = kStage64;
+  template <int SIDE>
   static __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, int, int, char *st,
                                                    int lane, double *accI, double *accJ) {
-    if (I == J)
-      pairs64<true, DIFF, KERN>(sg, I, J, k0, k1, st, lane, accI, accJ);
+    if (SIDE == SIDE_BOTH && I == J)
+      pairs64<SIDE_BOTH, true, DIFF, KERN>(sg, I, J, k0, k1, st, lane, accI, accJ);
     else
-      pairs64<false, DIFF, KERN>(sg, I, J, k0, k1, st, lane, accI, accJ);
+      pairs64<SIDE, false, DIFF, KERN>(sg, I, J, k0, k1, st, lane, accI, accJ);
   }
 };
 
@@ -224,15 +228,31 @@ __global__ void __launch_bounds__(kThreads, Shape64<KERN>::blocks)
   tile_item<Pair64<DIFF, KERN>>(items, segs, jbase, slots);
 }
 
+template <bool DIFF, int KERN>
+__global__ void __launch_bounds__(kThreads, Shape64<KERN>::blocks)
+    sym_f64_group_sided_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
+                               const int *__restrict__ jbase, double *__restrict__ slots) {
+  sided_item<Pair64<DIFF, KERN>, true>(items, segs, jbase, slots);
+}
+
+template <bool DIFF, int KERN>
+__global__ void __launch_bounds__(kThreads, Shape64<KERN>::blocks)
+    sym_f64_tile_sided_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
+                              const int *__restrict__ jbase, double *__restrict__ slots) {
+  sided_item<Pair64<DIFF, KERN>, false>(items, segs, jbase, slots);
+}
+
 template <int KERN>
-SymKernel select_k(bool group, bool diffusion) {
+SymKernel select_k(bool group, bool sided, bool diffusion) {
+  if (sided && group) return diffusion ? &sym_f64_group_sided_kernel<true, KERN> : &sym_f64_group_sided_kernel<false, KERN>;
+  if (sided) return diffusion ? &sym_f64_tile_sided_kernel<true, KERN> : &sym_f64_tile_sided_kernel<false, KERN>;
   if (group) return diffusion ? &sym_f64_group_kernel<true, KERN> : &sym_f64_group_kernel<false, KERN>;
   return diffusion ? &sym_f64_tile_kernel<true, KERN> : &sym_f64_tile_kernel<false, KERN>;
 }
 
-SymKernel select(bool group, bool diffusion, int kernel) {
-  return kernel == KERNEL_GAUSSIAN ? select_k<KERNEL_GAUSSIAN>(group, diffusion)
-                                   : select_k<KERNEL_HIGHORDER>(group, diffusion);
+SymKernel select(bool group, bool sided, bool diffusion, int kernel) {
+  return kernel == KERNEL_GAUSSIAN ? select_k<KERNEL_GAUSSIAN>(group, sided, diffusion)
+                                   : select_k<KERNEL_HIGHORDER>(group, sided, diffusion);
 }
 
 }  // namespace
@@ -243,12 +263,12 @@ bool pairs_f64_supported(const PairConfig &c, int kernel) {
 }
 
 cudaError_t sym_f64_occupancy(bool diffusion, int kernel, int *blocks_per_sm) {
-  return sym_occupancy(select(true, diffusion, kernel), sym_smem_bytes(SYM_GROUP, kStage64), blocks_per_sm);
+  return sym_occupancy(select(true, false, diffusion, kernel), sym_smem_bytes(SYM_GROUP, kStage64), blocks_per_sm);
 }
 
-cudaError_t launch_sym_f64(bool group, bool diffusion, int kernel, const SymItem *items, int n_items, int,
+cudaError_t launch_sym_f64(bool group, bool sided, bool diffusion, int kernel, const SymItem *items, int n_items, int,
                            const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
-  return sym_launch(select(group, diffusion, kernel), group ? SYM_GROUP : SYM_TILE, kStage64, items, n_items, segs,
+  return sym_launch(select(group, sided, diffusion, kernel), group ? SYM_GROUP : SYM_TILE, kStage64, items, n_items, segs,
                     jbase, slots, s);
 }
 

@@ -109,21 +109,26 @@ __device__ __forceinline__ void rotate(Sums9 &a, int m) {
   a.gz = __shfl_xor_sync(kFull, a.gz, m);
 }
 
-// Adds a pair's weight m to both particles' W and Q sums.
+// Adds a pair's weight m to the W and Q sums of both particles, or of one.
+template <int SIDE>
 __device__ __forceinline__ void add_wq(const FarTarget &T, const float4 &s, const float4 &e, float m, Sums9 &a,
                                        Sums9 &b) {
-  a.wx = fmaf(m, e.x, a.wx);
-  a.wy = fmaf(m, e.y, a.wy);
-  a.wz = fmaf(m, e.z, a.wz);
-  a.qx = fmaf(m, s.x, a.qx);
-  a.qy = fmaf(m, s.y, a.qy);
-  a.qz = fmaf(m, s.z, a.qz);
-  b.wx = fmaf(m, T.bx, b.wx);
-  b.wy = fmaf(m, T.by, b.wy);
-  b.wz = fmaf(m, T.bz, b.wz);
-  b.qx = fmaf(m, T.ax, b.qx);
-  b.qy = fmaf(m, T.ay, b.qy);
-  b.qz = fmaf(m, T.az, b.qz);
+  if (SIDE != SIDE_J) {
+    a.wx = fmaf(m, e.x, a.wx);
+    a.wy = fmaf(m, e.y, a.wy);
+    a.wz = fmaf(m, e.z, a.wz);
+    a.qx = fmaf(m, s.x, a.qx);
+    a.qy = fmaf(m, s.y, a.qy);
+    a.qz = fmaf(m, s.z, a.qz);
+  }
+  if (SIDE != SIDE_I) {
+    b.wx = fmaf(m, T.bx, b.wx);
+    b.wy = fmaf(m, T.by, b.wy);
+    b.wz = fmaf(m, T.bz, b.wz);
+    b.qx = fmaf(m, T.ax, b.qx);
+    b.qy = fmaf(m, T.ay, b.qy);
+    b.qz = fmaf(m, T.az, b.qz);
+  }
 }
 
 // t~ = alpha_j.beta_i + alpha_i.beta_j
@@ -135,7 +140,7 @@ __device__ __forceinline__ float far_t(const FarTarget &T, const float4 &s, cons
 // 32 sources of a far tile with the Z terms against R targets per lane.  kap:
 // the diffusion factor in the units of the G sums (5 nu, or 80 nu / h with one
 // radius).
-template <bool UNI, bool DIFF, int KERN, int R>
+template <int SIDE, bool UNI, bool DIFF, int KERN, int R>
 __device__ __forceinline__ void far_block_z(const Stage &st, int lane, const FarTarget (&T)[R], float hu,
                                             float kap, Sums9 (&a)[R], Sums9 &b) {
   const float s2u = 2.f * hu, c240 = -480.f * hu;
@@ -158,32 +163,62 @@ __device__ __forceinline__ void far_block_z(const Stage &st, int lane, const Far
         else
           kernel_scalars(T[r].h + p.w, rsqrtf(r2 + (T[r].h + p.w)), ri, m, fh, dp);
         const float g = -fh * far_t(T[r], s, e);
-        add_wq(T[r], s, e, m, a[r], b);
+        add_wq<SIDE>(T[r], s, e, m, a[r], b);
         if (DIFF) {
           const float kd = kap * dp;
           const float gx = fmaf(kd, fmaf(T[r].v, s.x, -s.w * T[r].ax), g * dx);
           const float gy = fmaf(kd, fmaf(T[r].v, s.y, -s.w * T[r].ay), g * dy);
           const float gz = fmaf(kd, fmaf(T[r].v, s.z, -s.w * T[r].az), g * dz);
-          a[r].gx += gx;
-          a[r].gy += gy;
-          a[r].gz += gz;
-          b.gx += gx;
-          b.gy += gy;
-          b.gz += gz;
+          if (SIDE != SIDE_J) {
+            a[r].gx += gx;
+            a[r].gy += gy;
+            a[r].gz += gz;
+          }
+          if (SIDE != SIDE_I) {
+            b.gx += gx;
+            b.gy += gy;
+            b.gz += gz;
+          }
         } else {
-          a[r].gx = fmaf(g, dx, a[r].gx);
-          a[r].gy = fmaf(g, dy, a[r].gy);
-          a[r].gz = fmaf(g, dz, a[r].gz);
-          b.gx = fmaf(g, dx, b.gx);
-          b.gy = fmaf(g, dy, b.gy);
-          b.gz = fmaf(g, dz, b.gz);
+          if (SIDE != SIDE_J) {
+            a[r].gx = fmaf(g, dx, a[r].gx);
+            a[r].gy = fmaf(g, dy, a[r].gy);
+            a[r].gz = fmaf(g, dz, a[r].gz);
+          }
+          if (SIDE != SIDE_I) {
+            b.gx = fmaf(g, dx, b.gx);
+            b.gy = fmaf(g, dy, b.gy);
+            b.gz = fmaf(g, dz, b.gz);
+          }
         }
       }
       // lane l holds the sums of source l ^ k and next takes l ^ (k + 1)
       const int k = kk + u;
-      rotate(b, (k ^ (k + 1)) & 31);
+      if (SIDE != SIDE_I) rotate(b, (k ^ (k + 1)) & 31);
     }
   }
+}
+
+// Weight m and 1/rho^2 of two pairs without the Z terms, from rho^2 and (unless
+// UNI) sigma^2.
+template <int CLS, bool UNI, int KERN>
+__device__ __forceinline__ float2 far_weights(float2 r2, float2 sig2, float hu, float2 &ri2) {
+  const float2 one2 = make_float2(1.f, 1.f), half2 = make_float2(0.5f, 0.5f), nhalf2 = make_float2(-0.5f, -0.5f);
+  const float2 h2 = make_float2(hu, hu), nh2 = make_float2(-hu, -hu), s2u2 = make_float2(2.f * hu, 2.f * hu);
+  const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+  ri2 = __fmul2_rn(ri, ri);
+  if (CLS == FAR_SER && KERN == KERNEL_GAUSSIAN) return __fmul2_rn(ri, ri2);
+  if (CLS == FAR_SER && UNI)
+    return __fmul2_rn(__fmul2_rn(__fmul2_rn(ri, ri2), __ffma2_rn(nh2, ri2, one2)), ri2);
+  if (CLS == FAR_SER) {
+    const float2 eps = __fmul2_rn(sig2, ri2);
+    return __fmul2_rn(__fmul2_rn(__fmul2_rn(eps, ri), ri2), __ffma2_rn(nhalf2, eps, one2));
+  }
+  const float2 sr = __fadd2_rn(r2, UNI ? s2u2 : sig2);
+  const float2 y = make_float2(rcp_approx(sr.x), rcp_approx(sr.y));
+  if (UNI) return __fmul2_rn(__fmul2_rn(__ffma2_rn(__fmul2_rn(h2, y), y, y), ri), ri2);
+  const float2 ph = __ffma2_rn(__fmul2_rn(__fmul2_rn(half2, sig2), y), y, y);
+  return __fmul2_rn(__fmul2_rn(__fmul2_rn(ph, sig2), ri), ri2);
 }
 
 // The same without the Z terms (FAR_NZ, FAR_SER), R even: two targets per
@@ -193,11 +228,9 @@ __device__ __forceinline__ void far_block_z(const Stage &st, int lane, const Far
 // half -- which is what the packing saves: 1,435 G interactions/s against 1,340
 // of the scalar loop in a loop of its own on one B200, 1,210 against 1,150 in
 // this kernel on the ring pair at N = 131,072.
-template <int CLS, bool UNI, int KERN, int R, int UNROLL>
+template <int SIDE, int CLS, bool UNI, int KERN, int R, int UNROLL>
 __device__ __forceinline__ void far_block(const Stage &st, int lane, const FarTarget (&T)[R], float hu,
                                           Sums9 (&a)[R], Sums9 &b) {
-  const float2 one2 = make_float2(1.f, 1.f), half2 = make_float2(0.5f, 0.5f), nhalf2 = make_float2(-0.5f, -0.5f);
-  const float2 h2 = make_float2(hu, hu), nh2 = make_float2(-hu, -hu), s2u2 = make_float2(2.f * hu, 2.f * hu);
 #pragma unroll 1
   for (int kk = 0; kk < 32; kk += UNROLL) {
     const int base = lane ^ kk;
@@ -210,43 +243,73 @@ __device__ __forceinline__ void far_block(const Stage &st, int lane, const FarTa
         const float2 dx = make_float2(X.x - p.x, Y.x - p.x), dy = make_float2(X.y - p.y, Y.y - p.y),
                      dz = make_float2(X.z - p.z, Y.z - p.z);
         const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-        const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-        const float2 ri2 = __fmul2_rn(ri, ri);
-        float2 m;
-        if (CLS == FAR_SER && KERN == KERNEL_GAUSSIAN) {
-          m = __fmul2_rn(ri, ri2);
-        } else if (CLS == FAR_SER && UNI) {
-          m = __fmul2_rn(__fmul2_rn(__fmul2_rn(ri, ri2), __ffma2_rn(nh2, ri2, one2)), ri2);
-        } else if (CLS == FAR_SER) {
-          const float2 eps = __fmul2_rn(make_float2(X.h + p.w, Y.h + p.w), ri2);
-          m = __fmul2_rn(__fmul2_rn(__fmul2_rn(eps, ri), ri2), __ffma2_rn(nhalf2, eps, one2));
-        } else if (UNI) {
-          const float2 sr = __fadd2_rn(r2, s2u2);
-          const float2 y = make_float2(rcp_approx(sr.x), rcp_approx(sr.y));
-          m = __fmul2_rn(__fmul2_rn(__ffma2_rn(__fmul2_rn(h2, y), y, y), ri), ri2);
-        } else {
-          const float2 sig2 = make_float2(X.h + p.w, Y.h + p.w);
-          const float2 sr = __fadd2_rn(r2, sig2);
-          const float2 y = make_float2(rcp_approx(sr.x), rcp_approx(sr.y));
-          const float2 ph = __ffma2_rn(__fmul2_rn(__fmul2_rn(half2, sig2), y), y, y);
-          m = __fmul2_rn(__fmul2_rn(__fmul2_rn(ph, sig2), ri), ri2);
-        }
+        float2 ri2;
+        const float2 m = far_weights<CLS, UNI, KERN>(r2, make_float2(X.h + p.w, Y.h + p.w), hu, ri2);
         const float2 g = __fmul2_rn(__fmul2_rn(m, ri2), make_float2(far_t(X, s, e), far_t(Y, s, e)));
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           const float gq = q ? g.y : g.x, ex = q ? dx.y : dx.x, ey = q ? dy.y : dy.x, ez = q ? dz.y : dz.x;
           Sums9 &c = a[r + q];
-          add_wq(T[r + q], s, e, q ? m.y : m.x, c, b);
-          c.gx = fmaf(gq, ex, c.gx);
-          c.gy = fmaf(gq, ey, c.gy);
-          c.gz = fmaf(gq, ez, c.gz);
-          b.gx = fmaf(gq, ex, b.gx);
-          b.gy = fmaf(gq, ey, b.gy);
-          b.gz = fmaf(gq, ez, b.gz);
+          add_wq<SIDE>(T[r + q], s, e, q ? m.y : m.x, c, b);
+          if (SIDE != SIDE_J) {
+            c.gx = fmaf(gq, ex, c.gx);
+            c.gy = fmaf(gq, ey, c.gy);
+            c.gz = fmaf(gq, ez, c.gz);
+          }
+          if (SIDE != SIDE_I) {
+            b.gx = fmaf(gq, ex, b.gx);
+            b.gy = fmaf(gq, ey, b.gy);
+            b.gz = fmaf(gq, ez, b.gz);
+          }
         }
       }
       const int k = kk + u;
-      rotate(b, (k ^ (k + 1)) & 31);
+      if (SIDE != SIDE_I) rotate(b, (k ^ (k + 1)) & 31);
+    }
+  }
+}
+
+// The sources' sums of a tile pair alone: each lane keeps four sources and their
+// sums in registers and meets the 128 targets in shared memory (t: 4 x 32 of
+// (x', h), (strength, volume), (beta)), in the order in which the travelling sums
+// of far_block meet them -- the same terms added in the same order, without the
+// shuffles.  The last rank of eight at N = 131,072, whose items are mostly of this
+// kind: 2.48 ms, 2.73 with the sums travelling (one-sided kernel 2.40).
+template <int CLS, bool UNI, int KERN>
+__device__ __forceinline__ void far_block_sources(const float4 *t, int lane, const FarTarget (&S)[4], float hu,
+                                                  Sums9 (&b)[4]) {
+#pragma unroll 1
+  for (int k = 0; k < 32; ++k) {
+    const float4 *const at = t + (lane ^ k);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float4 x = at[96 * r], ta = at[96 * r + 32], tb = at[96 * r + 64];
+      const FarTarget T{x.x, x.y, x.z, ta.x, ta.y, ta.z, tb.x, tb.y, tb.z, x.w, ta.w};
+#pragma unroll
+      for (int q = 0; q < 4; q += 2) {
+        const FarTarget &X = S[q], &Y = S[q + 1];
+        const float2 dx = make_float2(T.x - X.x, T.x - Y.x), dy = make_float2(T.y - X.y, T.y - Y.y),
+                     dz = make_float2(T.z - X.z, T.z - Y.z);
+        const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+        float2 ri2;
+        const float2 m = far_weights<CLS, UNI, KERN>(r2, make_float2(T.h + X.h, T.h + Y.h), hu, ri2);
+        float2 ft;
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+          const FarTarget &Z = S[q + o];
+          (o ? ft.y : ft.x) = far_t(T, make_float4(Z.ax, Z.ay, Z.az, 0.f), make_float4(Z.bx, Z.by, Z.bz, 0.f));
+        }
+        const float2 g = __fmul2_rn(__fmul2_rn(m, ri2), ft);
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+          const float gq = o ? g.y : g.x, ex = o ? dx.y : dx.x, ey = o ? dy.y : dy.x, ez = o ? dz.y : dz.x;
+          Sums9 &c = b[q + o], unused;
+          add_wq<SIDE_J>(T, x, x, o ? m.y : m.x, unused, c);
+          c.gx = fmaf(gq, ex, c.gx);
+          c.gy = fmaf(gq, ey, c.gy);
+          c.gz = fmaf(gq, ez, c.gz);
+        }
+      }
     }
   }
 }
@@ -267,13 +330,63 @@ __device__ __forceinline__ void fold_far(const Sums9 &s, float x, float y, float
   acc[5 * stride] += fma(g3, (double)s.gz, fma(px, Qy, -py * Qx));
 }
 
+// Particle i of a tile relative to the centre c, with its beta; `away` when there
+// is none.
+__device__ __forceinline__ FarTarget far_particle(const SymSeg &sg, int i, float cx, float cy, float cz, float away) {
+  FarTarget T{away, away, away, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 1.f, 0.f};
+  if (i < sg.n) {
+    const float4 p = sg.pos32[i], q = sg.vor32[i];
+    const float x = p.x - cx, y = p.y - cy, z = p.z - cz;
+    T = FarTarget{x, y, z, q.x, q.y, q.z, fmaf(q.y, z, -q.z * y), fmaf(q.z, x, -q.x * z), fmaf(q.x, y, -q.y * x),
+                  p.w, q.w};
+  }
+  return T;
+}
+
+// far_block_sources over a whole tile pair; t: shared memory of 6 KB of the warp's own.
+template <int CLS, bool UNI, int KERN>
+__device__ __forceinline__ void far_pair_sources(const SymSeg &sg, int I, int J, float cx, float cy, float cz, float hu,
+                                                 float4 *t, int lane, double *accJ) {
+  const double As2 = UNI ? kInv4Pi * 2.0 * (double)hu : kInv4Pi;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const FarTarget T = far_particle(sg, I * kT + 32 * r + lane, cx, cy, cz, kPadTarget);
+    t[96 * r + lane] = make_float4(T.x, T.y, T.z, T.h);
+    t[96 * r + 32 + lane] = make_float4(T.ax, T.ay, T.az, T.v);
+    t[96 * r + 64 + lane] = make_float4(T.bx, T.by, T.bz, 0.f);
+  }
+  FarTarget S[4];
+  Sums9 b[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    S[q] = far_particle(sg, J * kT + 32 * q + lane, cx, cy, cz, kPadSource);
+    b[q] = Sums9{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  }
+  __syncwarp();
+  far_block_sources<CLS, UNI, KERN>(t, lane, S, hu, b);
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int j = J * kT + 32 * q + lane;
+    const float4 l = j < sg.n ? sg.vorlo[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+    fold_far(b[q], S[q].x, S[q].y, S[q].z, S[q].ax, S[q].ay, S[q].az, l.x, l.y, l.z, As2, -3.0 * As2,
+             accJ + 32 * q + lane, kT);
+  }
+}
+
 // A far tile pair: sub-blocks [k0, k1) of 32 sources of tile J against all
 // targets of tile I, R per lane and pass.  accI: the warp's [6][128] target
 // sums; accJ: [6][128] source sums of tile J.
-template <int CLS, bool UNI, bool DIFF, int KERN, int R, int UNROLL>
+template <int SIDE, int CLS, bool UNI, bool DIFF, int KERN, int R, int UNROLL>
 __device__ __forceinline__ void far_pair(const SymSeg &sg, int I, int J, int k0, int k1, int ta, int tb,
                                          float cx, float cy, float cz, float hu, const Stage &st, int lane,
                                          double *accI, double *accJ) {
+  if constexpr (SIDE == SIDE_J && CLS != FAR_Z) {
+    if (k1 - k0 == 4) {  // (a constant where this is inlined; accI is the warp's, and not used for sums)
+      far_pair_sources<CLS, UNI, KERN>(sg, I, J, cx, cy, cz, hu, reinterpret_cast<float4 *>(accI), lane, accJ);
+      return;
+    }
+  }
   if (R == 4) {  // one pass over all targets
     if (ta > 0) return;
     tb = kT;
@@ -290,14 +403,7 @@ __device__ __forceinline__ void far_pair(const SymSeg &sg, int I, int J, int k0,
     Sums9 a[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int i = I * kT + t0 + 32 * r + lane;
-      T[r] = FarTarget{kPadTarget, kPadTarget, kPadTarget, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 1.f, 0.f};
-      if (i < n) {
-        const float4 p = pos[i], q = vor[i];
-        const float x = p.x - cx, y = p.y - cy, z = p.z - cz;
-        T[r] = FarTarget{x, y, z, q.x, q.y, q.z, fmaf(q.y, z, -q.z * y), fmaf(q.z, x, -q.x * z),
-                         fmaf(q.x, y, -q.y * x), p.w, q.w};
-      }
+      T[r] = far_particle(sg, I * kT + t0 + 32 * r + lane, cx, cy, cz, kPadTarget);
       a[r] = Sums9{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     }
 #pragma unroll 1
@@ -322,15 +428,18 @@ __device__ __forceinline__ void far_pair(const SymSeg &sg, int I, int J, int k0,
       __syncwarp();
       Sums9 b{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if constexpr (CLS == FAR_Z)
-        far_block_z<UNI, DIFF, KERN, R>(st, lane, T, hu, kap, a, b);
+        far_block_z<SIDE, UNI, DIFF, KERN, R>(st, lane, T, hu, kap, a, b);
       else
-        far_block<CLS, UNI, KERN, R, UNROLL>(st, lane, T, hu, a, b);
-      const float4 pj = st.s0[lane], qj = st.s1[lane], ej = st.s2[lane];
-      const float2 lj = st.s3[lane];
-      fold_far(b, pj.x, pj.y, pj.z, qj.x, qj.y, qj.z, ej.w, lj.x, lj.y, As2, -3.0 * As2,
-               accJ + 32 * k + lane, kT);
+        far_block<SIDE, CLS, UNI, KERN, R, UNROLL>(st, lane, T, hu, a, b);
+      if (SIDE != SIDE_I) {
+        const float4 pj = st.s0[lane], qj = st.s1[lane], ej = st.s2[lane];
+        const float2 lj = st.s3[lane];
+        fold_far(b, pj.x, pj.y, pj.z, qj.x, qj.y, qj.z, ej.w, lj.x, lj.y, As2, -3.0 * As2,
+                 accJ + 32 * k + lane, kT);
+      }
       __syncwarp();
     }
+    if (SIDE == SIDE_J) continue;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int i = I * kT + t0 + 32 * r + lane;
@@ -367,7 +476,7 @@ __device__ __forceinline__ void rotate(Sums6 &a, int m) {
 // kept; the pair of a particle with itself falls on step 0 of target `self`
 // (no target when it is outside 0..R-1).  kap: the diffusion factor in the
 // units of the s sums (15 nu, or 240 nu / h with one radius).
-template <bool UNI, bool DIAG, bool DIFF, int KERN, int R>
+template <int SIDE, bool UNI, bool DIAG, bool DIFF, int KERN, int R>
 __device__ __forceinline__ void near_block(const Stage &st, int lane, const NearTarget (&T)[R], int self,
                                            float hu, float kap, Sums6 (&a)[R], Sums6 &b) {
   // steps per iteration (the Gaussian scalars' code is four times as long): 20,011
@@ -421,13 +530,15 @@ __device__ __forceinline__ void near_block(const Stage &st, int lane, const Near
           sy = own ? 0.f : sy;
           sz = own ? 0.f : sz;
         }
-        a[r].ux = fmaf(q, cx, a[r].ux);
-        a[r].uy = fmaf(q, cy, a[r].uy);
-        a[r].uz = fmaf(q, cz, a[r].uz);
-        a[r].sx += sx;
-        a[r].sy += sy;
-        a[r].sz += sz;
-        if (!DIAG) {
+        if (SIDE != SIDE_J) {
+          a[r].ux = fmaf(q, cx, a[r].ux);
+          a[r].uy = fmaf(q, cy, a[r].uy);
+          a[r].uz = fmaf(q, cz, a[r].uz);
+          a[r].sx += sx;
+          a[r].sy += sy;
+          a[r].sz += sz;
+        }
+        if (!DIAG && SIDE != SIDE_I) {
           // alpha_i x d; subtracted at the fold
           b.ux = fmaf(q, fmaf(T[r].ay, dz, -T[r].az * dy), b.ux);
           b.uy = fmaf(q, fmaf(T[r].az, dx, -T[r].ax * dz), b.uy);
@@ -438,7 +549,7 @@ __device__ __forceinline__ void near_block(const Stage &st, int lane, const Near
         }
       }
       const int k = kk + u;
-      if (!DIAG) rotate(b, (k ^ (k + 1)) & 31);
+      if (!DIAG && SIDE != SIDE_I) rotate(b, (k ^ (k + 1)) & 31);
     }
   }
 }
@@ -454,7 +565,7 @@ __device__ __forceinline__ void fold_near(const Sums6 &s, double As2, double *ac
   acc[5 * stride] += As2 * s.sz;
 }
 
-template <bool UNI, bool DIAG, bool DIFF, int KERN>
+template <int SIDE, bool UNI, bool DIAG, bool DIFF, int KERN>
 __device__ __forceinline__ void near_pair(const SymSeg &sg, int I, int J, int k0, int k1, int ta, int tb,
                                           float hu, const Stage &st, int lane, double *accI, double *accJ) {
   constexpr int R = 2;
@@ -498,10 +609,12 @@ __device__ __forceinline__ void near_pair(const SymSeg &sg, int I, int J, int k0
       Sums6 a[R], b{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int r = 0; r < R; ++r) a[r] = b;
-      near_block<UNI, DIAG, DIFF, KERN, R>(st, lane, T, k - t0 / 32, hu, kap, a, b);
+      near_block<SIDE, UNI, DIAG, DIFF, KERN, R>(st, lane, T, k - t0 / 32, hu, kap, a, b);
+      if (SIDE != SIDE_J) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) fold_near(a[r], As2, accI + t0 + 32 * r + lane, kT);
-      if (!DIAG) fold_near(b, -As2, accJ + 32 * k + lane, kT);
+        for (int r = 0; r < R; ++r) fold_near(a[r], As2, accI + t0 + 32 * r + lane, kT);
+      }
+      if (!DIAG && SIDE != SIDE_I) fold_near(b, -As2, accJ + 32 * k + lane, kT);
       __syncwarp();
     }
   }
@@ -512,18 +625,18 @@ __device__ __forceinline__ void near_pair(const SymSeg &sg, int I, int J, int k0
 // the two tiles' boxes allow.  The classes and their bounds are pair_f32.cu's;
 // the far formulation is centred on the smaller of the two boxes, whose
 // half-diagonal bounds |x'_i| + |x'_j| by 3 |d| for every pair.
-template <bool DIFF, int KERN, int UNROLL>
+template <int SIDE, bool DIFF, int KERN, int UNROLL>
 __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, int ta, int tb,
                                           const Stage &st, int lane, double *accI, double *accJ) {
   const float4 alo = sg.boxes[2 * I], ahi = sg.boxes[2 * I + 1];
   const float4 blo = sg.boxes[2 * J], bhi = sg.boxes[2 * J + 1];
   const bool uni = KERN == KERNEL_HIGHORDER && alo.w == ahi.w && blo.w == bhi.w && alo.w == blo.w;
   const float hu = alo.w;
-  if (I == J) {
+  if (SIDE == SIDE_BOTH && I == J) {  // (a tile pair of one side has tiles of two processes)
     if (uni)
-      near_pair<true, true, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
+      near_pair<SIDE_BOTH, true, true, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
     else
-      near_pair<false, true, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
+      near_pair<SIDE_BOTH, false, true, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
     return;
   }
   const float gap2 = box_gap2(alo, ahi, blo, bhi);
@@ -532,9 +645,9 @@ __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0
   const bool far = gap2 > 0.f && gap2 >= sg.near2 && gap2 >= (first ? da : db);
   if (!far) {
     if (uni)
-      near_pair<true, false, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
+      near_pair<SIDE, true, false, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
     else
-      near_pair<false, false, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
+      near_pair<SIDE, false, false, DIFF, KERN>(sg, I, J, k0, k1, ta, tb, hu, st, lane, accI, accJ);
     return;
   }
   const float4 lo = first ? alo : blo, hi = first ? ahi : bhi;
@@ -542,35 +655,36 @@ __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0
   const float sig2max = ahi.w + bhi.w;
   if (KERN == KERNEL_GAUSSIAN) {
     if (gap2 >= 49.f * sig2max)
-      far_pair<FAR_SER, false, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<SIDE, FAR_SER, false, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_Z, false, DIFF, KERN, 2, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<SIDE, FAR_Z, false, DIFF, KERN, 2, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     return;
   }
   if (gap2 >= 256.f * sig2max) {
     if (uni)
-      far_pair<FAR_SER, true, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<SIDE, FAR_SER, true, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_SER, false, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<SIDE, FAR_SER, false, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
   } else if (gap2 >= 36.f * sig2max) {
     if (uni)
-      far_pair<FAR_NZ, true, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<SIDE, FAR_NZ, true, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_NZ, false, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<SIDE, FAR_NZ, false, DIFF, KERN, 4, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
   } else {
     if (uni)
-      far_pair<FAR_Z, true, DIFF, KERN, 2, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<SIDE, FAR_Z, true, DIFF, KERN, 2, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
     else
-      far_pair<FAR_Z, false, DIFF, KERN, 2, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
+      far_pair<SIDE, FAR_Z, false, DIFF, KERN, 2, UNROLL>(sg, I, J, k0, k1, ta, tb, cx, cy, cz, hu, st, lane, accI, accJ);
   }
 }
 
 template <bool DIFF, int KERN, int UNROLL>
 struct Pair32 {
   static constexpr int kStageBytes = ::pawan::kStageBytes;
+  template <int SIDE>
   static __device__ __forceinline__ void tile_pair(const SymSeg &sg, int I, int J, int k0, int k1, int ta, int tb,
                                                    char *st, int lane, double *accI, double *accJ) {
-    ::pawan::tile_pair<DIFF, KERN, UNROLL>(sg, I, J, k0, k1, ta, tb, stage_of(st), lane, accI, accJ);
+    ::pawan::tile_pair<SIDE, DIFF, KERN, UNROLL>(sg, I, J, k0, k1, ta, tb, stage_of(st), lane, accI, accJ);
   }
 };
 
@@ -611,27 +725,42 @@ __global__ void __launch_bounds__(Spread<2>::threads, 2)
 }
 
 template <bool DIFF, int KERN>
-SymKernel select_k(int shape) {
+__global__ void __launch_bounds__(kThreads, kBlocks)
+    sym_f32_group_sided_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
+                               const int *__restrict__ jbase, double *__restrict__ slots) {
+  sided_item<Pair32<DIFF, KERN, 2>, true>(items, segs, jbase, slots);
+}
+
+template <bool DIFF, int KERN>
+__global__ void __launch_bounds__(kThreads, kBlocks)
+    sym_f32_tile_sided_kernel(const SymItem *__restrict__ items, const SymSeg *segs,
+                              const int *__restrict__ jbase, double *__restrict__ slots) {
+  sided_item<TilePair32<DIFF, KERN>, false>(items, segs, jbase, slots);
+}
+
+template <bool DIFF, int KERN>
+SymKernel select_k(int shape, bool sided) {
+  if (sided) return shape == SYM_GROUP ? &sym_f32_group_sided_kernel<DIFF, KERN> : &sym_f32_tile_sided_kernel<DIFF, KERN>;
   return shape == SYM_GROUP  ? &sym_f32_group_kernel<DIFF, KERN>
          : shape == SYM_TILE ? &sym_f32_tile_kernel<DIFF, KERN>
          : shape == SYM_WIDE ? &sym_f32_wide_kernel<DIFF, KERN>
                              : &sym_f32_spread_kernel<DIFF, KERN>;
 }
 
-SymKernel select(int shape, bool diffusion, int kernel) {
+SymKernel select(int shape, bool sided, bool diffusion, int kernel) {
   if (kernel == KERNEL_GAUSSIAN)
-    return diffusion ? select_k<true, KERNEL_GAUSSIAN>(shape) : select_k<false, KERNEL_GAUSSIAN>(shape);
-  return diffusion ? select_k<true, KERNEL_HIGHORDER>(shape) : select_k<false, KERNEL_HIGHORDER>(shape);
+    return diffusion ? select_k<true, KERNEL_GAUSSIAN>(shape, sided) : select_k<false, KERNEL_GAUSSIAN>(shape, sided);
+  return diffusion ? select_k<true, KERNEL_HIGHORDER>(shape, sided) : select_k<false, KERNEL_HIGHORDER>(shape, sided);
 }
 
 }  // namespace
 
 cudaError_t sym_f32_occupancy(bool diffusion, int kernel, int *blocks_per_sm) {
-  return sym_occupancy(select(SYM_GROUP, diffusion, kernel), sym_smem_bytes(SYM_GROUP, kStageBytes), blocks_per_sm);
+  return sym_occupancy(select(SYM_GROUP, false, diffusion, kernel), sym_smem_bytes(SYM_GROUP, kStageBytes), blocks_per_sm);
 }
 
-cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem *items, int n_items, int sm_count,
-                           const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
+cudaError_t launch_sym_f32(bool group, bool sided, bool diffusion, int kernel, const SymItem *items, int n_items,
+                           int sm_count, const SymSeg *segs, const int *jbase, double *slots, cudaStream_t s) {
   // Up to one tile pair per SM a launch lasts as long as one tile pair's chain of
   // steps: eight warps take it in less time than four, and two SMs in less than
   // one (two warps a scheduler issue at 0.8 per cycle, one alone at 0.6).  One
@@ -639,10 +768,11 @@ cudaError_t launch_sym_f32(bool group, bool diffusion, int kernel, const SymItem
   // 512 16.2 / 13.0, 1,408 17.5 / 14.5.  With more than two blocks per SM-pair the
   // clusters are not placed evenly: 2,048 19.1 / 21.8 (four warps: 24.6).
   const int shape = group                     ? SYM_GROUP
+                    : sided                   ? SYM_TILE
                     : 2 * n_items <= sm_count ? SYM_SPREAD
                     : n_items <= sm_count     ? SYM_WIDE
                                               : SYM_TILE;
-  return sym_launch(select(shape, diffusion, kernel), shape, kStageBytes, items, n_items, segs, jbase, slots, s);
+  return sym_launch(select(shape, sided, diffusion, kernel), shape, kStageBytes, items, n_items, segs, jbase, slots, s);
 }
 
 }  // namespace pawan

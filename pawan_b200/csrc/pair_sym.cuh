@@ -3,8 +3,9 @@
 // and where its sums go.  F::tile_pair computes, in one warp, sub-blocks [k0, k1)
 // of 32 sources of tile J >= I against the targets [t0, t1) of tile I (a form
 // that needs all of them takes them when t0 is 0), adding to accI ([6][128], tile
-// I's sums) and accJ ([6][128], tile J's); F::kStageBytes is a warp's shared
-// memory.
+// I's sums) and accJ ([6][128], tile J's), or to one of them alone (its SIDE
+// parameter; those sums are the same, bit for bit); F::kStageBytes is a warp's
+// shared memory.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -21,7 +22,7 @@ constexpr int kT = kSymTile;  // particles per tile
 constexpr unsigned kFull = 0xffffffffu;
 
 // Large systems: item = group a of four tiles against the groups [b0, b1).
-template <class F>
+template <class F, int SIDE = SIDE_BOTH>
 __device__ __forceinline__ void group_item(const SymItem *__restrict__ items, const SymSeg *segs,
                                            const int *__restrict__ jbase, double *__restrict__ slots) {
   extern __shared__ float4 smem_sym[];
@@ -33,9 +34,11 @@ __device__ __forceinline__ void group_item(const SymItem *__restrict__ items, co
   start_next();
   const SymSeg &sg = wait_previous(segs)[it.seg];
   const int nt = (sg.n + kT - 1) / kT;
-  for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accI[q] = 0.0;
+  if (SIDE != SIDE_J)
+    for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accI[q] = 0.0;
   for (int b = it.b0; b < it.b1; ++b) {
-    for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accJ[q] = 0.0;
+    if (SIDE != SIDE_I)
+      for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accJ[q] = 0.0;
     __syncthreads();
     for (int r = 0; r < kWarps; ++r) {
       const int c = (warp + r) & 3;
@@ -43,12 +46,14 @@ __device__ __forceinline__ void group_item(const SymItem *__restrict__ items, co
       // inside one group: each unordered tile pair once (rounds 0, 1 and half of 2)
       const bool mine = b > it.a || r < 2 || (r == 2 && warp < 2);
       if (mine && I < nt && J < nt)
-        F::tile_pair(sg, min(I, J), max(I, J), 0, 4, 0, kT, st, lane,
-                     (I <= J ? accI + warp * 6 * kT : accJ + c * 6 * kT),
-                     (I <= J ? accJ + c * 6 * kT : accI + warp * 6 * kT));
+        F::template tile_pair<SIDE>(sg, min(I, J), max(I, J), 0, 4, 0, kT, st, lane,
+                                    (I <= J ? accI + warp * 6 * kT : accJ + c * 6 * kT),
+                                    (I <= J ? accJ + c * 6 * kT : accI + warp * 6 * kT));
       __syncthreads();
     }
-    if (b == it.a) {
+    if (SIDE == SIDE_I) {
+      continue;  // (nothing of group b is kept, and the round above ended in a barrier)
+    } else if (b == it.a) {
       for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accI[q] += accJ[q];
     } else {
       const int jb = jbase[it.jb + b];
@@ -66,7 +71,7 @@ __device__ __forceinline__ void group_item(const SymItem *__restrict__ items, co
 }
 
 // Small systems: item = one tile pair (a, b0); each warp 32 of its sources.
-template <class F>
+template <class F, int SIDE = SIDE_BOTH>
 __device__ __forceinline__ void tile_item(const SymItem *__restrict__ items, const SymSeg *segs,
                                           const int *__restrict__ jbase, double *__restrict__ slots) {
   extern __shared__ float4 smem_sym[];
@@ -83,7 +88,7 @@ __device__ __forceinline__ void tile_item(const SymItem *__restrict__ items, con
 #pragma unroll
   for (int k = 0; k < 6; ++k) accJ[k * kT + tid] = 0.0;
   const SymSeg &sg = wait_previous(segs)[it.seg];
-  F::tile_pair(sg, it.a, it.b0, warp, warp + 1, 0, kT, st, lane, mine, accJ);
+  F::template tile_pair<SIDE>(sg, it.a, it.b0, warp, warp + 1, 0, kT, st, lane, mine, accJ);
   const int jb = it.b0 > it.a ? jbase[it.jb + it.b0] : -1;
   if (jb >= 0) {
     // this thread's own source
@@ -132,8 +137,8 @@ __device__ __forceinline__ void spread_item(const SymItem *__restrict__ items, c
   for (int q = tid; q < (kSubs + 2) * kC; q += kN) accI[q] = 0.0;
   __syncthreads();
   wait_previous_for(sg.pos32, sg.vor32, sg.poslo, sg.vorlo, sg.pos64, sg.vor64, sg.boxes);
-  F::tile_pair(sg, it.a, it.b0, sub, sub + 1, half * (kT / 2), (half + 1) * (kT / 2), st, lane, accI + own * kC,
-               accJ + half * kC);
+  F::template tile_pair<SIDE_BOTH>(sg, it.a, it.b0, sub, sub + 1, half * (kT / 2), (half + 1) * (kT / 2), st, lane,
+                                   accI + own * kC, accJ + half * kC);
   if constexpr (C > 1)
     cg::this_cluster().sync();
   else
@@ -168,11 +173,41 @@ __device__ __forceinline__ void spread_item(const SymItem *__restrict__ items, c
   }
 }
 
+// Sharded systems: an item between a group of this process and one of another
+// forms the own group's sums alone (28 of a far step's 37 operations and none of
+// its shuffles, the sums bit for bit those of an unsharded launch).  One kernel for
+// all three kinds, so that a launch has one last wave.  A rank's right-hand side on
+// one B200, slowest of the ranks of 2 / 4 / 8, against forming both sides: ring pair
+// at N = 131,072 8.59 / 4.63 / 2.48 ms, 10.38 / 6.18 / 3.42 (one-sided kernel, every
+// ordered pair: 9.26 / 4.69 / 2.40); FP64 at 65,536 8.25 / 4.76 / 2.62, 9.15 / 5.45 /
+// 3.01; Gaussian at 65,536 2.36 / 1.45 / 0.88, 2.91 / 1.81 / 1.13.
+template <class F, bool GROUP>
+__device__ __forceinline__ void sided_item(const SymItem *__restrict__ items, const SymSeg *segs,
+                                           const int *__restrict__ jbase, double *__restrict__ slots) {
+  const int side = items[blockIdx.x].side;
+  if (GROUP) {
+    if (side == SIDE_I)
+      group_item<F, SIDE_I>(items, segs, jbase, slots);
+    else if (side == SIDE_J)
+      group_item<F, SIDE_J>(items, segs, jbase, slots);
+    else
+      group_item<F>(items, segs, jbase, slots);
+  } else {
+    if (side == SIDE_I)
+      tile_item<F, SIDE_I>(items, segs, jbase, slots);
+    else if (side == SIDE_J)
+      tile_item<F, SIDE_J>(items, segs, jbase, slots);
+    else
+      tile_item<F>(items, segs, jbase, slots);
+  }
+}
+
 using SymKernel = void (*)(const SymItem *, const SymSeg *, const int *, double *);
 
 // How a launch's blocks are shaped: groups of tiles, single tile pairs, or
 // single tile pairs over eight warps of one block or of a cluster of two.
 enum SymShape { SYM_GROUP = 0, SYM_TILE = 1, SYM_WIDE = 2, SYM_SPREAD = 3 };
+// (a sharded plan's kernel has the first two shapes only)
 
 inline int sym_cluster(int shape) { return shape == SYM_SPREAD ? 2 : 1; }
 inline int sym_threads(int shape) { return shape == SYM_WIDE ? Spread<1>::threads : kThreads; }

@@ -141,15 +141,16 @@ struct SymLayout {
   }
 };
 
-SymLayout sym_layout(size_t n, int items_per_slot, double bytes) {
+SymLayout sym_layout(size_t n, int items_per_slot, double bytes, int world = 1) {
   SymLayout l;
   const int nt = (int)((n + kSymTile - 1) / kSymTile);
   l.g = nt <= kSymTilesMax ? 1 : kSymGroup;
   l.ng = (nt + l.g - 1) / l.g;
   if (l.g > 1) {
     // longer runs write fewer target-side sums; at least some dozens of items
-    // per resident block (444 of them) keep the last ones from trailing
-    const double pairs = 0.5 * (double)l.ng * (double)(l.ng + 1);
+    // per resident block (444 of them) keep the last ones from trailing (a rank of
+    // a sharded system has its share of the pairs, most of them twice)
+    const double pairs = 0.5 * (double)l.ng * (double)(l.ng + 1) * std::min(1.0, 2.0 / world);
     l.run = std::max(1, std::min(4, (int)(pairs / (444.0 * std::max(1, items_per_slot)))));
   }
   const double slot = 48.0 * kSymTile * l.g;
@@ -199,7 +200,8 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, bool serving) {
   std::vector<SymLayout> lay;
   size_t n_phases = 0;
   for (auto *y : p.systems) {
-    lay.push_back(sym_layout(y->n, p.tile.items_per_slot, serving ? kSymSlotBytesServing : kSymSlotBytes));
+    lay.push_back(sym_layout(y->n, p.tile.items_per_slot, serving ? kSymSlotBytesServing : kSymSlotBytes,
+                             y->shard.active ? y->shard.world : 1));
     n_phases = std::max(n_phases, lay.back().rows.size() - 1);
   }
   // systems with the most tiles first
@@ -253,17 +255,23 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, bool serving) {
       std::vector<Costed> late;
       for (int a = r0; a < r1; ++a) {
         int k = 0;
-        for (int b0 = a; b0 < l.ng; b0 += l.run, ++k) {
-          const int b1 = std::min(l.ng, b0 + l.run);
+        for (int first = a; first < l.ng; first += l.run, ++k) {
+          int b0 = first, b1 = std::min(l.ng, first + l.run);
+          if (!owned(a)) {  // of the run the groups of this process alone (neighbours)
+            while (b0 < b1 && !owned(b0)) ++b0;
+            while (b0 < b1 && !owned(b1 - 1)) --b1;
+            if (b0 == b1) continue;
+          }
           double cost = 0.0;  // interactions credited: ordered pairs of owned targets
-          bool any = owned(a);
+          bool sources = false;
           for (int b = b0; b < b1; ++b) {
-            any = any || owned(b);
+            sources = sources || owned(b);
             const double both = particles(a) * particles(b);
             cost += (owned(a) ? both : 0.0) + (b != a && owned(b) ? both : 0.0);
           }
-          if (!any) continue;
-          const Costed c{SymItem{(int)s, a, b0, b1, i0[a] < 0 ? -1 : i0[a] + k, r0, jb}, cost, 0};
+          const int side = !owned(a) ? SIDE_J : sources ? SIDE_BOTH : SIDE_I;
+          if (side != SIDE_BOTH) p.sided = true;
+          const Costed c{SymItem{(int)s, a, b0, b1, i0[a] < 0 ? -1 : i0[a] + k, r0, jb, side}, cost, 0};
           if (b0 <= a + (l.g > 1 ? 1 : 2))
             mine[grouped].push_back(c);
           else
@@ -590,7 +598,7 @@ static int launch_sym_range(pawan_ctx *ctx, Plan &p, int first, int count) {
       if (lo >= hi) continue;
       double *slots = p.slots.p + (group ? 0 : p.tile_slots);
       const auto launch = p.precision == PAWAN_PREC_F64 ? launch_sym_f64 : launch_sym_f32;
-      PAWAN_CUDA(ctx, launch(group, p.diffusion, p.kernel, p.sym_items.p + lo, hi - lo, ctx->sm_count,
+      PAWAN_CUDA(ctx, launch(group, p.sided, p.diffusion, p.kernel, p.sym_items.p + lo, hi - lo, ctx->sm_count,
                              p.sym_segs.p, p.sym_jbase.p, slots, ctx->stream));
       ctx->launches++;
     }

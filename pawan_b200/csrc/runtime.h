@@ -192,6 +192,7 @@ struct Plan {
   // launch for the sums, `rates` not used
   bool fused_sums = false;
   double slot_bytes = 0.0;  // bytes of all slots that one right-hand side sums
+  bool sided = false;     // some items form one side's sums only
   size_t tile_slots = 0;  // doubles before the slots of the single-tile items
   DBuf<float4> boxes;
   DBuf<WorkItem> items;
