@@ -17,7 +17,7 @@ size_t pawan_system::device_bytes() const {
          vol.bytes() + wake_id.bytes() + pos32.bytes() + vor32.bytes() + poslo.bytes() +
          vorlo.bytes() + pos64.bytes() +
          vor64.bytes() + diag_scratch.bytes() + diag_out.bytes() + Xc.bytes() + field.bytes() + columns.bytes() +
-         (plan ? plan->partial.bytes() + plan->rates.bytes() + plan->tile_count.bytes() + plan->slots.bytes() : 0);
+         (plan ? plan->partial.bytes() + plan->rates.bytes() + plan->tile_count.bytes() + 8 * plan->slot_count : 0);
 }
 
 // =================================================================== C ABI

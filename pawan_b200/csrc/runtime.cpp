@@ -73,9 +73,13 @@ std::vector<TileChoice> tile_candidates(int precision, int kernel) {
   return v;
 }
 
-Plan::~Plan() {
+Plan::~Plan() { drop_graph(); }
+
+void Plan::drop_graph() {
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
   if (graph) cudaGraphDestroy(graph);
+  graph_exec = nullptr;
+  graph = nullptr;
 }
 
 bool Plan::stale() const {
@@ -122,10 +126,15 @@ static size_t shard_count(const pawan_system *y) {
 // blocks to fill the device from a few thousand particles on), a larger one by
 // groups of kSymGroup tiles, whose sums are written once per four tile pairs.
 constexpr int kSymTilesMax = 256;
-// Bound on one system's slots: the rows of groups are processed in phases, the
-// slots of a phase summed into the rates before the next reuses them.  The
-// serving engine holds many systems at a time, so its bound is smaller.
+// Bound on one system's slots: the rows of groups (or tiles) are processed in
+// phases, the slots of a phase summed into the rates before the next reuses them.
+// The serving engine holds many systems at a time, so its bound is smaller.  (One
+// row's slots are the least: 6 KB per 128 particles, and as much again.)
 constexpr double kSymSlotBytes = 2.0e9, kSymSlotBytesServing = 4.0e8;
+// Bound on the slots of all systems of a plan (or one phase of one of them): plans
+// over more run in waves that reuse them.  512 ragged rings of 512 to 16,384
+// particles hold 7.4e9 bytes in one wave.
+constexpr double kPlanSlotBytes = 8.0e9;
 
 namespace {
 
@@ -155,10 +164,6 @@ SymLayout sym_layout(size_t n, int items_per_slot, double bytes, int world = 1) 
   }
   const double slot = 48.0 * kSymTile * l.g;
   l.rows.push_back(0);
-  if (l.g == 1) {
-    l.rows.push_back(l.ng);
-    return l;
-  }
   int r0 = 0;
   while (r0 < l.ng) {
     int r1 = r0;
@@ -188,51 +193,113 @@ double sym_slot_bytes(size_t n, bool serving) {
   return most * 48.0 * kSymTile * l.g;
 }
 
-// Items, slots and sums of a plan on the symmetric engine.  A system's
-// decomposition depends on its own size and the tiling only, so its arithmetic
-// does not depend on the other systems of the plan.
-static int build_sym_work(pawan_ctx *ctx, Plan &p, bool serving) {
-  struct Costed {
-    SymItem w;
-    double cost;
-    int late;  // 0: holds tile pairs next to the diagonal (near ones, which take longest)
+namespace {
+
+// Whether this process computes particles of group t of a system (all of them
+// when it is not sharded; block starts are multiples of a group).
+bool sym_owned(const pawan_system *y, const SymLayout &l, int t) {
+  if (!y->shard.active) return true;
+  const size_t per = (size_t)kSymTile * l.g, f = shard_first(y);
+  return t * per < f + shard_count(y) && (t + 1) * per > f;
+}
+
+// The systems' decompositions, and which phases of which systems share a wave:
+// a wave's slots are summed before the next wave reuses them.
+struct SymWaves {
+  struct Unit {
+    size_t system;
+    int phase;
   };
   std::vector<SymLayout> lay;
-  size_t n_phases = 0;
-  for (auto *y : p.systems) {
-    lay.push_back(sym_layout(y->n, p.tile.items_per_slot, serving ? kSymSlotBytesServing : kSymSlotBytes,
-                             y->shard.active ? y->shard.world : 1));
-    n_phases = std::max(n_phases, lay.back().rows.size() - 1);
-  }
-  // systems with the most tiles first
+  std::vector<std::vector<Unit>> waves;  // systems with the most tiles first
+};
+
+SymWaves sym_waves(const Plan &p, bool serving) {
+  SymWaves w;
+  for (auto *y : p.systems)
+    w.lay.push_back(sym_layout(y->n, p.tile.items_per_slot, serving ? kSymSlotBytesServing : kSymSlotBytes,
+                               y->shard.active ? y->shard.world : 1));
   std::vector<size_t> order(p.systems.size());
   std::iota(order.begin(), order.end(), (size_t)0);
   std::stable_sort(order.begin(), order.end(),
                    [&](size_t a, size_t b) { return p.systems[a]->n > p.systems[b]->n; });
+  std::vector<double> used;  // bytes of each wave
+  for (size_t s : order) {
+    const SymLayout &l = w.lay[s];
+    size_t k = 0;  // a system's phases in waves of increasing number
+    for (size_t ph = 0; ph + 1 < l.rows.size(); ++ph, ++k) {
+      double need = 0.0;
+      for (int t = 0; t < l.ng; ++t)
+        if (sym_owned(p.systems[s], l, t)) need += l.slots(t, l.rows[ph], l.rows[ph + 1]);
+      need *= 48.0 * kSymTile * l.g;
+      while (k < used.size() && used[k] > 0.0 && used[k] + need > kPlanSlotBytes) ++k;
+      if (k == used.size()) {
+        used.push_back(0.0);
+        w.waves.emplace_back();
+      }
+      used[k] += need;
+      w.waves[k].push_back({s, (int)ph});
+    }
+  }
+  return w;
+}
+
+}  // namespace
+
+// At least `count` doubles of slots.  The larger buffer is taken before the old one
+// is given back, or, where both do not fit, after it.
+static int reserve_slots(pawan_ctx *ctx, SlotPool &pool, size_t count) {
+  if (pool.buf.n >= count) return PAWAN_OK;
+  DBuf<double> larger;
+  if (pool.buf.ordered) larger.ordered_on(pool.buf.stream);
+  cudaError_t e = larger.alloc(count);
+  if (e == cudaErrorMemoryAllocation && pool.buf.p) {
+    cudaGetLastError();
+    pool.buf.reset();
+    if (pool.buf.ordered) cudaStreamSynchronize(pool.buf.stream);
+    e = larger.alloc(count);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return cuda_fail(ctx, e, "pair-sum slots");
+  }
+  std::swap(pool.buf.p, larger.p);
+  std::swap(pool.buf.n, larger.n);
+  return PAWAN_OK;
+}
+
+// Items, slots and sums of a plan on the symmetric engine.  A system's
+// decomposition depends on its own size and the tiling only, so its arithmetic
+// does not depend on the other systems of the plan.
+static int build_sym_work(pawan_ctx *ctx, Plan &p, const SymWaves &w) {
+  struct Costed {
+    SymItem w;
+    double cost;
+  };
   std::vector<SymItem> items;
   std::vector<SymSum> sums;
   std::vector<int> jbase;
-  size_t group_slots = 0, tile_slots = 0;  // most doubles of any phase
-  std::vector<std::vector<SymSum>> tile_sums(n_phases);
-  p.phases.assign(n_phases, Plan::Phase{});
-  for (size_t ph = 0; ph < n_phases; ++ph) {
-    Plan::Phase &P = p.phases[ph];
+  size_t group_slots = 0, tile_slots = 0;  // most doubles of any wave
+  const size_t n_waves = w.waves.size();
+  std::vector<std::vector<SymSum>> tile_sums(n_waves);
+  p.waves.assign(n_waves, Plan::Wave{});
+  for (size_t k = 0; k < n_waves; ++k) {
+    Plan::Wave &P = p.waves[k];
     P.sum0 = (int)sums.size();
     size_t used[2] = {0, 0};  // slots so far: single-tile systems, grouped ones
+    // items in launch order: those with tile pairs next to the diagonal, which take
+    // longest, before a system's others
     std::vector<Costed> mine[2];
     std::vector<SymSum> of_tiles;
-    for (size_t s : order) {
-      const SymLayout &l = lay[s];
-      if (ph + 1 >= l.rows.size()) continue;
+    for (const SymWaves::Unit &unit : w.waves[k]) {
+      const size_t s = unit.system;
+      const int ph = unit.phase;
+      const SymLayout &l = w.lay[s];
       const pawan_system *y = p.systems[s];
       const int grouped = l.g > 1 ? 1 : 0, per = kSymTile * l.g;
       const int n = (int)y->n, nt = (n + kSymTile - 1) / kSymTile;
       const int r0 = l.rows[ph], r1 = l.rows[ph + 1];
-      // groups whose particles this process computes (all of them when the
-      // system is not sharded; block starts are multiples of a group)
-      const int f = y->shard.active ? (int)shard_first(y) : 0;
-      const int e = y->shard.active ? f + (int)shard_count(y) : n;
-      auto owned = [&](int t) { return t * per < e && (t + 1) * per > f; };
+      auto owned = [&](int t) { return sym_owned(y, l, t); };
       auto particles = [&](int t) { return (double)(std::min(n, (t + 1) * per) - t * per); };
       const int jb = (int)jbase.size();
       std::vector<int> i0(l.ng, -1);
@@ -254,8 +321,8 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, bool serving) {
       }
       std::vector<Costed> late;
       for (int a = r0; a < r1; ++a) {
-        int k = 0;
-        for (int first = a; first < l.ng; first += l.run, ++k) {
+        int run = 0;
+        for (int first = a; first < l.ng; first += l.run, ++run) {
           int b0 = first, b1 = std::min(l.ng, first + l.run);
           if (!owned(a)) {  // of the run the groups of this process alone (neighbours)
             while (b0 < b1 && !owned(b0)) ++b0;
@@ -271,7 +338,7 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, bool serving) {
           }
           const int side = !owned(a) ? SIDE_J : sources ? SIDE_BOTH : SIDE_I;
           if (side != SIDE_BOTH) p.sided = true;
-          const Costed c{SymItem{(int)s, a, b0, b1, i0[a] < 0 ? -1 : i0[a] + k, r0, jb, side}, cost, 0};
+          const Costed c{SymItem{(int)s, a, b0, b1, i0[a] < 0 ? -1 : i0[a] + run, r0, jb, side}, cost};
           if (b0 <= a + (l.g > 1 ? 1 : 2))
             mine[grouped].push_back(c);
           else
@@ -282,26 +349,23 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, bool serving) {
     }
     P.groups = (int)mine[1].size();
     P.tiles = (int)mine[0].size();
-    for (int k : {1, 0})
-      for (const Costed &c : mine[k]) {
+    for (int grouped : {1, 0})
+      for (const Costed &c : mine[grouped]) {
         items.push_back(c.w);
         p.item_costs.push_back(c.cost);
       }
     group_slots = std::max(group_slots, used[1] * 6 * kSymTile * kSymGroup);
     tile_slots = std::max(tile_slots, used[0] * 6 * kSymTile);
-    tile_sums[ph] = of_tiles;
+    tile_sums[k] = of_tiles;
     sums.insert(sums.end(), of_tiles.begin(), of_tiles.end());
     P.sums = (int)sums.size() - P.sum0;
   }
   // the single-tile items' slots lie behind the groups'
-  for (size_t ph = 0; ph < n_phases; ++ph) {
-    const size_t k = tile_sums[ph].size(), at = (size_t)(p.phases[ph].sum0 + p.phases[ph].sums) - k;
-    for (size_t q = 0; q < k; ++q) sums[at + q].first += (long long)group_slots;
+  for (size_t k = 0; k < n_waves; ++k) {
+    const size_t c = tile_sums[k].size(), at = (size_t)(p.waves[k].sum0 + p.waves[k].sums) - c;
+    for (size_t q = 0; q < c; ++q) sums[at + q].first += (long long)group_slots;
   }
   p.tile_slots = group_slots;
-  p.fused_sums = n_phases == 1;
-  for (auto *y : p.systems)
-    if (y->shard.active) p.fused_sums = false;
   for (const SymSum &s : sums) p.slot_bytes += (double)s.count * 48.0 * kSymTile;
   if (items.size() > (size_t)INT32_MAX) return fail(ctx, PAWAN_ERR_INVALID, "too many work items");
   p.n_items = (int)items.size();
@@ -312,7 +376,8 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, bool serving) {
     segs.push_back(SymSeg{g.pos32, g.vor32, g.poslo, g.vorlo, g.pos64, g.vor64, g.boxes,
                           (int)y->n, y->nu, (float)(y->r_near * y->r_near)});
   }
-  PAWAN_CUDA(ctx, p.slots.alloc(group_slots + tile_slots));
+  p.slot_count = group_slots + tile_slots;
+  PAWAN_TRY(reserve_slots(ctx, *p.pool, p.slot_count));
   PAWAN_CUDA(ctx, p.sym_items.alloc(items.size()));
   PAWAN_CUDA(ctx, p.sym_segs.alloc(segs.size()));
   PAWAN_CUDA(ctx, p.sym_jbase.alloc(jbase.size()));
@@ -337,7 +402,7 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, bool serving) {
 // target tile's chunks are consecutive.
 int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int precision,
                const TileChoice &tile, std::unique_ptr<Plan> &out, int fixed_chunk_sources,
-               bool ordered_alloc) {
+               bool ordered_alloc, bool own_slots) {
   if (systems.empty()) return fail(ctx, PAWAN_ERR_INVALID, "plan over no systems");
   const int kernel = systems[0]->kernel;
   for (auto *s : systems)
@@ -359,11 +424,23 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
     p->interactions += targets * (double)s->n;
   }
   int bps = 0;
+  SymWaves waves;
   p->sym = tile_symmetric(precision, tile.pc);
   if (p->sym) {
     cudaError_t e = precision == PAWAN_PREC_F64 ? sym_f64_occupancy(p->diffusion, kernel, &bps)
                                                 : sym_f32_occupancy(p->diffusion, kernel, &bps);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy query");
+    if (bps < 1) return fail(ctx, PAWAN_ERR_INVALID, "pair kernel does not fit on an SM");
+    waves = sym_waves(*p, fixed_chunk_sources > 0);
+    p->fused_sums = waves.waves.size() == 1;
+    for (auto *s : systems)
+      if (s->shard.active) p->fused_sums = false;
+    if (!own_slots) p->pool = ctx->slots.lock();
+    if (!p->pool) {
+      p->pool = std::make_shared<SlotPool>();
+      if (ordered_alloc) p->pool->buf.ordered_on(ctx->stream);
+      if (!own_slots) ctx->slots = p->pool;
+    }
   } else {
     PAWAN_TRY(occupancy(ctx, precision, tile.pc, p->diffusion, kernel, &bps));
   }
@@ -380,7 +457,8 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
   };
   std::vector<ItemCost> items;
   // per system: partial slots [target tiles][chunks][6][TPB] (none with one
-  // chunk), rates [6][n], one counter per target tile
+  // chunk), rates [6][n] (none where the stage sums the slots), one counter per
+  // target tile (one-sided kernels)
   if (TPB % 8 != 0) return fail(ctx, PAWAN_ERR_INVALID, "targets per block must be a multiple of 8");
   size_t partial_total = 0, box_total = 0, rates_total = 0, count_total = 0;
   std::vector<size_t> partial_off(systems.size()), box_off(systems.size());
@@ -400,9 +478,9 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
     partial_off[s] = partial_total;
     if (nch > 1) partial_total += target_tiles * (size_t)nch * 6 * (size_t)TPB;
     rates_off[s] = rates_total;
-    rates_total += 6 * (size_t)n;
+    if (!p->fused_sums) rates_total += 6 * (size_t)n;
     count_off[s] = count_total;
-    count_total += target_tiles;
+    if (!p->sym) count_total += target_tiles;
     box_off[s] = box_total;
     box_total += 2 * (size_t)src_tiles;
     // targets: all particles, or this process's block of a sharded system
@@ -446,7 +524,6 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
     p->sym_segs.ordered_on(ctx->stream);
     p->sym_jbase.ordered_on(ctx->stream);
     p->sym_sums.ordered_on(ctx->stream);
-    p->slots.ordered_on(ctx->stream);
   }
   PAWAN_CUDA(ctx, p->partial.alloc(partial_total));
   // the pair kernels discard the slots' L2 lines after summing them: every
@@ -455,7 +532,8 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
     return fail(ctx, PAWAN_ERR_CUDA, "partial-sum buffer not 128-byte aligned");
   PAWAN_CUDA(ctx, p->rates.alloc(rates_total));
   PAWAN_CUDA(ctx, p->tile_count.alloc(count_total));
-  PAWAN_CUDA(ctx, cudaMemsetAsync(p->tile_count.p, 0, p->tile_count.bytes(), ctx->stream));
+  if (count_total > 0)
+    PAWAN_CUDA(ctx, cudaMemsetAsync(p->tile_count.p, 0, p->tile_count.bytes(), ctx->stream));
   PAWAN_CUDA(ctx, p->boxes.alloc(box_total));
   std::vector<WorkItem> wh(items.size());
   p->item_costs.resize(items.size());
@@ -477,8 +555,8 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
     d.vor64 = y->vor64.p;
     d.boxes = p->boxes.p + box_off[s];
     d.partial = p->nchunks[s] > 1 ? p->partial.p + partial_off[s] : nullptr;
-    d.rates = p->rates.p + rates_off[s];
-    d.tile_count = p->tile_count.p + count_off[s];
+    d.rates = rates_total > 0 ? p->rates.p + rates_off[s] : nullptr;
+    d.tile_count = count_total > 0 ? p->tile_count.p + count_off[s] : nullptr;
     d.n = (int)y->n;
     d.nchunks = p->nchunks[s];
     d.nu = y->nu;
@@ -518,7 +596,7 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
   p->n_stage_blocks = (int)sih.size();
   p->n_shard_blocks = (int)shh.size();
   p->dts.assign(systems.size(), 0.0);
-  if (p->sym) PAWAN_TRY(build_sym_work(ctx, *p, fixed_chunk_sources > 0));
+  if (p->sym) PAWAN_TRY(build_sym_work(ctx, *p, waves));
   PAWAN_CUDA(ctx, p->items.alloc(wh.size()));
   PAWAN_CUDA(ctx, p->segs.alloc(sh.size()));
   PAWAN_CUDA(ctx, p->stage_items.alloc(sih.size()));
@@ -587,23 +665,24 @@ static cudaEvent_t take_event(pawan_ctx *ctx) {
 }
 
 // Work items [first, first + count) of a plan on the symmetric engine, and the
-// slot sums of every phase whose last item is among them.
+// slot sums of every wave whose last item is among them.
 static int launch_sym_range(pawan_ctx *ctx, Plan &p, int first, int count) {
+  PAWAN_TRY(reserve_slots(ctx, *p.pool, p.slot_count));
   int at = 0;
-  for (const Plan::Phase &ph : p.phases) {
+  for (const Plan::Wave &ph : p.waves) {
     for (bool group : {true, false}) {
       const int n = group ? ph.groups : ph.tiles;
       const int lo = std::max(first, at), hi = std::min(first + count, at + n);
       at += n;
       if (lo >= hi) continue;
-      double *slots = p.slots.p + (group ? 0 : p.tile_slots);
+      double *slots = p.pool->buf.p + (group ? 0 : p.tile_slots);
       const auto launch = p.precision == PAWAN_PREC_F64 ? launch_sym_f64 : launch_sym_f32;
       PAWAN_CUDA(ctx, launch(group, p.sided, p.diffusion, p.kernel, p.sym_items.p + lo, hi - lo, ctx->sm_count,
                              p.sym_segs.p, p.sym_jbase.p, slots, ctx->stream));
       ctx->launches++;
     }
     if (!p.fused_sums && at > first && at <= first + count) {
-      PAWAN_CUDA(ctx, launch_sym_sums(p.sym_sums.p + ph.sum0, ph.sums, p.stage_descs.p, p.slots.p, ctx->stream));
+      PAWAN_CUDA(ctx, launch_sym_sums(p.sym_sums.p + ph.sum0, ph.sums, p.stage_descs.p, p.pool->buf.p, ctx->stream));
       ctx->launches++;
     }
   }
@@ -701,7 +780,7 @@ int launch_stage_mode(pawan_ctx *ctx, Plan &p, int mode) {
     PAWAN_CUDA(ctx, cudaEventRecord(e0, ctx->stream));
   }
   cudaError_t e = p.fused_sums && mode != STAGE_PACK
-                      ? launch_sum_stage(mode, p.phases[0].sums, p.sym_sums.p, p.stage_descs.p, p.slots.p, ctx->stream)
+                      ? launch_sum_stage(mode, p.waves[0].sums, p.sym_sums.p, p.stage_descs.p, p.pool->buf.p, ctx->stream)
                       : launch_stage(mode, p.n_stage_blocks, p.stage_items.p, p.stage_descs.p, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "stage kernel launch");
   ctx->launches++;
@@ -739,6 +818,13 @@ int rk4_steps(pawan_ctx *ctx, Plan &p, size_t nsteps, bool use_graph) {
   if (!use_graph) {
     for (size_t k = 0; k < nsteps; ++k) PAWAN_TRY(rk4_one_step(ctx, p, true));
     return PAWAN_OK;
+  }
+  if (p.sym) {
+    // (a captured graph holds the slots' address: nothing can be reserved under
+    // capture, and a plan that needed more has moved them)
+    PAWAN_TRY(reserve_slots(ctx, *p.pool, p.slot_count));
+    if (p.graph_exec && p.graph_slots != p.pool->buf.p) p.drop_graph();
+    p.graph_slots = p.pool->buf.p;
   }
   if (!p.graph_exec) {
     for (size_t s = 0; s < p.systems.size(); ++s)

@@ -80,6 +80,15 @@ const std::vector<int> kTuneItemsPerSlot = {4, 8, 32, 64, 128};
 
 struct Plan;
 
+// Slots of the symmetric pair engine.  A right-hand side's slots are summed before
+// another plan of the context launches anything, and the launches are ordered on
+// its stream, so the plans of a context share one buffer of the size of the largest
+// plan's (at most 8 GB, or one row of tiles); the last plan to go gives it back.  A
+// plan whose stages are split over calls has slots of its own.
+struct SlotPool {
+  DBuf<double> buf;
+};
+
 }  // namespace pawan
 
 struct pawan_ctx {
@@ -109,6 +118,7 @@ struct pawan_ctx {
   char *staging = nullptr;
   size_t staging_bytes = 0;
   cudaEvent_t staging_events[4] = {};
+  std::weak_ptr<pawan::SlotPool> slots;  // held by the plans
   void *flush_buf = nullptr;
   size_t flush_bytes = 0;
   // autotune results: (precision, diffusion, log2 sum n^2, log2 segments) -> tile
@@ -175,21 +185,22 @@ struct Plan {
   DBuf<double> partial;   // per system [target tiles][chunks][6][tpb] (chunks > 1)
   DBuf<double> rates;     // per system [6][n]: the summed chunks
   DBuf<int> tile_count;   // per system and target tile; 0 between launches
-  // symmetric pair engine (sym): items in launch order, by phase; the slots are
-  // reused from phase to phase, each summed into the rates at its end
+  // symmetric pair engine (sym): items in launch order, by wave; the slots are
+  // reused from wave to wave, each summed into the rates at its end
   bool sym = false;
-  struct Phase {
+  struct Wave {
     int groups = 0, tiles = 0;  // items over groups, then over single tile pairs
     int sum0 = 0, sums = 0;     // its SymSum records
   };
-  std::vector<Phase> phases;
+  std::vector<Wave> waves;
   DBuf<SymItem> sym_items;
   DBuf<SymSeg> sym_segs;
   DBuf<int> sym_jbase;
   DBuf<SymSum> sym_sums;
-  DBuf<double> slots;
-  // the stage kernel sums the slots itself (one phase, not sharded): no
-  // launch for the sums, `rates` not used
+  std::shared_ptr<SlotPool> pool;
+  size_t slot_count = 0;  // doubles of the pool in use by a wave at most
+  // the stage kernel sums the slots itself (one wave, not sharded): no launch for
+  // the sums, no `rates`
   bool fused_sums = false;
   double slot_bytes = 0.0;  // bytes of all slots that one right-hand side sums
   bool sided = false;     // some items form one side's sums only
@@ -206,7 +217,9 @@ struct Plan {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   unsigned long long graph_kernels = 0;  // kernels one replay launches
+  const double *graph_slots = nullptr;   // where the slots were when it was captured
   ~Plan();
+  void drop_graph();
   bool stale() const;
 };
 
@@ -243,7 +256,7 @@ double sym_slot_bytes(size_t n, bool serving);
 
 int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int precision,
                const TileChoice &tile, std::unique_ptr<Plan> &out, int fixed_chunk_sources = 0,
-               bool ordered_alloc = false);
+               bool ordered_alloc = false, bool own_slots = false);
 // Whether n steps (dt[i], or dt0 for all when dt is null) are all valid.
 int check_dts(pawan_ctx *ctx, size_t n, const double *dt, double dt0);
 int set_plan_dt(pawan_ctx *ctx, Plan &p, const double *dt, double dt0);

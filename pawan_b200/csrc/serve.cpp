@@ -317,7 +317,7 @@ void worker_main(pawan_server *srv) {
     }
     for (Request *r : big) {
       if (st != PAWAN_OK || r->plan) continue;
-      st = build_plan(srv->ctx, {r->sys}, srv->cfg.precision, srv->tile, r->plan, kServeChunkSources, true);
+      st = build_plan(srv->ctx, {r->sys}, srv->cfg.precision, srv->tile, r->plan, kServeChunkSources, true, true);
       if (st == PAWAN_OK) st = set_plan_dt(srv->ctx, *r->plan, &r->dt, 0.0);
     }
     set_changed = false;

@@ -1,0 +1,99 @@
+"""Device memory of the symmetric engine's slots: bounded for a plan over many
+systems, which then runs in waves, and shared by the plans of a context."""
+import numpy as np
+import pytest
+import torch
+
+from pawan_b200 import Batch, Context, System
+from pawan_b200 import geometry as g
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def own():
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def used_bytes():
+    free, total = torch.cuda.mem_get_info()
+    return total - free
+
+
+def particles(n, seed):
+    sc = g.ring_pair(n_stations=-(-n // 16), seed=seed, nu=1e-3)
+    return [np.ascontiguousarray(a[:n]) for a in sc.union()]
+
+
+# 24 x 32,768 particles in single tiles, 10 x 131,072 in groups of tiles: 9.7 and
+# 10 GB of slots if they were all held at once
+@pytest.mark.parametrize("n,count,prec", [(32768, 24, "f64"), (131072, 10, "f32")])
+def test_a_batch_over_the_bound_runs_in_waves(own, n, count, prec):
+    sizes = [n] * count + [2000, 129]
+    arrays = [particles(k, 5) for k in (n, 2000, 129)]
+    alone = []
+    for a in arrays:
+        s = System(own, [len(a[0])], 1e-3, prec)
+        s.set_particles(*a)
+        s.solve()
+        alone.append(s.get_rates())
+        s.close()
+    systems = []
+    for k in sizes:
+        s = System(own, [k], 1e-3, prec)
+        s.set_particles(*arrays[[n, 2000, 129].index(k)])
+        systems.append(s)
+    before = used_bytes()
+    b = Batch(own, systems)
+    if prec == "f32":
+        b.set_config(128, unroll=4, packed=2, items_per_slot=32)  # the default, as the systems alone
+    b.solve()
+    # the slots' bound, and per particle the 48-byte rates, 24 of work tables and boxes
+    assert used_bytes() - before <= 8.0e9 + 100.0 * sum(sizes) + (64 << 20)
+    for k, s in zip(sizes, systems):
+        assert np.array_equal(s.get_rates(), alone[[n, 2000, 129].index(k)])
+    b.close()
+    for s in systems:
+        s.close()
+
+
+def test_systems_of_a_context_share_their_slots(own):
+    a = particles(32768, 6)
+    systems = []
+    before = 0
+    for k in range(8):
+        s = System(own, [32768], 1e-3, "f32")
+        s.set_particles(*a)
+        s.solve()
+        systems.append(s)
+        if k == 0:
+            before = used_bytes()
+    # 0.4 GB of slots each; their other arrays are some 20 MB
+    assert used_bytes() - before <= 7 * (64 << 20)
+    first = systems[0].get_rates()
+    for s in systems[::-1]:
+        s.solve()
+        assert np.array_equal(s.get_rates(), first)
+        s.close()
+    assert used_bytes() < before  # the last one gives the slots back
+
+
+def test_a_captured_step_follows_its_slots(own):
+    """Graph replays before and after a larger plan has moved the shared slots."""
+    def run(larger):
+        s = System(own, [3000], 1e-3, "f32")
+        s.set_particles(*particles(3000, 7))
+        s.rk4(0.005, 2, use_graph=True)
+        if larger:
+            t = System(own, [20000], 1e-3, "f32")
+            t.set_particles(*particles(20000, 8))
+            t.solve()
+        s.rk4(0.005, 2, use_graph=True)
+        out = s.get_states()
+        s.close()
+        if larger:
+            t.close()
+        return out
+    assert np.array_equal(run(False), run(True))
