@@ -705,10 +705,10 @@ int pawan_system_autotune(pawan_system *sys) {
   CHECK_SYS(sys);
   if (!sys->has_particles) return fail(sys->ctx, PAWAN_ERR_STATE, "particles not set");
   TileChoice best;
+  sys->plan.reset();  // (its buffers make room for the candidates')
   PAWAN_TRY(autotune_plan(sys->ctx, {sys}, sys->precision, &best));
   sys->tile = best;
   sys->fixed_tile = true;
-  sys->plan.reset();
   const double n2 = (double)sys->n * (double)sys->n;
   sys->ctx->tune_cache[std::make_tuple(sys->precision, sys->nu != 0.0 ? 1 : 0,
                                        (int)std::log2(std::max(1.0, n2)), 0)] = best;
@@ -874,11 +874,11 @@ int pawan_batch_autotune(pawan_batch *b) {
   for (auto *s : b->systems)
     if (!s->has_particles) return fail(b->ctx, PAWAN_ERR_STATE, "a batch system has no particles");
   TileChoice best;
+  b->plans.clear();  // (their buffers make room for the candidates')
+  b->members.clear();
   PAWAN_TRY(autotune_plan(b->ctx, b->systems, b->precision, &best));
   b->tile = best;
   b->tuned = true;
-  b->plans.clear();
-  b->members.clear();
   return batch_ensure_plan(b);
 }
 

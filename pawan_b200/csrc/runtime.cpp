@@ -254,15 +254,11 @@ static int reserve_slots(pawan_ctx *ctx, SlotPool &pool, size_t count) {
   if (pool.buf.ordered) larger.ordered_on(pool.buf.stream);
   cudaError_t e = larger.alloc(count);
   if (e == cudaErrorMemoryAllocation && pool.buf.p) {
-    cudaGetLastError();
     pool.buf.reset();
     if (pool.buf.ordered) cudaStreamSynchronize(pool.buf.stream);
     e = larger.alloc(count);
   }
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return cuda_fail(ctx, e, "pair-sum slots");
-  }
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "pair-sum slots");
   std::swap(pool.buf.p, larger.p);
   std::swap(pool.buf.n, larger.n);
   return PAWAN_OK;
@@ -889,6 +885,19 @@ int autotune_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, in
     *ms = f / reps;
     return PAWAN_OK;
   };
+  // A tiling whose buffers do not fit beside what the device holds is no candidate.
+  bool any = false;
+  auto candidate = [&](const TileChoice &t) -> int {
+    double ms = 0;
+    const int st = time_tile(t, &ms);
+    if (st != PAWAN_OK) return st;
+    any = true;
+    if (ms < best_ms) {
+      best_ms = ms;
+      best_t = t;
+    }
+    return PAWAN_OK;
+  };
   // 1) tile shape at the default chunking, 2) chunking for the best shape.
   bool sym_timed = false;
   for (TileChoice t : tile_candidates(precision, systems[0]->kernel)) {
@@ -898,26 +907,18 @@ int autotune_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, in
       sym_timed = true;
       t.pc = default_tile(precision).pc;
     }
-    double ms = 0;
-    status = time_tile(t, &ms);
-    if (status != PAWAN_OK) break;
-    if (ms < best_ms) {
-      best_ms = ms;
-      best_t = t;
-    }
+    status = candidate(t);
+    if (status != PAWAN_OK && status != PAWAN_ERR_NOMEM) break;
   }
-  if (status == PAWAN_OK) {
+  if (any && (status == PAWAN_OK || status == PAWAN_ERR_NOMEM)) {
+    const TileChoice shape = best_t;
     for (int ips : kTuneItemsPerSlot) {
-      TileChoice t = best_t;
+      TileChoice t = shape;
       t.items_per_slot = ips;
-      double ms = 0;
-      status = time_tile(t, &ms);
-      if (status != PAWAN_OK) break;
-      if (ms < best_ms) {
-        best_ms = ms;
-        best_t = t;
-      }
+      status = candidate(t);
+      if (status != PAWAN_OK && status != PAWAN_ERR_NOMEM) break;
     }
+    if (status == PAWAN_ERR_NOMEM) status = PAWAN_OK;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);

@@ -43,6 +43,7 @@ struct DBuf {
                             : cudaMalloc(reinterpret_cast<void **>(&p), count * sizeof(T));
     if (e != cudaSuccess) {
       p = nullptr;
+      cudaGetLastError();  // (the next launch's check is not to find it)
       return e;
     }
     n = count;

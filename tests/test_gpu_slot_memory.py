@@ -6,6 +6,7 @@ import torch
 
 from pawan_b200 import Batch, Context, System
 from pawan_b200 import geometry as g
+from helpers import TOL_F32_RMS, rms_rel
 
 pytestmark = pytest.mark.gpu
 
@@ -97,3 +98,33 @@ def test_a_captured_step_follows_its_slots(own):
             t.close()
         return out
     assert np.array_equal(run(False), run(True))
+
+
+@pytest.mark.parametrize("batched", [False, True])
+def test_autotune_passes_over_what_does_not_fit(own, batched):
+    """128 MB left on the device: the symmetric engine's slots (403 MB) do not fit,
+    a one-sided tiling's partial sums do."""
+    a = particles(32768, 9)
+    s = System(own, [32768], 1e-3, "f32")
+    s.set_config(128, unroll=4, items_per_slot=4)  # one-sided
+    s.set_particles(*a)
+    s.solve()
+    want = s.get_rates()
+    b = Batch(own, [s])
+    b.set_config(128, unroll=4, items_per_slot=4)
+    b.solve()
+    torch.cuda.empty_cache()
+    filler = []
+    while torch.cuda.mem_get_info()[0] > (160 << 20):
+        filler.append(torch.empty(torch.cuda.mem_get_info()[0] - (128 << 20) >> 21 << 21, dtype=torch.uint8,
+                                  device="cuda"))
+    try:
+        (b if batched else s).autotune()
+        (b if batched else s).solve()
+        got = s.get_rates()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert rms_rel(got, want) <= TOL_F32_RMS
+    b.close()
+    s.close()
