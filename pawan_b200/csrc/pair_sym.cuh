@@ -92,7 +92,7 @@ __device__ __forceinline__ void tile_item(const SymItem *__restrict__ items, con
   const int jb = it.b0 > it.a ? jbase[it.jb + it.b0] : -1;
   if (jb >= 0) {
     // this thread's own source
-    double *out = slots + ((size_t)jb + it.a) * 6 * kT;
+    double *out = slots + ((size_t)jb + it.a - it.row0) * 6 * kT;
 #pragma unroll
     for (int k = 0; k < 6; ++k) out[k * kT + tid] = accJ[k * kT + tid];
   }
@@ -147,7 +147,7 @@ __device__ __forceinline__ void spread_item(const SymItem *__restrict__ items, c
   if (jb >= 0) {
     // thread: one of the block's 32 kSubs sources, three of its six sums
     const int at = 3 * (tid / (32 * kSubs)) * kT + 32 * kSubs * rank + tid % (32 * kSubs);
-    double *out = slots + ((size_t)jb + it.a) * kC;
+    double *out = slots + ((size_t)jb + it.a - it.row0) * kC;
 #pragma unroll
     for (int u = 0; u < 3; ++u) out[at + u * kT] = accJ[at + u * kT] + accJ[kC + at + u * kT];
   }

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from pawan_b200 import Batch, Context, System
+from pawan_b200 import Batch, Context, Server, System
 from pawan_b200 import geometry as g
 from helpers import TOL_F32_RMS, rms_rel
 
@@ -128,3 +128,19 @@ def test_autotune_passes_over_what_does_not_fit(own, batched):
     assert rms_rel(got, want) <= TOL_F32_RMS
     b.close()
     s.close()
+
+
+def test_a_served_request_in_phases_of_single_tiles(own):
+    """32,768 particles: 403 MB of slots, above the serving engine's bound, in two
+    phases."""
+    sc = g.ring_pair(n_stations=2048, seed=11, nu=1e-3, steps=1)
+    srv = Server(own, budget_bytes=8 << 30)
+    rid = srv.submit_scenario(sc)[1]
+    assert srv.wait(rid, 120)
+    out = srv.fetch(rid)[0]
+    srv.close()
+    solo = System.from_scenario(own, sc, "f32")
+    solo.rk4(sc.dt, sc.steps)
+    st0 = sc.state()
+    assert rms_rel(out - st0, solo.get_states() - st0) < 1e-12
+    solo.close()
