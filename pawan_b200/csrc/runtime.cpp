@@ -212,13 +212,13 @@ struct SymWaves {
   };
   std::vector<SymLayout> lay;
   std::vector<std::vector<Unit>> waves;  // systems with the most tiles first
+  double bytes = 0.0;                    // of the largest wave's slots
 };
 
-SymWaves sym_waves(const Plan &p, bool serving) {
+SymWaves sym_waves(const Plan &p, double system_bytes, double plan_bytes) {
   SymWaves w;
   for (auto *y : p.systems)
-    w.lay.push_back(sym_layout(y->n, p.tile.items_per_slot, serving ? kSymSlotBytesServing : kSymSlotBytes,
-                               y->shard.active ? y->shard.world : 1));
+    w.lay.push_back(sym_layout(y->n, p.tile.items_per_slot, system_bytes, y->shard.active ? y->shard.world : 1));
   std::vector<size_t> order(p.systems.size());
   std::iota(order.begin(), order.end(), (size_t)0);
   std::stable_sort(order.begin(), order.end(),
@@ -232,12 +232,13 @@ SymWaves sym_waves(const Plan &p, bool serving) {
       for (int t = 0; t < l.ng; ++t)
         if (sym_owned(p.systems[s], l, t)) need += l.slots(t, l.rows[ph], l.rows[ph + 1]);
       need *= 48.0 * kSymTile * l.g;
-      while (k < used.size() && used[k] > 0.0 && used[k] + need > kPlanSlotBytes) ++k;
+      while (k < used.size() && used[k] > 0.0 && used[k] + need > plan_bytes) ++k;
       if (k == used.size()) {
         used.push_back(0.0);
         w.waves.emplace_back();
       }
       used[k] += need;
+      w.bytes = std::max(w.bytes, used[k]);
       w.waves[k].push_back({s, (int)ph});
     }
   }
@@ -254,9 +255,11 @@ static int reserve_slots(pawan_ctx *ctx, SlotPool &pool, size_t count) {
   if (pool.buf.ordered) larger.ordered_on(pool.buf.stream);
   cudaError_t e = larger.alloc(count);
   if (e == cudaErrorMemoryAllocation && pool.buf.p) {
+    const size_t had = pool.buf.n;
     pool.buf.reset();
     if (pool.buf.ordered) cudaStreamSynchronize(pool.buf.stream);
     e = larger.alloc(count);
+    if (e != cudaSuccess) pool.buf.alloc(had);  // the other plans' (at worst at their next launch)
   }
   if (e != cudaSuccess) return cuda_fail(ctx, e, "pair-sum slots");
   std::swap(pool.buf.p, larger.p);
@@ -275,9 +278,7 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, const SymWaves &w) {
   std::vector<SymItem> items;
   std::vector<SymSum> sums;
   std::vector<int> jbase;
-  size_t group_slots = 0, tile_slots = 0;  // most doubles of any wave
   const size_t n_waves = w.waves.size();
-  std::vector<std::vector<SymSum>> tile_sums(n_waves);
   p.waves.assign(n_waves, Plan::Wave{});
   for (size_t k = 0; k < n_waves; ++k) {
     Plan::Wave &P = p.waves[k];
@@ -350,18 +351,13 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, const SymWaves &w) {
         items.push_back(c.w);
         p.item_costs.push_back(c.cost);
       }
-    group_slots = std::max(group_slots, used[1] * 6 * kSymTile * kSymGroup);
-    tile_slots = std::max(tile_slots, used[0] * 6 * kSymTile);
-    tile_sums[k] = of_tiles;
+    // the single-tile items' slots lie behind the groups'
+    P.tile_slots = used[1] * 6 * kSymTile * kSymGroup;
+    for (SymSum &t : of_tiles) t.first += (long long)P.tile_slots;
     sums.insert(sums.end(), of_tiles.begin(), of_tiles.end());
     P.sums = (int)sums.size() - P.sum0;
+    p.slot_count = std::max(p.slot_count, P.tile_slots + used[0] * 6 * kSymTile);
   }
-  // the single-tile items' slots lie behind the groups'
-  for (size_t k = 0; k < n_waves; ++k) {
-    const size_t c = tile_sums[k].size(), at = (size_t)(p.waves[k].sum0 + p.waves[k].sums) - c;
-    for (size_t q = 0; q < c; ++q) sums[at + q].first += (long long)group_slots;
-  }
-  p.tile_slots = group_slots;
   for (const SymSum &s : sums) p.slot_bytes += (double)s.count * 48.0 * kSymTile;
   if (items.size() > (size_t)INT32_MAX) return fail(ctx, PAWAN_ERR_INVALID, "too many work items");
   p.n_items = (int)items.size();
@@ -372,7 +368,6 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, const SymWaves &w) {
     segs.push_back(SymSeg{g.pos32, g.vor32, g.poslo, g.vorlo, g.pos64, g.vor64, g.boxes,
                           (int)y->n, y->nu, (float)(y->r_near * y->r_near)});
   }
-  p.slot_count = group_slots + tile_slots;
   PAWAN_TRY(reserve_slots(ctx, *p.pool, p.slot_count));
   PAWAN_CUDA(ctx, p.sym_items.alloc(items.size()));
   PAWAN_CUDA(ctx, p.sym_segs.alloc(segs.size()));
@@ -427,16 +422,28 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
                                                 : sym_f32_occupancy(p->diffusion, kernel, &bps);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy query");
     if (bps < 1) return fail(ctx, PAWAN_ERR_INVALID, "pair kernel does not fit on an SM");
-    waves = sym_waves(*p, fixed_chunk_sources > 0);
-    p->fused_sums = waves.waves.size() == 1;
-    for (auto *s : systems)
-      if (s->shard.active) p->fused_sums = false;
     if (!own_slots) p->pool = ctx->slots.lock();
     if (!p->pool) {
       p->pool = std::make_shared<SlotPool>();
       if (ordered_alloc) p->pool->buf.ordered_on(ctx->stream);
       if (!own_slots) ctx->slots = p->pool;
     }
+    // Where the device has no room for the slots, in more and smaller phases and
+    // waves, down to one row of tiles at a time.
+    double share = 1.0, before = -1.0;
+    for (;;) {
+      waves = sym_waves(*p, share * (fixed_chunk_sources > 0 ? kSymSlotBytesServing : kSymSlotBytes),
+                        share * kPlanSlotBytes);
+      const int st = waves.bytes == before ? PAWAN_ERR_NOMEM
+                                           : reserve_slots(ctx, *p->pool, (size_t)(waves.bytes / sizeof(double)));
+      if (st == PAWAN_OK) break;
+      if (st != PAWAN_ERR_NOMEM || share < 1e-4) return st;
+      before = waves.bytes;
+      share *= 0.25;
+    }
+    p->fused_sums = waves.waves.size() == 1;
+    for (auto *s : systems)
+      if (s->shard.active) p->fused_sums = false;
   } else {
     PAWAN_TRY(occupancy(ctx, precision, tile.pc, p->diffusion, kernel, &bps));
   }
@@ -671,7 +678,7 @@ static int launch_sym_range(pawan_ctx *ctx, Plan &p, int first, int count) {
       const int lo = std::max(first, at), hi = std::min(first + count, at + n);
       at += n;
       if (lo >= hi) continue;
-      double *slots = p.pool->buf.p + (group ? 0 : p.tile_slots);
+      double *slots = p.pool->buf.p + (group ? 0 : ph.tile_slots);
       const auto launch = p.precision == PAWAN_PREC_F64 ? launch_sym_f64 : launch_sym_f32;
       PAWAN_CUDA(ctx, launch(group, p.sided, p.diffusion, p.kernel, p.sym_items.p + lo, hi - lo, ctx->sm_count,
                              p.sym_segs.p, p.sym_jbase.p, slots, ctx->stream));

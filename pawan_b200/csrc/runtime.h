@@ -192,6 +192,7 @@ struct Plan {
   struct Wave {
     int groups = 0, tiles = 0;  // items over groups, then over single tile pairs
     int sum0 = 0, sums = 0;     // its SymSum records
+    size_t tile_slots = 0;      // doubles before the slots of the single-tile items
   };
   std::vector<Wave> waves;
   DBuf<SymItem> sym_items;
@@ -205,7 +206,6 @@ struct Plan {
   bool fused_sums = false;
   double slot_bytes = 0.0;  // bytes of all slots that one right-hand side sums
   bool sided = false;     // some items form one side's sums only
-  size_t tile_slots = 0;  // doubles before the slots of the single-tile items
   DBuf<float4> boxes;
   DBuf<WorkItem> items;
   DBuf<SegDesc> segs;

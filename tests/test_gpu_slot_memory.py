@@ -100,6 +100,36 @@ def test_a_captured_step_follows_its_slots(own):
     assert np.array_equal(run(False), run(True))
 
 
+def filled(leave):
+    """Takes all device memory but about `leave` bytes."""
+    torch.cuda.empty_cache()
+    filler = []
+    while torch.cuda.mem_get_info()[0] > leave + (32 << 20):
+        filler.append(torch.empty(torch.cuda.mem_get_info()[0] - leave >> 21 << 21, dtype=torch.uint8, device="cuda"))
+    return filler
+
+
+@pytest.mark.parametrize("n,prec", [(32768, "f32"), (32768, "f64"), (65536, "f32")])
+def test_a_full_device_takes_smaller_phases(own, n, prec):
+    """128 MB left on the device: the slots (403 MB) in phases of as many rows as fit."""
+    a = particles(n, 10)
+    rates = []
+    for full in (False, True):
+        s = System(own, [n], 1e-3, prec)
+        filler = filled(128 << 20) if full else []
+        try:
+            s.set_particles(*a)
+            s.rk4(0.005, 1, use_graph=True)
+            s.set_states(np.concatenate([a[0].ravel(), a[1].ravel()]))
+            s.solve()
+            rates.append(s.get_rates())
+        finally:
+            del filler
+            torch.cuda.empty_cache()
+            s.close()
+    assert rms_rel(rates[1], rates[0]) < 1e-12  # (the grouping of the FP64 sums)
+
+
 @pytest.mark.parametrize("batched", [False, True])
 def test_autotune_passes_over_what_does_not_fit(own, batched):
     """128 MB left on the device: the symmetric engine's slots (403 MB) do not fit,
@@ -113,11 +143,7 @@ def test_autotune_passes_over_what_does_not_fit(own, batched):
     b = Batch(own, [s])
     b.set_config(128, unroll=4, items_per_slot=4)
     b.solve()
-    torch.cuda.empty_cache()
-    filler = []
-    while torch.cuda.mem_get_info()[0] > (160 << 20):
-        filler.append(torch.empty(torch.cuda.mem_get_info()[0] - (128 << 20) >> 21 << 21, dtype=torch.uint8,
-                                  device="cuda"))
+    filler = filled(128 << 20)
     try:
         (b if batched else s).autotune()
         (b if batched else s).solve()
