@@ -128,9 +128,8 @@ static size_t shard_count(const pawan_system *y) {
 constexpr int kSymTilesMax = 256;
 // Bound on one system's slots: the rows of groups (or tiles) are processed in
 // phases, the slots of a phase summed into the rates before the next reuses them.
-// The serving engine holds many systems at a time, so its bound is smaller.  (One
-// row's slots are the least: 6 KB per 128 particles, and as much again.)
-constexpr double kSymSlotBytes = 2.0e9, kSymSlotBytesServing = 4.0e8;
+// (One row's slots are the least: 6 KB per 128 particles, and as much again.)
+constexpr double kSymSlotBytes = 2.0e9;
 // Bound on the slots of all systems of a plan (or one phase of one of them): plans
 // over more run in waves that reuse them.  512 ragged rings of 512 to 16,384
 // particles hold 7.4e9 bytes in one wave.
@@ -182,8 +181,8 @@ SymLayout sym_layout(size_t n, int items_per_slot, double bytes, int world = 1) 
 
 }  // namespace
 
-double sym_slot_bytes(size_t n, bool serving) {
-  const SymLayout l = sym_layout(n, 32, serving ? kSymSlotBytesServing : kSymSlotBytes);
+double sym_slot_bytes(size_t n, double bytes) {
+  const SymLayout l = sym_layout(n, 32, bytes);
   double most = 0.0;
   for (size_t p = 0; p + 1 < l.rows.size(); ++p) {
     double c = 0.0;
@@ -393,7 +392,7 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, const SymWaves &w) {
 // target tile's chunks are consecutive.
 int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int precision,
                const TileChoice &tile, std::unique_ptr<Plan> &out, int fixed_chunk_sources,
-               bool ordered_alloc, bool own_slots) {
+               const PlanMemory &memory) {
   if (systems.empty()) return fail(ctx, PAWAN_ERR_INVALID, "plan over no systems");
   const int kernel = systems[0]->kernel;
   for (auto *s : systems)
@@ -422,18 +421,18 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
                                                 : sym_f32_occupancy(p->diffusion, kernel, &bps);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "occupancy query");
     if (bps < 1) return fail(ctx, PAWAN_ERR_INVALID, "pair kernel does not fit on an SM");
-    if (!own_slots) p->pool = ctx->slots.lock();
+    if (!memory.own_slots) p->pool = ctx->slots.lock();
     if (!p->pool) {
       p->pool = std::make_shared<SlotPool>();
-      if (ordered_alloc) p->pool->buf.ordered_on(ctx->stream);
-      if (!own_slots) ctx->slots = p->pool;
+      if (memory.ordered) p->pool->buf.ordered_on(ctx->stream);
+      if (!memory.own_slots) ctx->slots = p->pool;
     }
     // Where the device has no room for the slots, in more and smaller phases and
     // waves, down to one row of tiles at a time.
     double share = 1.0, before = -1.0;
     for (;;) {
-      waves = sym_waves(*p, share * (fixed_chunk_sources > 0 ? kSymSlotBytesServing : kSymSlotBytes),
-                        share * kPlanSlotBytes);
+      waves = sym_waves(*p, share * (memory.system_bytes > 0.0 ? memory.system_bytes : kSymSlotBytes),
+                        share * (memory.plan_bytes > 0.0 ? memory.plan_bytes : kPlanSlotBytes));
       const int st = waves.bytes == before ? PAWAN_ERR_NOMEM
                                            : reserve_slots(ctx, *p->pool, (size_t)(waves.bytes / sizeof(double)));
       if (st == PAWAN_OK) break;
@@ -513,7 +512,7 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
   if (items.size() > (size_t)INT32_MAX) return fail(ctx, PAWAN_ERR_INVALID, "too many work items");
   p->n_items = (int)items.size();
 
-  if (ordered_alloc) {
+  if (memory.ordered) {
     p->partial.ordered_on(ctx->stream);
     p->rates.ordered_on(ctx->stream);
     p->tile_count.ordered_on(ctx->stream);
@@ -625,7 +624,7 @@ int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int p
   PAWAN_TRY(launch_stage_mode(ctx, *out, STAGE_PACK));
   // (the host tables were staged by the copies above; an ordered plan is used
   // on the same stream, so only the others wait here)
-  if (!ordered_alloc) PAWAN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if (!memory.ordered) PAWAN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return PAWAN_OK;
 }
 

@@ -252,12 +252,21 @@ bool tile_supported(int precision, const PairConfig &pc, int kernel);
 // Whether a precision and tiling run on the symmetric pair engine (each
 // unordered pair once): the packed FP32 tilings and FP64.
 bool tile_symmetric(int precision, const PairConfig &pc);
-// Device bytes of the symmetric engine's slots for one system of n particles.
-double sym_slot_bytes(size_t n, bool serving);
+// Device bytes of the symmetric engine's slots for one system of n particles, in
+// phases of at most `bytes` (or one row of tiles).
+double sym_slot_bytes(size_t n, double bytes);
+
+// Where a plan's memory comes from and how much its slots may take.
+struct PlanMemory {
+  bool ordered = false;       // from the memory pool, in the order of the stream
+  bool own_slots = false;     // slots of its own: stages are split over calls
+  double system_bytes = 0.0;  // bounds on the slots of one system and of all (0: the defaults)
+  double plan_bytes = 0.0;
+};
 
 int build_plan(pawan_ctx *ctx, const std::vector<pawan_system *> &systems, int precision,
                const TileChoice &tile, std::unique_ptr<Plan> &out, int fixed_chunk_sources = 0,
-               bool ordered_alloc = false, bool own_slots = false);
+               const PlanMemory &memory = {});
 // Whether n steps (dt[i], or dt0 for all when dt is null) are all valid.
 int check_dts(pawan_ctx *ctx, size_t n, const double *dt, double dt0);
 int set_plan_dt(pawan_ctx *ctx, Plan &p, const double *dt, double dt0);

@@ -33,6 +33,14 @@
 // device, and a request's particles are packed by the batched plan built
 // after its admission instead of a plan of its own.
 //
+// Memory.  A request holds its system's arrays and rates, some 440 bytes per
+// particle.  Slots: those that step together share the engine's buffer (an eighth
+// of the budget at most; larger sets run in waves), a large one has its own.  A
+// request whose slots do not fit beside its arrays runs on a plan of its own with
+// less: in FP32 the one-sided kernel's partial sums, in FP64 shorter phases.  What
+// is charged decides how many requests are admitted at a time; one that fits alone
+// is always accepted.
+//
 // A request's work is decomposed by its own size alone (and, on the one-sided
 // kernels, its sources chunked in chunks of a fixed size), so its arithmetic
 // does not depend on which other requests share its launches: its result is
@@ -74,31 +82,43 @@ struct Request {
   double nu = 0.0, dt = 0.0;
   size_t nsteps = 0, steps_done = 0;
   size_t n = 0;
-  double bytes = 0.0;
+  double bytes = 0.0;       // arrays and rates
+  double slots = 0.0;       // slots (or partial sums) of this request
+  bool spare = false;       // its slots would not fit: a plan of its own, with less
   double t_submit = 0.0, t_admit = -1.0, t_done = -1.0;
   bool cancel = false;
   pawan_system *sys = nullptr;
-  // a request whose RK4 step costs more than an iteration ("large"): its own
-  // plan, and the stage / work item it has reached
+  // a request with its own plan, and the stage / work item it has reached: one
+  // whose RK4 step costs more than an iteration ("large"), or a spare one
   bool large = false;
   std::unique_ptr<Plan> plan;
   int stage = 0, next_item = 0;
   std::vector<double> result;
 };
 
-// Device bytes a request holds while active: the system's buffers plus its
-// rates and slots in a batched plan (the symmetric engine's, or partial slots
-// of a fixed chunk size that cover whole target tiles of at most 512 particles).
-double request_bytes(size_t n, int precision, const TileChoice &tile) {
+// Device bytes a request holds while active: the system's buffers and its rates.
+double request_bytes(size_t n) {
   const double per = 5 * 48.0 + 16.0 + 4.0 + 64.0 + 64.0 + 1.0 + 48.0;
-  if (tile_symmetric(precision, tile.pc))
-    return (double)n * per + sym_slot_bytes(n, true) + 4096.0;
+  return (double)n * per + 4096.0;
+}
+
+// Partial slots of the one-sided kernels: chunks of a fixed size that cover whole
+// target tiles of at most 512 particles.
+double partial_bytes(size_t n, const TileChoice &tile) {
   const int tb = tile.pc.tb;
   const size_t chunk = ((kServeChunkSources + tb - 1) / tb) * (size_t)tb;
   const size_t nch = (n + chunk - 1) / chunk;
-  const double slots = nch > 1 ? 48.0 * (double)(n + 512) * (double)nch : 0.0;
-  return (double)n * per + slots + 4096.0;
+  return nch > 1 ? 48.0 * (double)(n + 512) * (double)nch : 0.0;
 }
+
+// Bounds on the slots of a batched plan and of one request (which shape a
+// request's decomposition, so they depend on the configuration alone): an eighth
+// of the budget, at most 500 MB and 400 MB.
+double plan_slot_bytes(const pawan_serve_config &cfg) {
+  return std::min(5.0e8, std::max(cfg.budget_bytes / 8.0, 4.0e6));
+}
+
+double system_slot_bytes(const pawan_serve_config &cfg) { return std::min(4.0e8, plan_slot_bytes(cfg)); }
 
 // The engine's tiling: for FP32 one that the symmetric pair engine runs; the
 // library default otherwise.
@@ -142,6 +162,55 @@ bool take(int &pending) {
   return true;
 }
 
+// The tiling and the memory of a spare request's plan.
+TileChoice spare_tile(const pawan_server *srv) {
+  TileChoice t = srv->tile;
+  if (srv->cfg.precision == PAWAN_PREC_F32) {
+    t.pc = PairConfig{128, 1, 4, 1, 0, 2};
+    t.pc.onesided = true;
+  }
+  return t;
+}
+
+double spare_slot_bytes(const pawan_server *srv, double request) {
+  return std::max(1.0, std::min(system_slot_bytes(srv->cfg), srv->cfg.budget_bytes - request));
+}
+
+// What a request takes, by itself: fills in bytes, slots and spare.
+void size_request(const pawan_server *srv, Request *r) {
+  const int precision = srv->cfg.precision;
+  const double budget = srv->cfg.budget_bytes;
+  r->bytes = request_bytes(r->n);
+  if (!tile_symmetric(precision, srv->tile.pc)) {
+    r->slots = partial_bytes(r->n, srv->tile);
+    return;
+  }
+  r->slots = sym_slot_bytes(r->n, system_slot_bytes(srv->cfg));
+  if (r->bytes + r->slots <= budget) return;
+  r->spare = true;
+  // (FP64 in the shortest phases may take more than a one-sided kernel's partial
+  // sums; it is charged those, and accepted where they fit)
+  const double partial = partial_bytes(r->n, srv->tile);
+  r->slots = precision == PAWAN_PREC_F32
+                 ? partial
+                 : std::min(sym_slot_bytes(r->n, spare_slot_bytes(srv, r->bytes)), partial);
+}
+
+// Device bytes of requests active together.
+double bytes_of(const pawan_server *srv, const std::vector<Request *> &a, const std::vector<Request *> &b = {},
+                const Request *c = nullptr) {
+  double total = 0.0, shared = 0.0;
+  auto add = [&](const Request *r) {
+    total += r->bytes;
+    (r->large || r->spare ? total : shared) += r->slots;
+  };
+  for (const Request *r : a) add(r);
+  for (const Request *r : b) add(r);
+  if (c) add(c);
+  if (tile_symmetric(srv->cfg.precision, srv->tile.pc)) shared = std::min(shared, plan_slot_bytes(srv->cfg));
+  return total + shared;
+}
+
 void finish(pawan_server *srv, Request *r, int state) {
   r->state = state;
   r->t_done = now_since(srv->t0);
@@ -156,7 +225,11 @@ int plan_iteration(pawan_server *srv, std::vector<Request *> &act, std::unique_p
     plan.reset();
     std::vector<pawan_system *> sys;
     for (Request *r : act) sys.push_back(r->sys);
-    int st = build_plan(ctx, sys, srv->cfg.precision, srv->tile, plan, kServeChunkSources, true);
+    PlanMemory memory;
+    memory.ordered = true;
+    memory.system_bytes = system_slot_bytes(srv->cfg);
+    memory.plan_bytes = plan_slot_bytes(srv->cfg);
+    int st = build_plan(ctx, sys, srv->cfg.precision, srv->tile, plan, kServeChunkSources, memory);
     if (st != PAWAN_OK) return st;
   }
   std::vector<double> dts;
@@ -244,15 +317,17 @@ void worker_main(pawan_server *srv) {
         for (Request *a : srv->active) n2 += (double)a->n * (double)a->n;
         for (Request *a : admit) n2 += (double)a->n * (double)a->n;
         const bool empty = na == 0;
-        if (srv->bytes_in_use + r->bytes > srv->cfg.budget_bytes) break;
+        const double target = srv->cfg.iteration_seconds > 0.0 ? srv->cfg.iteration_seconds : kIterTarget;
+        r->large = 4.0 * (double)r->n * (double)r->n / std::max(1e9, srv->rate) > target;
+        if (!empty && bytes_of(srv, srv->active, admit, r) > srv->cfg.budget_bytes) break;
         if (srv->cfg.max_active > 0 && (int)na >= srv->cfg.max_active) break;
         if (srv->cfg.max_step_interactions > 0 && n2 > srv->cfg.max_step_interactions && !empty)
           break;
         srv->queue.pop_front();
-        srv->bytes_in_use += r->bytes;
         r->state = PAWAN_REQ_ACTIVE;
         r->t_admit = now_since(srv->t0);
         admit.push_back(r);
+        srv->bytes_in_use = bytes_of(srv, srv->active, admit);
       }
       if (srv->active.empty() && admit.empty()) {
         if (srv->stop) break;
@@ -279,7 +354,6 @@ void worker_main(pawan_server *srv) {
         srv->worker_error = srv->ctx->err;
         if (r->sys) pawan_system_destroy(r->sys);
         r->sys = nullptr;
-        srv->bytes_in_use -= r->bytes;
         finish(srv, r, PAWAN_REQ_REJECTED);
         srv->stats.rejected++;
         srv->cv_done.notify_all();
@@ -288,14 +362,13 @@ void worker_main(pawan_server *srv) {
       // (the pageable particle copies were staged before system_upload returned)
       std::vector<double>().swap(r->pos);
       std::vector<double>().swap(r->vor);
-      const double target = srv->cfg.iteration_seconds > 0.0 ? srv->cfg.iteration_seconds : kIterTarget;
-      r->large = 4.0 * (double)r->n * (double)r->n / std::max(1e9, srv->rate) > target;
       srv->active.push_back(r);
       srv->stats.admitted++;
       set_changed = true;
     }
     if (!admit.empty()) {
       std::lock_guard<std::mutex> lk(srv->mu);
+      srv->bytes_in_use = bytes_of(srv, srv->active);
       srv->stats.admit_seconds +=
           std::chrono::duration<double>(std::chrono::steady_clock::now() - ta0).count();
     }
@@ -307,7 +380,7 @@ void worker_main(pawan_server *srv) {
     if (act.empty()) continue;
     // requests that step together, and large ones that advance by slices
     std::vector<Request *> reg, big;
-    for (Request *r : act) (r->large ? big : reg).push_back(r);
+    for (Request *r : act) (r->large || r->spare ? big : reg).push_back(r);
     const auto tp0 = std::chrono::steady_clock::now();
     int st = PAWAN_OK;
     if (!reg.empty()) {
@@ -317,7 +390,12 @@ void worker_main(pawan_server *srv) {
     }
     for (Request *r : big) {
       if (st != PAWAN_OK || r->plan) continue;
-      st = build_plan(srv->ctx, {r->sys}, srv->cfg.precision, srv->tile, r->plan, kServeChunkSources, true, true);
+      PlanMemory memory;
+      memory.ordered = memory.own_slots = true;
+      memory.system_bytes = memory.plan_bytes =
+          r->spare ? spare_slot_bytes(srv, r->bytes) : system_slot_bytes(srv->cfg);
+      st = build_plan(srv->ctx, {r->sys}, srv->cfg.precision, r->spare ? spare_tile(srv) : srv->tile, r->plan,
+                      kServeChunkSources, memory);
       if (st == PAWAN_OK) st = set_plan_dt(srv->ctx, *r->plan, &r->dt, 0.0);
     }
     set_changed = false;
@@ -396,7 +474,7 @@ void worker_main(pawan_server *srv) {
       r->sys = nullptr;
       std::lock_guard<std::mutex> lk(srv->mu);
       srv->active.erase(std::find(srv->active.begin(), srv->active.end(), r));
-      srv->bytes_in_use -= r->bytes;
+      srv->bytes_in_use = bytes_of(srv, srv->active);
       finish(srv, r, state);
       if (state == PAWAN_REQ_DONE) srv->stats.completed++;
       else if (state == PAWAN_REQ_REJECTED) srv->stats.rejected++;
@@ -503,7 +581,7 @@ int pawan_server_submit(pawan_server *srv, size_t n_wakes, const size_t *num_par
   r->nu = nu;
   r->dt = dt;
   r->nsteps = nsteps;
-  r->bytes = request_bytes(n, srv->cfg.precision, srv->tile);
+  size_request(srv, r.get());
   std::lock_guard<std::mutex> lk(srv->mu);
   r->id = srv->next_id++;
   r->t_submit = now_since(srv->t0);
@@ -515,7 +593,7 @@ int pawan_server_submit(pawan_server *srv, size_t n_wakes, const size_t *num_par
     srv->reqs[r->id] = std::move(r);
     return PAWAN_ERR_REJECTED;
   }
-  if (r->bytes > srv->cfg.budget_bytes) {
+  if (r->bytes + r->slots > srv->cfg.budget_bytes) {
     finish(srv, r.get(), PAWAN_REQ_REJECTED);
     srv->stats.rejected++;
     srv->reqs[r->id] = std::move(r);
