@@ -31,7 +31,10 @@
 // memory pool in the order of the engine's stream (cudaMallocAsync /
 // cudaFreeAsync): admitting and retiring requests never synchronises the
 // device, and a request's particles are packed by the batched plan built
-// after its admission instead of a plan of its own.
+// after its admission instead of a plan of its own.  The slots of the batched
+// plans are one buffer that the engine takes at its creation and keeps: taken and
+// freed with every change of the active set, they cost pauses of 0.1 to 0.5 s now
+// and then (the 99th percentile of a run's latencies 0.03 to 2.4 s).
 //
 // Memory.  A request holds its system's arrays and rates, some 440 bytes per
 // particle.  Slots: those that step together share the engine's buffer (an eighth
@@ -148,6 +151,7 @@ struct pawan_server {
   TileChoice tile;
   double rate = kRateGuess;  // measured interactions/s of the iterations (worker only)
   cudaMemPool_t pool = nullptr;
+  std::shared_ptr<SlotPool> slots;  // of the batched plans, kept between them
   // host-side fault injection (pawan_server_inject), under `mu`
   int fail_alloc = 0, fail_iteration = 0, slow_iterations = 0;
   double slow_seconds = 0.0;
@@ -528,6 +532,15 @@ int pawan_server_create(pawan_ctx *ctx, const pawan_serve_config *cfg, pawan_ser
   } else {
     srv->pool = nullptr;
   }
+  srv->slots = std::make_shared<SlotPool>();
+  srv->slots->buf.ordered_on(srv->ctx->stream);
+  srv->ctx->slots = srv->slots;
+  // taken now, as an allocation of this size may take 0.2 s, where it is a small part
+  // of what the device has left (otherwise the plans take what they need)
+  size_t free_bytes = 0, total_bytes = 0;
+  if (tile_symmetric(cfg->precision, srv->tile.pc) &&
+      cudaMemGetInfo(&free_bytes, &total_bytes) == cudaSuccess && plan_slot_bytes(*cfg) < 0.1 * (double)free_bytes)
+    (void)srv->slots->buf.alloc((size_t)(plan_slot_bytes(*cfg) / sizeof(double)));
   srv->t0 = std::chrono::steady_clock::now();
   pawan_server *raw = srv.get();
   try {
@@ -556,6 +569,7 @@ void pawan_server_destroy(pawan_server *srv) {
     kv.second->plan.reset();
     if (kv.second->sys) pawan_system_destroy(kv.second->sys);
   }
+  srv->slots.reset();
   cudaStreamSynchronize(srv->ctx->stream);
   if (srv->pool) cudaMemPoolTrimTo(srv->pool, 0);
   pawan_ctx_destroy(srv->ctx);
