@@ -546,6 +546,7 @@ int pawan_server_create(pawan_ctx *ctx, const pawan_serve_config *cfg, pawan_ser
   try {
     srv->worker = std::thread(worker_main, raw);
   } catch (...) {
+    srv->slots.reset();  // (returned in the order of the context's stream)
     pawan_ctx_destroy(srv->ctx);
     return fail(ctx, PAWAN_ERR_NOMEM, "cannot start the serving thread");
   }
