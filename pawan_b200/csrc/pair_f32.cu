@@ -157,7 +157,7 @@ __device__ __forceinline__ void tile_far(const float4 *__restrict__ sa,
       float qh, fh, dp;
       if (NZ && SER) {
         // Z-free far field by the series (kernel_scalars_series), or the
-        // Gaussian kernel's far field (gauss_far)
+        // Gaussian kernel's far field (pair_scalars.cuh)
         float nfh;
         if (KERN == KERNEL_GAUSSIAN) {
           const float ri = rsqrtf(r2);
@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(TB, MINB)
       const bool near = diag || !far_tiles(gap2, slo, shi, sg.near2);
       // every pair at rho >= 6 sigma: the Z-free far field (w of a box = the
       // range of h = s^2/2, so thi.w + shi.w is the largest sigma^2)
-      // Gaussian kernel, every pair at rho >= 7 sigma: its far field (gauss_far),
+      // Gaussian kernel, every pair at rho >= 7 sigma: its far field (pair_scalars.cuh),
       // taken by the series branches of the far loops
       const bool gfar = KERN == KERNEL_GAUSSIAN && !near && gap2 >= 49.f * (thi.w + shi.w);
       const bool nz = (KERN == KERNEL_HIGHORDER && !near && gap2 >= 36.f * (thi.w + shi.w)) || gfar;
@@ -843,21 +843,6 @@ size_t smem_bytes(const PairConfig &c) {
   return 8 * (size_t)c.tb * sizeof(float4) + 10 * fq * sizeof(float4) + 2 * fq * sizeof(float2);
 }
 
-// Opts a kernel in to its dynamic shared memory beyond the default 48 KB (once
-// per kernel and device).
-cudaError_t prepare(KernelFn f, size_t bytes) {
-  static std::mutex mu;
-  static std::set<std::pair<int, KernelFn>> done;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> lk(mu);
-  if (done.count({dev, f})) return cudaSuccess;
-  e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) done.insert({dev, f});
-  return e;
-}
-
 }  // namespace
 
 bool pairs_f32_supported(const PairConfig &c, int kernel) {
@@ -868,7 +853,7 @@ cudaError_t pairs_f32_occupancy(const PairConfig &c, bool diffusion, int kernel,
   const KernelFn f = select(c, diffusion, kernel);
   if (!f) return cudaErrorInvalidValue;
   const size_t bytes = smem_bytes(c);
-  cudaError_t e = prepare(f, bytes);
+  cudaError_t e = allow_dynamic_smem((const void *)f, bytes);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, c.tb, bytes);
 }
@@ -879,7 +864,7 @@ cudaError_t launch_pairs_f32(const PairConfig &c, bool diffusion, int kernel, in
   const KernelFn f = select(c, diffusion, kernel);
   if (!f) return cudaErrorInvalidValue;
   const size_t bytes = smem_bytes(c);
-  cudaError_t e = prepare(f, bytes);
+  cudaError_t e = allow_dynamic_smem((const void *)f, bytes);
   if (e != cudaSuccess) return e;
   f<<<grid, c.tb, bytes, s>>>(items, n_items, segs, next_item);
   return cudaGetLastError();

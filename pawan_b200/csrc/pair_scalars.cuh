@@ -120,7 +120,7 @@ __device__ __forceinline__ void kernel_scalars_series(float sig2, float r2, floa
 // come from their power series in y = -x2/2,
 //   gq = K sum_m y^m / (m! (2m+3)),   gf = -K sum_m y^m / (m! (2m+5)),
 // nine terms (relative truncation error < 1e-8 at x2 = 1).
-// Far field of the Gaussian kernel (gauss_far): where every pair of a tile pair
+// Far field of the Gaussian kernel: where every pair of a tile pair
 // has x = rho/sigma >= 7 (checked on the tiles' boxes), e = exp(-x2/2) <=
 // 2.3e-11 and erf(x/sqrt 2) = 1 - 2.6e-12, so gq = 1/x^3 to 1.3e-10 relative
 // (K e x against 1), gf = -3/x^5 to 2.1e-9 (K e x^3/3 against 1) and dp is 0
