@@ -228,9 +228,10 @@ def state_update_roofline(prof_stage: dict) -> dict:
             "ms_per_launch": ms, "bytes_per_launch": prof_stage["stage_bytes"] / n,
             "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": (gbs / peak) if gbs else None,
             "peak_source": src,
-            "bytes": "per particle: the 48-byte slots of the pair kernel's sums (or rates), the FP64 state vectors "
-                     "the stage reads and writes, radius and volume, and 128 bytes of packed tile data "
-                     "(336-384 bytes for an RK4 stage)"}
+            "bytes": "per particle: every 48-byte slot of the pair kernel's sums (some 210 a particle at N = "
+                     "131,072; traffic of the symmetric engine's own making), the FP64 state vectors the stage reads "
+                     "and writes, radius and volume, and 128 bytes of packed tile data (288-336 bytes for an RK4 "
+                     "stage without the slots)"}
 
 
 def profiled_tiling_matches(tile: dict) -> bool:

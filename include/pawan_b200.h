@@ -277,7 +277,10 @@ int pawan_batch_autotune(pawan_batch *batch);
  * memory pool (stream-ordered) and keeps freed memory there until it is
  * destroyed.  No reference counterpart. */
 typedef struct {
-  double budget_bytes;          /* device memory the admitted requests may hold */
+  double budget_bytes;          /* device memory the admitted requests may hold, the slots of
+                                   the pair kernel's sums among it: those of requests that
+                                   step together share an eighth of it, at most 500 MB,
+                                   which the engine takes at its creation and keeps */
   double max_step_interactions; /* cap on sum N^2 of the requests in one iteration (0: none) */
   int max_active;               /* cap on admitted requests (0: none) */
   int max_queue;                /* waiting requests beyond this are rejected (0: none) */
@@ -327,9 +330,10 @@ int pawan_server_fetch(pawan_server *srv, long long id, double *state, size_t si
                        double *t_submit, double *t_admit, double *t_done);
 int pawan_server_cancel(pawan_server *srv, long long id);
 int pawan_server_stats(pawan_server *srv, pawan_serve_stats *out);
-/* The tiling the engine's pair launches use (FP32: the symmetric engine, in
- * slots of at most 400 MB per request), for running a request alone with the
- * same FP32 arithmetic. */
+/* The tiling the engine's pair launches use (FP32: the symmetric engine), for
+ * running a request alone with the same FP32 arithmetic.  (A request that fits
+ * the budget with one-sided partial sums only runs on the one-sided kernel and
+ * agrees within the FP32 tolerance.) */
 int pawan_server_get_tiling(pawan_server *srv, pawan_tiling *out);
 /* Host-side fault injection, for testing how callers and the engine recover
  * (no GPU fault is made).  PAWAN_FAULT_ALLOC: the next `count` admissions
@@ -351,11 +355,12 @@ int pawan_server_inject(pawan_server *srv, int fault, int count, double seconds)
  * particles with the high-order smoothing kernel, whatever
  * pawan_system_set_kernel chose elsewhere) from caller-owned DEVICE arrays:
  * position and vorticity n x 3, radius and volume n; writes velocity and
- * vorticity rate (n x 3, device).  The pair kernel is pawan_system_solve's
- * with PAWAN_PREC_F32, but the FP32 positions are relative to particle 0
- * rather than the centroid, so results agree with pawan_system_solve within
- * the FP32 tolerance, not bit for bit.  All working memory is one static
- * device array reserved by every GPU that loads the library (about 4.2 MB),
+ * vorticity rate (n x 3, device).  The pair kernel is the one-sided FP32 one
+ * (pawan_system_solve's with a tiling of packed = 0; its default is the
+ * symmetric engine), and the FP32 positions are relative to particle 0 rather
+ * than the centroid, so results agree with pawan_system_solve within the FP32
+ * tolerance, not bit for bit.  All working memory is one static device array
+ * reserved by every GPU that loads the library (5.0 MB),
  * so n <= PAWAN_NOALLOC_MAX_PARTICLES; larger n, n < 2 or a negative or
  * non-finite nu returns PAWAN_ERR_INVALID.  The first call on a device
  * resolves that array's address (make it before any stream capture).  Calls

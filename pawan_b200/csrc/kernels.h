@@ -112,7 +112,7 @@ cudaError_t launch_pairs_plain(const PairConfig &c, int kernel, int grid, const 
 cudaError_t launch_stage(int mode, int n_blocks, const StageItem *items, const StageDesc *descs,
                          cudaStream_t s);
 
-// The same for a symmetric plan whose slots one phase wrote: sums each listed
+// The same for a symmetric plan whose slots one wave wrote: sums each listed
 // tile's slots and applies the stage (every mode but STAGE_PACK, STAGE_SHARD).
 cudaError_t launch_sum_stage(int mode, int n_sums, const SymSum *sums, const StageDesc *descs,
                              const double *slots, cudaStream_t s);

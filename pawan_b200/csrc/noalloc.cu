@@ -25,14 +25,15 @@
 // the call's last kernel, so that calls that raced leave nothing wrong for the
 // calls after them; the rest is fully overwritten before it is read.
 //
-// The pair kernel is pawan_system_solve's in PAWAN_PREC_F32 with the
-// high-order smoothing kernel only, on the one-sided kernel (the symmetric
-// engine's slots would not fit the array).  The array holds 512 chunk slots of
-// 128 targets, so a system of t tiles is split into 512 / t source chunks, and
-// several threads share a target's sources (noalloc_config below): a few
-// thousand particles fill the device that way.  With one thread per target
-// and fixed chunks of 4,096 sources, one call at N = 4,096 ran 32 blocks for
-// 540 us, now 70 (N = 16,384: 560 us, now 513).  The FP32 positions are taken
+// The pair kernel is the one-sided FP32 kernel (pair_f32.cu) with the high-order
+// smoothing kernel only, where pawan_system_solve runs the symmetric engine by
+// default: the array holds 512 slots of 128 targets, and that engine takes t^2 of
+// them for t tiles, so they would do up to 22 tiles (2,816 particles).  A system of
+// t tiles is split into 512 / t source chunks, and several threads share a target's
+// sources (noalloc_config below): a few thousand particles fill the device that
+// way.  With one thread per target and fixed chunks of 4,096 sources, one call at
+// N = 4,096 ran 32 blocks for 540 us, now 75, 58 of them in the pair kernel
+// (N = 16,384: 560 us, now 513).  The FP32 positions are taken
 // relative to particle 0 (pawan_system_set_particles uses the centroid), and
 // the near-tile radius max(4 s_max, 0.03 x extent) measures the extent from
 // particle 0, so it can be up to twice the allocating path's: more tile pairs
@@ -98,6 +99,7 @@ NoallocConfig noalloc_config(int n) {
   return c;
 }
 
+static_assert(sizeof(NoallocScratch) < 5050000, "the array is 5.0 MB, as pawan_b200.h says");
 static_assert(offsetof(NoallocScratch, boxes) % 256 == 0 && offsetof(NoallocScratch, partial) % 256 == 0 &&
                   offsetof(NoallocScratch, rates) % 256 == 0,
               "scratch arrays on 256-byte boundaries");

@@ -21,7 +21,7 @@
 // diffusion vector is formed as v_i w + (v_i mu - v_j) alpha_i - v_j lo_i from
 // the w = alpha_j - mu alpha_i that alpha_i x alpha_j is formed from, accurate for
 // nearly equal strengths and volumes whatever mu's rounding (14 operations; from
-// alpha_j - alpha_i in hi and lo 20: 20,011 unordered particles 846 us, 871).
+// alpha_j - alpha_i in hi and lo 20, and 3 % more time on near tiles).
 //
 // Layout.  A warp computes a 128 x 128 tile pair (I, J): each lane holds R
 // targets of I (4 on far tiles, 2 on near ones) and their sums in registers,
@@ -41,7 +41,7 @@
 // pipe (21 of its cycles per step) would be the limit.  One right-hand side of
 // the ring pair at N = 131,072: 13.9 ms (1,236 G interactions/s) against 18.4 ms
 // one-sided; 20,011 unordered particles (near tile pairs only, mixed radii)
-// 0.85 ms against 1.48.
+// 0.84 ms against 1.48.
 //
 // Compiled without contraction of multiply-adds (every FMA is written out), so
 // that the kernels of the launch shapes below round alike and a system's result
@@ -479,8 +479,8 @@ __device__ __forceinline__ void rotate(Sums6 &a, int m) {
 template <int SIDE, bool UNI, bool DIAG, bool DIFF, int KERN, int R>
 __device__ __forceinline__ void near_block(const Stage &st, int lane, const NearTarget (&T)[R], int self,
                                            float hu, float kap, Sums6 (&a)[R], Sums6 &b) {
-  // steps per iteration (the Gaussian scalars' code is four times as long): 20,011
-  // unordered particles 844 us with two, 835 with four, 842 with eight
+  // steps per iteration (the Gaussian scalars' code is four times as long): against
+  // four, two and eight take 1 % more on near tiles
   constexpr int kUnroll = KERN == KERNEL_GAUSSIAN ? 2 : 4;
   const float s2u = 2.f * hu, c240 = -480.f * hu;
 #pragma unroll 1

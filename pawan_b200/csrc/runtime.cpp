@@ -742,11 +742,12 @@ static void note_repack(Plan &p) {
   }
 }
 
-// Algorithmic HBM bytes of one stage launch: per particle the rates (48
-// bytes: the pair kernel's summed chunks, or the gathered rates of a sharded
-// system; the slots themselves where the stage sums them), the FP64 state vectors the mode reads and writes, radius and
-// volume, and the 128 bytes of packed FP32 / FP64 tile data; 32 bytes of
-// bounding box per tile.  An RK4 stage is 336-384 bytes per particle.
+// Algorithmic HBM bytes of one stage launch: per particle the rates (48 bytes:
+// the pair kernel's summed chunks, or the gathered rates of a sharded system; all
+// slots of 48 bytes where the stage sums them itself), the FP64 state vectors the
+// mode reads and writes, radius and volume, and the 128 bytes of packed FP32 /
+// FP64 tile data; 32 bytes of bounding box per tile.  An RK4 stage is 288-336
+// bytes per particle beside the rates or slots.
 static double stage_bytes(const Plan &p, int mode) {
   double total = 0.0;
   for (size_t s = 0; s < p.systems.size(); ++s) {

@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kStageThreads, kStageMinBlocks)
 }
 
 // The stage update of a plan on the symmetric engine whose slots are all written
-// by one phase: one block per 128-particle tile sums the tile's slots (four
+// by one wave: one block per 128-particle tile sums the tile's slots (four
 // threads per particle, a quarter of the slots each, the quarters then in
 // order), updates the 768 state components one per thread -- contiguous in
 // the state vectors, where one thread per particle strides by three -- and
@@ -240,7 +240,7 @@ __device__ __forceinline__ double slot_sum(const double (*part)[6][kSymTile], in
 }
 
 // The sums alone, into rates[.][128 t ..] (added to what is there when `add`):
-// sharded systems, whose rates are exchanged, and plans of several phases.
+// sharded systems, whose rates are exchanged, and plans of several waves.
 __global__ void __launch_bounds__(kSumThreads, 1)
     sum_slots_kernel(const SymSum *__restrict__ sums, const StageDesc *descs, const double *slots) {
   __shared__ double part[4][6][kSymTile];
