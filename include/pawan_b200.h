@@ -279,7 +279,7 @@ int pawan_batch_autotune(pawan_batch *batch);
 typedef struct {
   double budget_bytes;          /* device memory the admitted requests may hold, the slots of
                                    the pair kernel's sums among it: those of requests that
-                                   step together share an eighth of it, at most 500 MB,
+                                   step together share an eighth of it, at most 250 MB,
                                    which the engine takes at its creation and keeps */
   double max_step_interactions; /* cap on sum N^2 of the requests in one iteration (0: none) */
   int max_active;               /* cap on admitted requests (0: none) */

@@ -30,8 +30,8 @@
 // The engine's systems and plans take their device memory from the device's
 // memory pool in the order of the engine's stream (cudaMallocAsync /
 // cudaFreeAsync): admitting and retiring requests never synchronises the
-// device, and a request's particles are packed by the batched plan built
-// after its admission instead of a plan of its own.  The slots of the batched
+// device, and a request's particles are packed by the batched plan built after its
+// admission instead of a plan of its own.  The slots of the batched
 // plans are one buffer that the engine takes at its creation and keeps: taken and
 // freed with every change of the active set, they cost pauses of 0.1 to 0.5 s now
 // and then (the 99th percentile of a run's latencies 0.03 to 2.4 s).
@@ -116,12 +116,15 @@ double partial_bytes(size_t n, const TileChoice &tile) {
 
 // Bounds on the slots of a batched plan and of one request (which shape a
 // request's decomposition, so they depend on the configuration alone): an eighth
-// of the budget, at most 500 MB and 400 MB.
-double plan_slot_bytes(const pawan_serve_config &cfg) {
-  return std::min(5.0e8, std::max(cfg.budget_bytes / 8.0, 4.0e6));
+// of the budget, at most 250 and 400 MB (a request above the first is a wave of its
+// own).
+// (250 MB take 2 ms to allocate; a wave of them is 0.7 ms of pair work.)
+double slot_bytes(const pawan_serve_config &cfg, double most) {
+  return std::min(most, std::max(cfg.budget_bytes / 8.0, 4.0e6));
 }
 
-double system_slot_bytes(const pawan_serve_config &cfg) { return std::min(4.0e8, plan_slot_bytes(cfg)); }
+double plan_slot_bytes(const pawan_serve_config &cfg) { return slot_bytes(cfg, 2.5e8); }
+double system_slot_bytes(const pawan_serve_config &cfg) { return slot_bytes(cfg, 4.0e8); }
 
 // The engine's tiling: for FP32 one that the symmetric pair engine runs; the
 // library default otherwise.
@@ -203,15 +206,17 @@ void size_request(const pawan_server *srv, Request *r) {
 // Device bytes of requests active together.
 double bytes_of(const pawan_server *srv, const std::vector<Request *> &a, const std::vector<Request *> &b = {},
                 const Request *c = nullptr) {
-  double total = 0.0, shared = 0.0;
+  double total = 0.0, shared = 0.0, largest = 0.0;
   auto add = [&](const Request *r) {
     total += r->bytes;
     (r->large || r->spare ? total : shared) += r->slots;
+    if (!r->large && !r->spare) largest = std::max(largest, r->slots);
   };
   for (const Request *r : a) add(r);
   for (const Request *r : b) add(r);
   if (c) add(c);
-  if (tile_symmetric(srv->cfg.precision, srv->tile.pc)) shared = std::min(shared, plan_slot_bytes(srv->cfg));
+  if (tile_symmetric(srv->cfg.precision, srv->tile.pc))
+    shared = std::min(shared, std::max(largest, plan_slot_bytes(srv->cfg)));
   return total + shared;
 }
 
