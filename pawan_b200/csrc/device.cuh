@@ -124,12 +124,14 @@ struct SymSeg {
 
 // Group a against the groups [b0, b1), a <= b0.  Slots hold the six sums of a
 // group's particles ([tile][6][128] doubles): the item's sums of group a go to
-// slot `islot`, those of group b to slot jbase[jb + b] + a - row0 (none where
-// islot or jbase is negative: another process's targets).  side: which of the
+// slot `islot`, those of group b to slot jbase[jb + b] + a (jbase counts from the
+// phase's first row, so it may be negative); none where islot or jbase is kNoSlot:
+// another process's targets.  side: which of the
 // sums the item forms at all (SIDE_I: group a's alone, SIDE_J: the groups b's).
+constexpr int kNoSlot = INT32_MIN;
 enum SymSide : int { SIDE_BOTH = 0, SIDE_I = 1, SIDE_J = 2 };
 struct SymItem {
-  int seg, a, b0, b1, islot, row0, jb, side;
+  int seg, a, b0, b1, islot, jb, side;
 };
 
 // One tile of the slot sums: `count` slots `stride` doubles apart from

@@ -57,14 +57,14 @@ __device__ __forceinline__ void group_item(const SymItem *__restrict__ items, co
       for (int q = tid; q < kWarps * 6 * kT; q += kThreads) accI[q] += accJ[q];
     } else {
       const int jb = jbase[it.jb + b];
-      if (jb >= 0) {
-        double *out = slots + ((size_t)jb + it.a - it.row0) * kWarps * 6 * kT;
+      if (jb != kNoSlot) {
+        double *out = slots + (size_t)(jb + it.a) * kWarps * 6 * kT;
         for (int q = tid; q < kWarps * 6 * kT; q += kThreads) out[q] = accJ[q];
       }
     }
     __syncthreads();
   }
-  if (it.islot >= 0) {
+  if (it.islot != kNoSlot) {
     double *out = slots + (size_t)it.islot * kWarps * 6 * kT;
     for (int q = tid; q < kWarps * 6 * kT; q += kThreads) out[q] = accI[q];
   }
@@ -89,15 +89,15 @@ __device__ __forceinline__ void tile_item(const SymItem *__restrict__ items, con
   for (int k = 0; k < 6; ++k) accJ[k * kT + tid] = 0.0;
   const SymSeg &sg = wait_previous(segs)[it.seg];
   F::template tile_pair<SIDE>(sg, it.a, it.b0, warp, warp + 1, 0, kT, st, lane, mine, accJ);
-  const int jb = it.b0 > it.a ? jbase[it.jb + it.b0] : -1;
-  if (jb >= 0) {
+  const int jb = it.b0 > it.a ? jbase[it.jb + it.b0] : kNoSlot;
+  if (jb != kNoSlot) {
     // this thread's own source
-    double *out = slots + ((size_t)jb + it.a - it.row0) * 6 * kT;
+    double *out = slots + (size_t)(jb + it.a) * 6 * kT;
 #pragma unroll
     for (int k = 0; k < 6; ++k) out[k * kT + tid] = accJ[k * kT + tid];
   }
   __syncthreads();
-  if (it.islot >= 0) {
+  if (it.islot != kNoSlot) {
     double *out = slots + (size_t)it.islot * 6 * kT;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -143,15 +143,15 @@ __device__ __forceinline__ void spread_item(const SymItem *__restrict__ items, c
     cg::this_cluster().sync();
   else
     __syncthreads();
-  const int jb = it.b0 > it.a ? jbase[it.jb + it.b0] : -1;
-  if (jb >= 0) {
+  const int jb = it.b0 > it.a ? jbase[it.jb + it.b0] : kNoSlot;
+  if (jb != kNoSlot) {
     // thread: one of the block's 32 kSubs sources, three of its six sums
     const int at = 3 * (tid / (32 * kSubs)) * kT + 32 * kSubs * rank + tid % (32 * kSubs);
-    double *out = slots + ((size_t)jb + it.a - it.row0) * kC;
+    double *out = slots + (size_t)(jb + it.a) * kC;
 #pragma unroll
     for (int u = 0; u < 3; ++u) out[at + u * kT] = accJ[at + u * kT] + accJ[kC + at + u * kT];
   }
-  if (it.islot >= 0) {
+  if (it.islot != kNoSlot) {
     const double *c[4];  // the runs of sources in order
 #pragma unroll
     for (int k = 0; k < 4; ++k) {

@@ -302,13 +302,13 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, const SymWaves &w) {
       for (int t = 0; t < l.ng; ++t) {
         const int c = l.slots(t, r0, r1);
         if (!owned(t) || c == 0) {
-          jbase.push_back(-1);
+          jbase.push_back(kNoSlot);
           continue;
         }
         const size_t first = used[grouped];
         used[grouped] += (size_t)c;
         if (used[grouped] > (size_t)INT32_MAX / 2) return fail(ctx, PAWAN_ERR_INVALID, "too many work items");
-        jbase.push_back(t > r0 ? (int)first : -1);
+        jbase.push_back(t > r0 ? (int)first - r0 : kNoSlot);
         if (t >= r0 && t < r1) i0[t] = (int)first + (t - r0);
         for (int q = 0; q < l.g && t * l.g + q < nt; ++q) {
           const long long at = (long long)first * 6 * per + (long long)q * 6 * kSymTile;
@@ -334,7 +334,7 @@ static int build_sym_work(pawan_ctx *ctx, Plan &p, const SymWaves &w) {
           }
           const int side = !owned(a) ? SIDE_J : sources ? SIDE_BOTH : SIDE_I;
           if (side != SIDE_BOTH) p.sided = true;
-          const Costed c{SymItem{(int)s, a, b0, b1, i0[a] < 0 ? -1 : i0[a] + run, r0, jb, side}, cost};
+          const Costed c{SymItem{(int)s, a, b0, b1, i0[a] < 0 ? kNoSlot : i0[a] + run, jb, side}, cost};
           if (b0 <= a + (l.g > 1 ? 1 : 2))
             mine[grouped].push_back(c);
           else
