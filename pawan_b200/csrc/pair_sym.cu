@@ -41,7 +41,7 @@
 // pipe (21 of its cycles per step) would be the limit.  One right-hand side of
 // the ring pair at N = 131,072: 13.9 ms (1,236 G interactions/s) against 18.4 ms
 // one-sided; 20,011 unordered particles (near tile pairs only, mixed radii)
-// 0.84 ms against 1.48.
+// 0.83 ms against 1.48.
 //
 // Compiled without contraction of multiply-adds (every FMA is written out), so
 // that the kernels of the launch shapes below round alike and a system's result
